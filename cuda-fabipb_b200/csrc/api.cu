@@ -8,6 +8,7 @@
 #include <string>
 
 #include "context.cuh"
+#include "fastmath.cuh"
 #include "quad.cuh"
 
 namespace fb {
@@ -303,7 +304,7 @@ int create_context(const fabipb_b200_params *p, int n, const double *vtx, const 
     ok = false;
   }
   StageTimer tm("create", c->stream);
-  ok = ok && init_quad_tables();
+  ok = ok && init_quad_tables() && init_exp_tab();
   ok = ok && setup_geometry(*c, vtx, normal, area);
   tm.mark("tree_and_geometry");
   ok = ok && setup_near(*c);

@@ -1,0 +1,50 @@
+"""The near-field kernels at the sizes where their tiling can go wrong, against the FP64 restatement oracle.
+
+Surfaces are cut from a 1,280-panel sphere, so that leaves hold anything from one panel to more than a tile and the
+special-pair table has open edges.  Tolerances: FP64 1e-12 relative L2, the parity tolerance of the golden cases; mixed
+5e-6 (FP32 pair terms).
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from fabipb_b200 import lib, meshgen, meshio
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def cut_sphere(panels, seed=0):
+    """`panels` faces of the 1,280-panel sphere: a patch, so that some leaves are full and some hold one panel."""
+    unit, faces = meshgen.icosphere(3)
+    pan = meshio.build_panels(20.0 * unit, unit, faces)
+    axis = np.random.default_rng(seed).normal(size=3)
+    keep = np.sort(np.argsort(-(pan.vtx.mean(1) @ axis))[:panels])
+    return meshio.PanelSet(pan.vtx[keep], pan.normal[keep], pan.area[keep], pan.face_index[keep])
+
+
+def both(pan, precision, **opts):
+    s = lib.Surface(pan, lib.params(precision=precision, **opts))
+    o = O.Oracle(pan, O.make_params(**opts))
+    return s, o
+
+
+def check(s, o, tol):
+    rng = np.random.default_rng(7)
+    u, v = rng.standard_normal(2 * s.n), rng.standard_normal(2 * s.n)
+    k = o.near_apply(v)
+    assert rel_l2(s.apply(v, part=lib.NEAR), k) < tol
+    kt = s.apply_adjoint(u, part=lib.NEAR)   # the transposed operator, by duality
+    assert abs(u @ k - kt @ v) <= tol * np.linalg.norm(u) * np.linalg.norm(k)
+
+
+@pytest.mark.parametrize("q", [2, 3])
+@pytest.mark.parametrize("panels,depth", [(2, 2), (37, 2), (319, 3), (640, 2)])
+def test_quadrature_near_field(panels, depth, q):
+    check(*both(cut_sphere(panels), lib.FP64, order=3, depth=depth, quad_order=q), 1e-12)
+
+
+@pytest.mark.parametrize("kappa", [0.0, 1e-3, 40.0])
+def test_quadrature_near_field_screening(kappa):
+    """No screening, and so much that e^{-kappa r} underflows for most pairs."""
+    check(*both(cut_sphere(200), lib.FP64, order=3, depth=3, quad_order=2, kappa=kappa), 1e-12)
