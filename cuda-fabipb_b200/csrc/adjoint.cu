@@ -119,8 +119,8 @@ energy_weights_f2_kernel(int n, int m, const double *__restrict__ vtx, const dou
         const float2 r = __fmul2_rn(r2, ri);
         const float2 ea = __fmul2_rn(ke, r);
         float2 e;
-        e.x = expneg_t(1.f, ea.x);
-        e.y = expneg_t(1.f, ea.y);
+        e.x = expneg_t(ea.x);
+        e.y = expneg_t(ea.y);
         a0 = __ffma2_rn(q, __ffma2_rn(make_float2(-e.x, -e.y), ri, ri), a0);   // q (G0 - Gk) 4 pi
         const float2 ip = __ffma2_rn(nz, dz, __ffma2_rn(ny, dy, __fmul2_rn(nx, dx)));
         const float2 w = __fmul2_rn(ip, __fmul2_rn(__fmul2_rn(ri, ri), ri));
@@ -230,8 +230,8 @@ __device__ __forceinline__ void grad_pair2(const float4 Q0, const float4 Q1, con
   const float2 r = __fmul2_rn(r2, ri), ri2 = __fmul2_rn(ri, ri), ri3 = __fmul2_rn(ri2, ri);
   const float2 ea = __fmul2_rn(f2(kexp), r);
   float2 e;
-  e.x = expneg_t(1.f, ea.x);
-  e.y = expneg_t(1.f, ea.y);
+  e.x = expneg_t(ea.x);
+  e.y = expneg_t(ea.y);
   const float2 c = __fmul2_rn(__ffma2_rn(f2(kappa), r, f2(1.f)), e);
   const float2 nx = make_float2(Q2.x, Q2.y), ny = make_float2(Q2.z, Q2.w), nz = make_float2(Q3.x, Q3.y);
   const float2 ip = __ffma2_rn(nz, z, __ffma2_rn(ny, y, __fmul2_rn(nx, x)));

@@ -15,6 +15,7 @@ struct ChargeTreeDev;
 struct PrecondDev;
 struct AdjointDev;
 struct GraphCache;
+struct NearTask;
 
 struct Context {
   fabipb_b200_params prm{};
@@ -32,7 +33,7 @@ struct Context {
   int *d_leafStart = nullptr, *d_leafCount = nullptr, *d_leafOfPanel = nullptr;
   int *d_nearOff = nullptr, *d_nearSrc = nullptr;
   double *d_leafCtr = nullptr;             // 3 per leaf: enclosing-box centre
-  int nWork = 0;                           // near-field warp tasks
+  int nWork = 0;                           // blocks of the near field's finishing kernel
   int2 *d_work = nullptr;                  // (leaf, 32-target group)
   long long nearPanelPairs = 0;
   int maxLeaf = 0;
@@ -40,23 +41,20 @@ struct Context {
   // ---- near field -------------------------------------------------------
   bool mixed = false;                      // FP32 P2P when true
   void *d_tgtP = nullptr, *d_tgtN = nullptr;   // T4: {rel pos, area}, {normal, 0}
-  void *d_srcA = nullptr, *d_srcB = nullptr;   // T4: {rel pos, A*s_dpdn}, {normal, A*s_pot}
+  void *d_recA = nullptr, *d_recB = nullptr;   // T4: {rel pos, A*s_dpdn}, {normal, A*s_pot} of the current apply
   long long nSpecial = 0;
   int *d_spOff = nullptr, *d_spSrc = nullptr;  // CSR by destination panel
   double4 *d_spK = nullptr;                    // exact minus one-point coefficient
   double4 *d_spKT = nullptr;                   // the same for the transposed operator
   void *d_tgtP64 = nullptr, *d_tgtN64 = nullptr;   // FP64 records of a mixed context (refinement residuals)
-  // the symmetric near field: unordered leaf pairs (register leaf, tile leaf, scratch offsets),
-  // per near-list entry its scratch offset (-1: the ordered kernel computes it); scratch and
-  // records in the context's near-field precision (2 and 4 floats or doubles per entry)
-  int nSymTasks = 0;
-  int nSym32 = 0;                              // the first nSym32 tasks are 32-wide, the rest half-warp
-  long long symPanelPairs = 0;                 // unordered panel pairs of those leaf pairs
-  int4 *d_symTask = nullptr;
-  int *d_symOff = nullptr;
+  // the symmetric near field: its tasks (the first nSym32 on a warp, the rest on a half-warp), the
+  // scratch slots of their sums (two floats or doubles each) listed by leaf for the finishing kernel,
+  // and by leaf the source leaves that no task covers
+  int nSymTasks = 0, nSym32 = 0;
+  NearTask *d_symTask = nullptr;
+  int *d_gatOff = nullptr, *d_gatSlot = nullptr;
+  int *d_ordOff = nullptr, *d_ordSrc = nullptr;
   void *d_symScr = nullptr;
-  void *d_symA = nullptr, *d_symB = nullptr;   // records {position, A*sigma_dpdn}, {normal, A*sigma_pot}
-  void *d_srcA64 = nullptr, *d_srcB64 = nullptr;
 
   // ---- FMM ----------------------------------------------------------
   int P = 0, NM = 0;                       // max order, nmom(max order)

@@ -44,109 +44,19 @@ template <>
 struct Vec4<double> {
   typedef double4 t;
 };
-template <typename T>
-struct Pair2;
-template <>
-struct Pair2<float> {
-  typedef float2 t;
-};
-template <>
-struct Pair2<double> {
-  typedef double2 t;
-};
-
-// The ordered kernels' gathers, written so that their loads overlap instead of
-// forming one dependent chain per near leaf or special pair.
-//
-// sym_scratch_sums: the symmetric kernels' sums of this target (offset xo in its
-// leaf) over the near-list entries [p0, p1) that they took, in list order:
-// the warp reads 32 entries' slots at once and keeps up to 8 scratch loads in
-// flight.  take: the lane adds (one lane per target).
-template <typename T>
-__device__ __forceinline__ void sym_scratch_sums(int p0, int p1, int lane, bool take, int xo,
-                                                 const int *__restrict__ symOff, const T *__restrict__ symScr,
-                                                 T &a0, T &a1) {
-  typedef typename Pair2<T>::t P;
-  const P *scr = reinterpret_cast<const P *>(symScr);
-  for (int q0 = p0; q0 < p1; q0 += 32) {
-    const int o = q0 + lane < p1 ? symOff[q0 + lane] : -1;
-    unsigned m = __ballot_sync(0xffffffffu, o >= 0);
-    while (m) {   // warp-uniform
-      T v0[8], v1[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        v0[u] = v1[u] = (T)0;
-        if (m) {   // warp-uniform
-          const int oj = __shfl_sync(0xffffffffu, o, __ffs(m) - 1);
-          m &= m - 1;
-          if (take) {
-            const P v = scr[(size_t)oj + xo];
-            v0[u] = v.x;
-            v1[u] = v.y;
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        a0 += v0[u];
-        a1 += v1[u];
-      }
-    }
-  }
-}
-
-// special_sums: the FP64 special-pair corrections of target X in table order,
-// four entries' loads (index, coefficients, then the two densities) at a time.
-__device__ __forceinline__ void special_sums(int X, int n, const int *__restrict__ spOff,
-                                             const int *__restrict__ spSrc, const double4 *__restrict__ spK,
-                                             const double *__restrict__ sgm, double &e0, double &e1) {
-  int e = spOff[X];
-  const int e1End = spOff[X + 1];
-  for (; e + 4 <= e1End; e += 4) {
-    int Y[4];
-    double4 d[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      Y[u] = spSrc[e + u];
-      d[u] = spK[e + u];
-    }
-    double sp[4], sd[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      sp[u] = sgm[Y[u]];
-      sd[u] = sgm[n + Y[u]];
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      e0 += d[u].x * sd[u] + d[u].y * sp[u];
-      e1 += d[u].z * sd[u] + d[u].w * sp[u];
-    }
-  }
-  for (; e < e1End; e++) {
-    const int Y = spSrc[e];
-    const double4 d = spK[e];
-    const double sp = sgm[Y], sd = sgm[n + Y];
-    e0 += d.x * sd + d.y * sp;
-    e1 += d.z * sd + d.w * sp;
-  }
-}
-
 // FP32: the single MUFU instructions (PTX rsqrt.approx / ex2.approx, flush
-// to zero; relative error ~2^-22, far below the FP32 P2P tolerance).  FP64:
-// the library functions.
+// to zero; relative error ~2^-22, far below the FP32 P2P tolerance).
 __device__ __forceinline__ float rsqrt_t(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
-// e^{-kappa r}: float evaluates 2^(kexp r) with kexp = -kappa*log2(e)
-__device__ __forceinline__ float expneg_t(float kexp, float r) {
+// 2^x: e^{-kappa r} is taken at x = -kappa log2(e) r
+__device__ __forceinline__ float expneg_t(float x) {
   float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(kexp * r));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ double expneg_t(double kexp, double r) { return exp(kexp * r); }
 
 template <typename T>
 __global__ void near_targets_kernel(int n, const double *__restrict__ vtx, const double *__restrict__ nrm,
@@ -169,275 +79,508 @@ __global__ void near_targets_kernel(int n, const double *__restrict__ vtx, const
   tgtN[i] = q;
 }
 
-// Source records of one apply: {position, A*sigma_dpdn}, {normal, A*sigma_pot}.
-// scaleNormal 1 (2): the normal is stored multiplied by the second (first)
-// weight, for the packed FP32 kernel, whose pair formula takes the source
-// normal only in terms that carry that weight.
+// Record of panel i for the density sgm: {position, A*sigma_dpdn}, {normal, A*sigma_pot}.
+template <typename T>
+__device__ __forceinline__ void near_record(int i, int n, const typename Vec4<T>::t *__restrict__ tgtP,
+                                            const typename Vec4<T>::t *__restrict__ tgtN,
+                                            const double *__restrict__ area, const double *__restrict__ sgm,
+                                            typename Vec4<T>::t &a, typename Vec4<T>::t &b) {
+  a = tgtP[i];
+  b = tgtN[i];
+  const double A = area[i];
+  a.w = (T)(A * sgm[n + i]);   // weight of the dpdn density
+  b.w = (T)(A * sgm[i]);       // weight of the potential density
+}
+
+// the records of one apply, for the symmetric tasks, which read each many times
 template <typename T>
 __global__ void near_pack_kernel(int n, const typename Vec4<T>::t *__restrict__ tgtP,
                                  const typename Vec4<T>::t *__restrict__ tgtN, const double *__restrict__ area,
-                                 const double *__restrict__ sgm, typename Vec4<T>::t *srcA,
-                                 typename Vec4<T>::t *srcB, int scaleNormal) {
+                                 const double *__restrict__ sgm, typename Vec4<T>::t *recA,
+                                 typename Vec4<T>::t *recB) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  typename Vec4<T>::t a = tgtP[i], b = tgtN[i];
-  double A = area[i];
-  const double wa = A * sgm[n + i], wb = A * sgm[i];
-  a.w = (T)wa;  // weight of the dpdn density
-  b.w = (T)wb;  // weight of the potential density
-  if (scaleNormal) {
-    const T w = (T)(scaleNormal == 1 ? wb : wa);
-    b.x *= w;
-    b.y *= w;
-    b.z *= w;
-  }
-  srcA[i] = a;
-  srcB[i] = b;
+  typename Vec4<T>::t a, b;
+  near_record<T>(i, n, tgtP, tgtN, area, sgm, a, b);
+  recA[i] = a;
+  recB[i] = b;
 }
 
 constexpr int kNearWarps = 4;
-// resident blocks per SM the register allocation of near_apply_kernel<float> aims at
-#ifndef FB_NEAR_MIN_BLOCKS
-#define FB_NEAR_MIN_BLOCKS 8
-#endif
-// FP32 near field with packed f32x2 arithmetic (near_apply_f2_kernel)
-#ifndef FB_NEAR_PACKED
-#define FB_NEAR_PACKED 1
-#endif
 
 // One disjoint pair, one-point rule: the four KER4 kernels (src/kernel.c:109-147)
 // at d = target - source, times the source weights a.w = A*sigma_dpdn and
 // b.w = A*sigma_pot (the 4 pi and the target area are applied once at the end).
+// With g = 1/r, h = g^3, c = (kappa r + 1) e^{-kappa r}, the pair's terms are
+//   F  = h (eps c - 1),   Fi = h (c/eps - 1),   H1 = h (c - 1),
+//   y0 = g - g e,   y1 = (n_s.d) F,   y2 = (n_t.d) Fi,
+//   y3 = (n_t.n_s) H1 - (n_t.d)(n_s.d) (3 g^2 H1 + kappa^2 h e).
 //
-// ADJ: the transposed pair block.  With d = target - source, swapping the
-// roles of the two panels gives K0 and K3 unchanged, K1(s,t) = -t2 (eps c - 1)
-// and K2(s,t) = -t1 (c/eps - 1), so
-//   out_pot  += y3 * a.w - t2 (eps c - 1) * b.w
-//   out_dpdn += y0 * b.w - t1 (c/eps - 1) * a.w
+// ADJ: the transposed pair block.  Swapping the roles of the two panels gives
+// K0 and K3 unchanged, K1(s,t) = -(n_t.d) F and K2(s,t) = -(n_s.d) Fi, so
+//   out_pot  += y3 * a.w - (n_t.d) F * b.w
+//   out_dpdn += y0 * b.w - (n_s.d) Fi * a.w
 // with a.w = A*lambda_dpdn and b.w = A*lambda_pot of the source panel.
-template <bool ADJ, typename T, typename V>
-__device__ __forceinline__ void near_pair(const V a, const V b, T tx, T ty, T tz, const V tn, T kappa, T kexp, T eps,
-                                          T ieps, T kap2, T &acc0, T &acc1) {
-  const T dx = tx - a.x, dy = ty - a.y, dz = tz - a.z;
-  const T r2 = dx * dx + dy * dy + dz * dz;
-  const T g = r2 > (T)0 ? rsqrt_t(r2) : (T)0;   // 1/r, 0 for the coincident pair
-  const T r = r2 * g;
-  const T e = expneg_t(kexp, r);
-  const T c = (kappa * r + (T)1) * e;           // (kappa r + 1) e^{-kappa r}
-  const T g2 = g * g;
-  const T h = g2 * g;
-  const T ipX = tn.x * dx + tn.y * dy + tn.z * dz;
-  const T ipY = b.x * dx + b.y * dy + b.z * dz;
-  const T ip0 = tn.x * b.x + tn.y * b.y + tn.z * b.z;
-  const T t1 = ipY * h;                          // dG0/dn_y * 4 pi
-  const T t2 = ipX * h;                          // dG0/dn_x * 4 pi
-  const T u = ipX * t1;
-  const T y0 = g - g * e;                        // G0 - Gk
-  const T y1 = t1 * (eps * c - (T)1);            // eps dGk/dn_y - dG0/dn_y
-  const T y2 = t2 * (c * ieps - (T)1);           // dGk/dn_x / eps - dG0/dn_x
-  const T dd = (ip0 * g - (T)3 * u) * g2;        // d2 G0 / dn_x dn_y
-  const T y3 = dd * (c - (T)1) - kap2 * e * u;
+struct NearConstD {
+  double kappa, kexp, eps, ieps, kap2;
+};
+struct NearConstF {
+  float kappa, kexp, eps, ieps, kap2;
+};
+
+template <bool ADJ>
+__device__ __forceinline__ void near_pair(const double4 a, const double4 b, double tx, double ty, double tz,
+                                          const double4 tn, const NearConstD &K, double &acc0, double &acc1) {
+  const double dx = tx - a.x, dy = ty - a.y, dz = tz - a.z;
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  const double g = r2 > 0.0 ? rsqrt(r2) : 0.0;   // 1/r, 0 for the coincident pair
+  const double r = r2 * g;
+  const double e = exp(K.kexp * r);
+  const double g2 = g * g, h = g2 * g, he = h * e, hc = he * (K.kappa * r + 1.0);
+  const double H1 = hc - h, F = K.eps * hc - h, Fi = K.ieps * hc - h;
+  const double ipX = tn.x * dx + tn.y * dy + tn.z * dz;
+  const double ipY = b.x * dx + b.y * dy + b.z * dz;
+  const double ip0 = tn.x * b.x + tn.y * b.y + tn.z * b.z;
+  const double y0 = g - g * e;
+  const double y3 = ip0 * H1 - ipX * ipY * (3.0 * (g2 * H1) + K.kap2 * he);
   if (ADJ) {
-    acc0 += y3 * a.w - t2 * (eps * c - (T)1) * b.w;
-    acc1 += y0 * b.w - t1 * (c * ieps - (T)1) * a.w;
+    acc0 += y3 * a.w - ipX * F * b.w;
+    acc1 += y0 * b.w - ipY * Fi * a.w;
   } else {
-    acc0 += y0 * a.w + y1 * b.w;
-    acc1 += y2 * a.w + y3 * b.w;
+    acc0 += y0 * a.w + ipY * F * b.w;
+    acc1 += ipX * Fi * a.w + y3 * b.w;
   }
 }
 
-// One warp per task (leaf L, group of up to 32 target panels).  A full group
-// puts one target on each lane; a partial group of mt targets gives each
-// target k = 32/mt lanes, which take every k-th source of a tile, and their
-// partial sums are added at the end, so short groups keep most lanes busy.
-template <typename T, bool ADJ>
-__global__ void __launch_bounds__(kNearWarps * 32, sizeof(T) == 4 ? FB_NEAR_MIN_BLOCKS : 1)
-near_apply_kernel(int nWork, const int2 *__restrict__ work, const int *__restrict__ leafStart,
-                  const int *__restrict__ leafCount, const int *__restrict__ nearOff,
-                  const int *__restrict__ nearSrc, const double *__restrict__ leafCtr,
-                  const typename Vec4<T>::t *__restrict__ tgtP, const typename Vec4<T>::t *__restrict__ tgtN,
-                  const typename Vec4<T>::t *__restrict__ srcA, const typename Vec4<T>::t *__restrict__ srcB,
-                  const int *__restrict__ spOff, const int *__restrict__ spSrc,
-                  const double4 *__restrict__ spK, const double *__restrict__ sgm,
-                  const double *__restrict__ area, int n, T kappa, T kexp, T eps, T ieps, T kap2,
-                  double coef, int accumulate, double *out, const int *__restrict__ symOff,
-                  const T *__restrict__ symScr) {
-  typedef typename Vec4<T>::t V;
-  __shared__ V sA[kNearWarps][32];
-  __shared__ V sB[kNearWarps][32];
-  __shared__ T sR[kNearWarps][2][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * kNearWarps + warp;
-  if (task >= nWork) return;  // warp-uniform
-  const int2 wk = work[task];
-  const int L = wk.x;
-  const int base = leafStart[L], cnt = leafCount[L];
-  const int g0 = 32 * wk.y;
-  const int mt = min(32, cnt - g0);   // targets in this group
-  const int k = 32 / mt;              // lanes per target
-  const int t = lane / k, sub = lane - t * k;
-  const bool valid = t < mt;
-  const int X = base + g0 + (valid ? t : 0);
-  const V tp = tgtP[X], tn = tgtN[X];
-  const double cx = leafCtr[3 * L], cy = leafCtr[3 * L + 1], cz = leafCtr[3 * L + 2];
-  T acc0 = (T)0, acc1 = (T)0;
-  const int pBeg = nearOff[L], p1 = nearOff[L + 1];
-  // the leaf pairs of the symmetric kernel: their sums for this target are in the scratch
-  if (symOff) sym_scratch_sums<T>(pBeg, p1, lane, valid && sub == 0, X - base, symOff, symScr, acc0, acc1);
-  // the other near leaves
-  for (int p = pBeg; p < p1; p++) {
-    if (symOff && symOff[p] >= 0) continue;   // warp-uniform: summed above
-    const int S = nearSrc[p];
-    const int sb = leafStart[S], sc = leafCount[S];
-    const T tx = tp.x + (T)(cx - leafCtr[3 * S]);
-    const T ty = tp.y + (T)(cy - leafCtr[3 * S + 1]);
-    const T tz = tp.z + (T)(cz - leafCtr[3 * S + 2]);
-    for (int j0 = 0; j0 < sc; j0 += 32) {
-      const int m = min(32, sc - j0);
-      if (lane < m) {
-        sA[warp][lane] = srcA[sb + j0 + lane];
-        sB[warp][lane] = srcB[sb + j0 + lane];
-      }
-      __syncwarp();
-      if (k == 1) {   // warp-uniform: a full group, unit stride
-#pragma unroll 4
-        for (int jj = 0; jj < m; jj++)
-          near_pair<ADJ>(sA[warp][jj], sB[warp][jj], tx, ty, tz, tn, kappa, kexp, eps, ieps, kap2, acc0, acc1);
-      } else {
-#pragma unroll 4
-        for (int jj = sub; jj < m; jj += k)
-          near_pair<ADJ>(sA[warp][jj], sB[warp][jj], tx, ty, tz, tn, kappa, kexp, eps, ieps, kap2, acc0, acc1);
-      }
-      __syncwarp();
+// The same in FP32 for two sources at once (packed f32x2: sm_100
+// FFMA2/FMUL2/FADD2).  A source pair is four float4
+//   A = (-x0 -x1 -y0 -y1), B = (-z0 -z1 wa0 wa1), C = (nx0 nx1 ny0 ny1), D = (nz0 nz1 wb0 wb1),
+// so the packed operands come straight from the loads.  Signs are arranged so
+// that no packed operand has to be negated but 1/r.  ADJ: wb is stored negated
+// and acc1 is the negated sum:
+//   acc0 += y3 wa + (n_t.d) F wb,  acc1 += y0 wb + (n_s.d) Fi wa.
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+
+struct NearPairF2 {
+  float2 y0, y3, a1, a2, b1, b2;   // a1 = (n_s.d) F, a2 = (n_t.d) F, b1 = (n_s.d) Fi, b2 = (n_t.d) Fi
+};
+template <int G>
+struct NearTargetsF2 {   // G targets, each value in both halves
+  float2 x[G], y[G], z[G], nx[G], ny[G], nz[G];
+};
+
+// The terms of a source pair and G targets, operation by operation over the
+// targets: a packed FMA with three register operands takes three to four
+// cycles of register reads instead of two, and neighbours that share one are
+// what the operand reuse of the scheduler can shorten.
+// SELF (the target's own leaf, the only tile holding the coincident pair
+// d = 0): 1/r is taken as 0 there, which zeroes every term.
+template <bool SELF, int G>
+__device__ __forceinline__ void near_terms2(const float4 A, const float4 B, const float4 C, const float4 D,
+                                            const NearTargetsF2<G> &t, const NearConstF &K, NearPairF2 (&p)[G]) {
+#define FB_EACH _Pragma("unroll") for (int k = 0; k < G; k++)
+  const float2 nx = make_float2(C.x, C.y), ny = make_float2(C.z, C.w), nz = make_float2(D.x, D.y);
+  float2 dx[G], dy[G], dz[G], r2[G], g[G], ng[G], e[G], c1[G], g2[G], nh[G], he[G], hc[G], H1[G], F[G], Fi[G];
+  float2 ipX[G], ipY[G], ip0[G], w[G];
+  FB_EACH dx[k] = __fadd2_rn(t.x[k], make_float2(A.x, A.y));
+  FB_EACH dy[k] = __fadd2_rn(t.y[k], make_float2(A.z, A.w));
+  FB_EACH dz[k] = __fadd2_rn(t.z[k], make_float2(B.x, B.y));
+  FB_EACH r2[k] = __fmul2_rn(dx[k], dx[k]);
+  FB_EACH r2[k] = __ffma2_rn(dy[k], dy[k], r2[k]);
+  FB_EACH r2[k] = __ffma2_rn(dz[k], dz[k], r2[k]);
+  FB_EACH {
+    if (SELF) {
+      g[k].x = r2[k].x > 0.f ? rsqrt_t(r2[k].x) : 0.f;
+      g[k].y = r2[k].y > 0.f ? rsqrt_t(r2[k].y) : 0.f;
+    } else {   // distinct leaves: distinct panel centroids, r > 0
+      g[k].x = rsqrt_t(r2[k].x);
+      g[k].y = rsqrt_t(r2[k].y);
     }
+    ng[k] = make_float2(-g[k].x, -g[k].y);
   }
-  if (k > 1) {   // warp-uniform: add the k partial sums of each target
-    sR[warp][0][lane] = acc0;
-    sR[warp][1][lane] = acc1;
-    __syncwarp();
-    if (valid && sub == 0)
-      for (int i = 1; i < k; i++) {
-        acc0 += sR[warp][0][lane + i];
-        acc1 += sR[warp][1][lane + i];
+  FB_EACH r2[k] = __fmul2_rn(r2[k], g[k]);   // r
+  FB_EACH {
+    const float2 ea = __fmul2_rn(f2(K.kexp), r2[k]);
+    e[k].x = expneg_t(ea.x);
+    e[k].y = expneg_t(ea.y);
+  }
+  FB_EACH c1[k] = __ffma2_rn(f2(-K.kappa), r2[k], f2(-1.f));   // -(kappa r + 1)
+  FB_EACH g2[k] = __fmul2_rn(g[k], g[k]);
+  FB_EACH nh[k] = __fmul2_rn(g2[k], ng[k]);                    // -h
+  FB_EACH he[k] = __fmul2_rn(nh[k], e[k]);                     // -h e
+  FB_EACH hc[k] = __fmul2_rn(he[k], c1[k]);                    // h c
+  FB_EACH H1[k] = __fadd2_rn(hc[k], nh[k]);
+  FB_EACH F[k] = __ffma2_rn(f2(K.eps), hc[k], nh[k]);
+  FB_EACH Fi[k] = __ffma2_rn(f2(K.ieps), hc[k], nh[k]);
+  FB_EACH ipX[k] = __fmul2_rn(t.nx[k], dx[k]);                 // n_t.d
+  FB_EACH ipX[k] = __ffma2_rn(t.ny[k], dy[k], ipX[k]);
+  FB_EACH ipX[k] = __ffma2_rn(t.nz[k], dz[k], ipX[k]);
+  FB_EACH ipY[k] = __fmul2_rn(nx, dx[k]);                      // n_s.d
+  FB_EACH ipY[k] = __ffma2_rn(ny, dy[k], ipY[k]);
+  FB_EACH ipY[k] = __ffma2_rn(nz, dz[k], ipY[k]);
+  FB_EACH ip0[k] = __fmul2_rn(nx, t.nx[k]);                    // n_t.n_s
+  FB_EACH ip0[k] = __ffma2_rn(ny, t.ny[k], ip0[k]);
+  FB_EACH ip0[k] = __ffma2_rn(nz, t.nz[k], ip0[k]);
+  FB_EACH w[k] = __ffma2_rn(f2(-3.f), __fmul2_rn(g2[k], H1[k]), __fmul2_rn(f2(K.kap2), he[k]));
+  FB_EACH p[k].y0 = __ffma2_rn(ng[k], e[k], g[k]);
+  FB_EACH p[k].y3 = __ffma2_rn(__fmul2_rn(ipX[k], ipY[k]), w[k], __fmul2_rn(ip0[k], H1[k]));
+  FB_EACH p[k].a1 = __fmul2_rn(ipY[k], F[k]);
+  FB_EACH p[k].a2 = __fmul2_rn(ipX[k], F[k]);
+  FB_EACH p[k].b1 = __fmul2_rn(ipY[k], Fi[k]);
+  FB_EACH p[k].b2 = __fmul2_rn(ipX[k], Fi[k]);
+}
+
+template <bool ADJ, bool SELF>
+__device__ __forceinline__ void near_pair2(const float4 A, const float4 B, const float4 C, const float4 D,
+                                           const NearTargetsF2<1> &t, const NearConstF &K, float2 &acc0,
+                                           float2 &acc1) {
+  NearPairF2 p[1];
+  near_terms2<SELF, 1>(A, B, C, D, t, K, p);
+  const float2 wa = make_float2(B.z, B.w), wb = make_float2(D.z, D.w);
+  if (ADJ) {
+    acc0 = __ffma2_rn(p[0].a2, wb, __ffma2_rn(p[0].y3, wa, acc0));
+    acc1 = __ffma2_rn(p[0].b1, wa, __ffma2_rn(p[0].y0, wb, acc1));
+  } else {
+    acc0 = __ffma2_rn(p[0].a1, wb, __ffma2_rn(p[0].y0, wa, acc0));
+    acc1 = __ffma2_rn(p[0].y3, wb, __ffma2_rn(p[0].b2, wa, acc1));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Symmetric near field.  The pair terms of K(X, Y) and K(Y, X) share r, 1/r,
+// e^{-kappa r}, the normal products and F, Fi, y0, y3; with d = x_X - x_Y,
+// swapping the panels negates d, so
+//   K(Y,X): out_pot  += y0 wa_X - (n_X.d) F wb_X,
+//           out_dpdn += y3 wb_X - (n_Y.d) Fi wa_X.
+// So every unordered pair of distinct near leaves (R, T) is evaluated once
+// for both directions, without atomics: the sums go to a scratch slot per
+// (leaf, task), which the finishing kernel adds in a fixed order.
+//
+// A task is a leaf pair, or a chunk of R's panels against all of T, on W lanes
+// (a warp, or a half-warp for pairs that pad badly into 32-panel groups).
+// Every lane holds one or two target panels of R in registers; T passes in
+// tiles of W sources through shared memory.  In step s, lane t takes the
+// tile's sources t + s and t + s + W/2 (mod W) as one packed pair, so the
+// lanes hold distinct sources; the sources' own sums travel with them, one
+// lane down per step, and are added to by the same FMAs that form the terms.
+//
+// Bound by the FP32 FMA pipe: 44 packed operations (two cycles each) for the
+// two directions of two pairs.  Two targets per lane halve the shared-memory
+// reads and shuffles per pair, which beside 46 + 2 operations with one target
+// per lane and gathered sums had left the pipe at 75%.
+// Measured (whole products, before -> after): two-shell 2,096,704 panels 25.8
+// -> 23.4 ms, its quarter transposed 9.45 -> 8.11 ms, star 204,800 panels 605 ->
+// 553 us, sphere 20,480 panels 144 -> 80 us (there by the split into tasks).
+// ---------------------------------------------------------------------------
+// steps of a tile unrolled together, and resident blocks per SM that the
+// register allocation aims at (two targets per lane: 4 at 128 registers)
+#ifndef FB_NEAR_SYM_UNROLL
+#define FB_NEAR_SYM_UNROLL 2
+#endif
+#ifndef FB_NEAR_SYM_MIN_BLOCKS
+#define FB_NEAR_SYM_MIN_BLOCKS 4
+#endif
+constexpr int kSymUnroll = FB_NEAR_SYM_UNROLL;
+constexpr int kSymWarps = 4;
+
+// a task: leaves R (registers) and T (tiles), R's panels [r0, r1), and the
+// first scratch slots of R's and T's sums
+struct NearTask {
+  int R, T, r0, r1, scrR, scrT;
+};
+
+// G * W targets of R from r0 against all of T.  first: the sums of T start here.
+template <bool ADJ, int W, int G>
+__device__ __forceinline__ void near_sym_group(float4 *Q, unsigned mask, int hl, int r0, int r1, int rb, int tb,
+                                               int tc, float sx, float sy, float sz, bool first,
+                                               const float4 *__restrict__ recA, const float4 *__restrict__ recB,
+                                               const NearConstF &K, float2 *scrR, float2 *scrT) {
+  NearTargetsF2<G> tg;
+  float2 wat[G], wbt[G], nwat[G], nwbt[G], acc0[G], acc1[G];
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    const int t = r0 + k * W + hl;
+    // a lane past the end: far away, zero weights (its terms vanish, its sums are dropped)
+    const float4 a = t < r1 ? recA[rb + t] : make_float4(1e4f, 1e4f, 1e4f, 0.f);
+    const float4 b = t < r1 ? recB[rb + t] : make_float4(0.f, 0.f, 1.f, 0.f);
+    tg.x[k] = f2(a.x + sx); tg.y[k] = f2(a.y + sy); tg.z[k] = f2(a.z + sz);
+    tg.nx[k] = f2(b.x); tg.ny[k] = f2(b.y); tg.nz[k] = f2(b.z);
+    wat[k] = f2(a.w); wbt[k] = f2(b.w); nwat[k] = f2(-a.w); nwbt[k] = f2(-b.w);
+    acc0[k] = acc1[k] = f2(0.f);
+  }
+  // the tile's source hl, or a padding source far away with zero weights; loaded one tile ahead
+  const float4 farA = make_float4(-1e4f, -1e4f, -1e4f, 0.f), farB = make_float4(0.f, 0.f, 1.f, 0.f);
+  float4 na = hl < tc ? recA[tb + hl] : farA, nb = hl < tc ? recB[tb + hl] : farB;
+  for (int j0 = 0; j0 < tc; j0 += W) {
+    const int j = j0 + hl;
+    const float4 sa = na, sb = nb;
+    na = j + W < tc ? recA[tb + j + W] : farA;
+    nb = j + W < tc ? recB[tb + j + W] : farB;
+    const float2 prev = first || j >= tc ? f2(0.f) : scrT[j];
+    // slot m holds source m first and source m + W/2 (mod W) second
+    const float ox = __shfl_xor_sync(mask, sa.x, W / 2), oy = __shfl_xor_sync(mask, sa.y, W / 2);
+    const float oz = __shfl_xor_sync(mask, sa.z, W / 2), ow = __shfl_xor_sync(mask, sa.w, W / 2);
+    const float px = __shfl_xor_sync(mask, sb.x, W / 2), py = __shfl_xor_sync(mask, sb.y, W / 2);
+    const float pz = __shfl_xor_sync(mask, sb.z, W / 2), pw = __shfl_xor_sync(mask, sb.w, W / 2);
+    __syncwarp(mask);   // the previous tile's reads are done
+    Q[hl] = make_float4(-sa.x, -ox, -sa.y, -oy);
+    Q[W + hl] = make_float4(-sa.z, -oz, sa.w, ow);
+    Q[2 * W + hl] = make_float4(sb.x, px, sb.y, py);
+    Q[3 * W + hl] = ADJ ? make_float4(sb.z, pz, -sb.w, -pw) : make_float4(sb.z, pz, sb.w, pw);
+    __syncwarp(mask);
+    float2 o0 = f2(0.f), o1 = f2(0.f);   // the travelling sums (pot, dpdn) of this lane's two sources
+#pragma unroll kSymUnroll
+    for (int st = 0; st < W / 2; st++) {
+      const int slot = (hl + st) & (W - 1);
+      const float4 A = Q[slot], B = Q[W + slot], C = Q[2 * W + slot], D = Q[3 * W + slot];
+      const float2 wa = make_float2(B.z, B.w), wb = make_float2(D.z, D.w);
+      NearPairF2 p[G];
+      near_terms2<false, G>(A, B, C, D, tg, K, p);
+      if (ADJ) {   // wb negated, acc1 the negated sum
+        FB_EACH acc0[k] = __ffma2_rn(p[k].y3, wa, acc0[k]);
+        FB_EACH acc1[k] = __ffma2_rn(p[k].b1, wa, acc1[k]);
+        FB_EACH acc0[k] = __ffma2_rn(p[k].a2, wb, acc0[k]);
+        FB_EACH acc1[k] = __ffma2_rn(p[k].y0, wb, acc1[k]);
+        FB_EACH {
+          o0 = __ffma2_rn(p[k].a1, wbt[k], __ffma2_rn(p[k].y3, wat[k], o0));
+          o1 = __ffma2_rn(p[k].b2, wat[k], __ffma2_rn(p[k].y0, wbt[k], o1));
+        }
+      } else {
+        FB_EACH acc0[k] = __ffma2_rn(p[k].y0, wa, acc0[k]);
+        FB_EACH acc1[k] = __ffma2_rn(p[k].b2, wa, acc1[k]);
+        FB_EACH acc0[k] = __ffma2_rn(p[k].a1, wb, acc0[k]);
+        FB_EACH acc1[k] = __ffma2_rn(p[k].y3, wb, acc1[k]);
+        FB_EACH {
+          o0 = __ffma2_rn(p[k].a2, nwbt[k], __ffma2_rn(p[k].y0, wat[k], o0));
+          o1 = __ffma2_rn(p[k].b1, nwat[k], __ffma2_rn(p[k].y3, wbt[k], o1));
+        }
       }
+      const int up = (hl + 1) & (W - 1);
+      o0.x = __shfl_sync(mask, o0.x, up, W);
+      o0.y = __shfl_sync(mask, o0.y, up, W);
+      o1.x = __shfl_sync(mask, o1.x, up, W);
+      o1.y = __shfl_sync(mask, o1.y, up, W);
+    }
+    // after W/2 steps the second source's sums are home, the first's half a turn away
+    const float s0 = o0.y + __shfl_xor_sync(mask, o0.x, W / 2), s1 = o1.y + __shfl_xor_sync(mask, o1.x, W / 2);
+    if (j < tc) scrT[j] = make_float2(prev.x + s0, prev.y + s1);
   }
-  if (!valid || sub != 0) return;
-  double e0 = 0.0, e1 = 0.0;
-  special_sums(X, n, spOff, spSrc, spK, sgm, e0, e1);
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    const int t = r0 + k * W + hl;
+    const float v1 = acc1[k].x + acc1[k].y;
+    if (t < r1) scrR[t] = make_float2(acc0[k].x + acc0[k].y, ADJ ? -v1 : v1);
+  }
+}
+
+template <bool ADJ, int W>
+__device__ __forceinline__ void near_sym_task(const NearTask tk, float4 *Q, const int *__restrict__ leafStart,
+                                              const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
+                                              const float4 *__restrict__ recA, const float4 *__restrict__ recB,
+                                              const NearConstF &K, float2 *scr) {
+  const int hl = threadIdx.x % W;
+  const unsigned mask = W == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16);
+  const int rb = leafStart[tk.R], tb = leafStart[tk.T], tc = leafCount[tk.T];
+  const float sx = (float)(leafCtr[3 * tk.R] - leafCtr[3 * tk.T]);
+  const float sy = (float)(leafCtr[3 * tk.R + 1] - leafCtr[3 * tk.T + 1]);
+  const float sz = (float)(leafCtr[3 * tk.R + 2] - leafCtr[3 * tk.T + 2]);
+  float2 *scrR = scr + tk.scrR, *scrT = scr + tk.scrT;
+  int r0 = tk.r0;
+  for (; r0 + W < tk.r1; r0 += 2 * W)
+    near_sym_group<ADJ, W, 2>(Q, mask, hl, r0, tk.r1, rb, tb, tc, sx, sy, sz, r0 == tk.r0, recA, recB, K, scrR, scrT);
+  if (r0 < tk.r1)
+    near_sym_group<ADJ, W, 1>(Q, mask, hl, r0, tk.r1, rb, tb, tc, sx, sy, sz, r0 == tk.r0, recA, recB, K, scrR, scrT);
+}
+
+// one launch: the first blocks take the warp tasks, the rest the half-warp ones
+template <bool ADJ>
+__global__ void __launch_bounds__(kSymWarps * 32, FB_NEAR_SYM_MIN_BLOCKS)
+near_sym_f2_kernel(int n32, int nTasks, const NearTask *__restrict__ tasks, const int *__restrict__ leafStart,
+                   const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
+                   const float4 *__restrict__ recA, const float4 *__restrict__ recB, NearConstF K, float2 *scr) {
+  __shared__ float4 sQ[kSymWarps * 32 * 4];
+  const int blocks32 = (n32 + kSymWarps - 1) / kSymWarps;
+  if ((int)blockIdx.x < blocks32) {
+    const int warp = threadIdx.x >> 5, task = blockIdx.x * kSymWarps + warp;
+    if (task < n32)   // warp-uniform
+      near_sym_task<ADJ, 32>(tasks[task], sQ + warp * 128, leafStart, leafCount, leafCtr, recA, recB, K, scr);
+  } else {
+    const int half = threadIdx.x >> 4, task = n32 + ((int)blockIdx.x - blocks32) * 2 * kSymWarps + half;
+    if (task < nTasks)   // uniform over the half-warp
+      near_sym_task<ADJ, 16>(tasks[task], sQ + half * 64, leafStart, leafCount, leafCtr, recA, recB, K, scr);
+  }
+}
+
+// The same symmetric scheme in FP64 scalar arithmetic: lane t takes source
+// (t + s) mod 32 in step s of 32.
+template <bool ADJ>
+__global__ void __launch_bounds__(kSymWarps * 32, 2)
+near_sym_kernel(int nTasks, const NearTask *__restrict__ tasks, const int *__restrict__ leafStart,
+                const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
+                const double4 *__restrict__ recA, const double4 *__restrict__ recB, NearConstD K, double2 *scr) {
+  __shared__ double4 sA[kSymWarps][32], sB[kSymWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * kSymWarps + warp;
+  if (task >= nTasks) return;  // warp-uniform
+  const NearTask tk = tasks[task];
+  const int rb = leafStart[tk.R], tb = leafStart[tk.T], tc = leafCount[tk.T];
+  const double sx = leafCtr[3 * tk.R] - leafCtr[3 * tk.T];
+  const double sy = leafCtr[3 * tk.R + 1] - leafCtr[3 * tk.T + 1];
+  const double sz = leafCtr[3 * tk.R + 2] - leafCtr[3 * tk.T + 2];
+  double2 *scrR = scr + tk.scrR, *scrT = scr + tk.scrT;
+  for (int g0 = tk.r0; g0 < tk.r1; g0 += 32) {
+    const int t = g0 + lane;
+    const bool valid = t < tk.r1;
+    // a lane past the end: far away, zero weights
+    const double4 a = valid ? recA[rb + t] : make_double4(1e4, 1e4, 1e4, 0.0);
+    const double4 b = valid ? recB[rb + t] : make_double4(0.0, 0.0, 1.0, 0.0);
+    const double tx = a.x + sx, ty = a.y + sy, tz = a.z + sz;
+    double acc0 = 0.0, acc1 = 0.0;
+    for (int j0 = 0; j0 < tc; j0 += 32) {
+      const int j = j0 + lane;
+      const double4 pa = j < tc ? recA[tb + j] : make_double4(-1e4, -1e4, -1e4, 0.0);
+      const double4 pb = j < tc ? recB[tb + j] : make_double4(0.0, 0.0, 1.0, 0.0);
+      __syncwarp();
+      sA[warp][lane] = pa;
+      sB[warp][lane] = pb;
+      __syncwarp();
+      double own0 = 0.0, own1 = 0.0;
+#pragma unroll 2
+      for (int st = 0; st < 32; st++) {
+        const int q = (lane + st) & 31;
+        const double4 A = sA[warp][q], B = sB[warp][q];
+        const double dx = tx - A.x, dy = ty - A.y, dz = tz - A.z;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const double g = rsqrt(r2);   // distinct leaves: r > 0
+        const double r = r2 * g;
+        const double e = exp(K.kexp * r);
+        const double g2 = g * g, h = g2 * g, he = h * e, hc = he * (K.kappa * r + 1.0);
+        const double H1 = hc - h, F = K.eps * hc - h, Fi = K.ieps * hc - h;
+        const double ipX = b.x * dx + b.y * dy + b.z * dz;
+        const double ipY = B.x * dx + B.y * dy + B.z * dz;
+        const double ip0 = b.x * B.x + b.y * B.y + b.z * B.z;
+        const double y0 = g - g * e;
+        const double y3 = ip0 * H1 - ipX * ipY * (3.0 * (g2 * H1) + K.kap2 * he);
+        const double a1 = ipY * F, a2 = ipX * F, b1 = ipY * Fi, b2 = ipX * Fi;
+        double s0, s1;
+        if (ADJ) {
+          acc0 += y3 * A.w - a2 * B.w;
+          acc1 += y0 * B.w - b1 * A.w;
+          s0 = y3 * a.w + a1 * b.w;
+          s1 = y0 * b.w + b2 * a.w;
+        } else {
+          acc0 += y0 * A.w + a1 * B.w;
+          acc1 += b2 * A.w + y3 * B.w;
+          s0 = y0 * a.w - a2 * b.w;
+          s1 = y3 * b.w - b1 * a.w;
+        }
+        const int from = (lane - st) & 31;   // the lane whose source this step is this lane's
+        own0 += __shfl_sync(0xffffffffu, s0, from);
+        own1 += __shfl_sync(0xffffffffu, s1, from);
+      }
+      if (j < tc) {
+        const double2 prev = g0 == tk.r0 ? make_double2(0.0, 0.0) : scrT[j];
+        scrT[j] = make_double2(prev.x + own0, prev.y + own1);
+      }
+    }
+    if (valid) scrR[t] = make_double2(acc0, acc1);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The finishing kernel: the pairs that the symmetric tasks leave out (each
+// leaf with itself, pairs with a leaf of a few panels, every pair when there
+// are no tasks), the tasks' scratch sums, and the special pairs in FP64.
+//
+// A block of four warps takes up to 32 target panels of one leaf (one target
+// per lane; a short group of mt targets gives each target 32/mt lanes).  The
+// warps share all three sums -- whole source leaves when there are several,
+// else equal parts of the leaf's panels; every fourth scratch slot and special
+// pair -- and the partial sums are added in a fixed order.  The kernel is a
+// chain of dependent loads per target, which four warps shorten (one warp per
+// group took 23.4 us for 20,480 panels, four take 12.5).
+// ---------------------------------------------------------------------------
+// this lane's share (every step-th slot from first) of the scratch sums of panel xo of the leaf
+template <typename P, typename S>
+__device__ __forceinline__ void near_gather(int g0, int g1, int first, int step, int xo,
+                                            const int *__restrict__ slot, const P *__restrict__ scr, S &a0, S &a1) {
+#pragma unroll 4
+  for (int i = g0 + first; i < g1; i += step) {
+    const P v = scr[(size_t)slot[i] + xo];
+    a0 += v.x;
+    a1 += v.y;
+  }
+}
+
+// this lane's share of the FP64 special-pair corrections of target X
+__device__ __forceinline__ void special_sums(int X, int n, int first, int step, const int *__restrict__ spOff,
+                                             const int *__restrict__ spSrc, const double4 *__restrict__ spK,
+                                             const double *__restrict__ sgm, double &e0, double &e1) {
+  const int end = spOff[X + 1];
+#pragma unroll 4
+  for (int e = spOff[X] + first; e < end; e += step) {
+    const int Y = spSrc[e];
+    const double4 d = spK[e];
+    const double sp = sgm[Y], sd = sgm[n + Y];
+    e0 += d.x * sd + d.y * sp;
+    e1 += d.z * sd + d.w * sp;
+  }
+}
+
+// adds the warps' and lanes' partial sums; thread t < mt of the block returns with target t's
+struct NearPartial {
+  double s0, s1, e0, e1;
+};
+__device__ __forceinline__ NearPartial near_partials(NearPartial p, int mt, int k) {
+  __shared__ NearPartial red[kNearWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  red[warp][lane] = p;
+  __syncthreads();
+  NearPartial t{0.0, 0.0, 0.0, 0.0};
+  if ((int)threadIdx.x < mt)
+    for (int w = 0; w < kNearWarps; w++)
+      for (int i = 0; i < k; i++) {
+        const NearPartial v = red[w][threadIdx.x * k + i];
+        t.s0 += v.s0;
+        t.s1 += v.s1;
+        t.e0 += v.e0;
+        t.e1 += v.e1;
+      }
+  return t;
+}
+
+// this warp's share of source leaf S: all of it when the leaves are dealt over the warps, else a quarter
+__device__ __forceinline__ void near_share(int warp, bool byLeaf, int cnt, int &j0, int &j1) {
+  j0 = 0;
+  j1 = cnt;
+  if (!byLeaf) {
+    const int part = ((cnt + kNearWarps - 1) / kNearWarps + 1) & ~1;
+    j0 = min(cnt, warp * part);
+    j1 = min(cnt, j0 + part);
+  }
+}
+
+__device__ __forceinline__ void near_store(int X, int n, const NearPartial t, const double *__restrict__ area,
+                                           double coef, int accumulate, double *out) {
   const double AX = area[X] * kFourPiI;
-  const double v0 = coef * (AX * (double)acc0 + e0), v1 = coef * (AX * (double)acc1 + e1);
+  const double v0 = coef * (AX * t.s0 + t.e0), v1 = coef * (AX * t.s1 + t.e1);
   out[X] = accumulate ? out[X] + v0 : v0;   // each output has exactly one writer
   out[X + n] = accumulate ? out[X + n] + v1 : v1;
 }
 
-// ---------------------------------------------------------------------------
-// FP32 near field with packed f32x2 arithmetic (sm_100 FFMA2/FMUL2/FADD2):
-// every lane evaluates two sources per step, so the issue slots per pair
-// drop by about half while the FP32 work stays the same.  A tile of 32
-// sources is staged as 16 source pairs, each as four float4
-// (-x0 -x1 -y0 -y1 | -z0 -z1 wa0 wa1 | nx0 nx1 ny0 ny1 | nz0 nz1 wb0 wb1),
-// so the packed operands come straight from the loads; an odd source count
-// is padded with a zero-weight source far away.  Same tasks, lane split,
-// pair formula (near_pair) and FP64 epilogue as near_apply_kernel.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-
-// m = w n_s is the source normal multiplied by the weight of the terms it
-// enters: wb in the forward block (y1 wb = t1(m) (eps c - 1), y3 wb = dd(m)
-// (c - 1) - kap2 e u(m)), wa in the transposed one; so those terms need no
-// weight multiply.  SELF (the target's own leaf, the only tile holding the
-// coincident pair d = 0): 1/r is taken as 0 there, which zeroes every term.
-template <bool ADJ, bool SELF>
-__device__ __forceinline__ void near_pair2(const float4 A, const float4 B, const float4 C, const float4 D, float2 tx,
-                                           float2 ty, float2 tz, float2 tnx, float2 tny, float2 tnz, float kappa,
-                                           float kexp, float eps, float ieps, float kap2, float2 &acc0,
-                                           float2 &acc1) {
-  const float2 one = f2(1.f), m1 = f2(-1.f);
-  const float2 dx = __fadd2_rn(tx, make_float2(A.x, A.y));
-  const float2 dy = __fadd2_rn(ty, make_float2(A.z, A.w));
-  const float2 dz = __fadd2_rn(tz, make_float2(B.x, B.y));
-  const float2 wa = make_float2(B.z, B.w), wb = make_float2(D.z, D.w);
-  const float2 mx = make_float2(C.x, C.y), my = make_float2(C.z, C.w), mz = make_float2(D.x, D.y);
-  const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-  float2 g;
-  if (SELF) {
-    g.x = r2.x > 0.f ? rsqrt_t(r2.x) : 0.f;
-    g.y = r2.y > 0.f ? rsqrt_t(r2.y) : 0.f;
-  } else {   // distinct leaves: distinct panel centroids, r > 0
-    g.x = rsqrt_t(r2.x);
-    g.y = rsqrt_t(r2.y);
-  }
-  const float2 r = __fmul2_rn(r2, g);
-  const float2 ea = __fmul2_rn(f2(kexp), r);
-  float2 e;
-  e.x = expneg_t(1.f, ea.x);
-  e.y = expneg_t(1.f, ea.y);
-  const float2 c = __fmul2_rn(__ffma2_rn(f2(kappa), r, one), e);    // (kappa r + 1) e^{-kappa r}
-  const float2 g2 = __fmul2_rn(g, g), h = __fmul2_rn(g2, g);
-  const float2 ipX = __ffma2_rn(tnz, dz, __ffma2_rn(tny, dy, __fmul2_rn(tnx, dx)));
-  const float2 ipY = __ffma2_rn(mz, dz, __ffma2_rn(my, dy, __fmul2_rn(mx, dx)));     // w n_s.d
-  const float2 ip0 = __ffma2_rn(tnz, mz, __ffma2_rn(tny, my, __fmul2_rn(tnx, mx)));  // w n_t.n_s
-  const float2 t1 = __fmul2_rn(ipY, h), t2 = __fmul2_rn(ipX, h), u = __fmul2_rn(ipX, t1);
-  const float2 y0 = __ffma2_rn(make_float2(-e.x, -e.y), g, g);                       // G0 - Gk
-  const float2 dd = __fmul2_rn(__ffma2_rn(u, f2(-3.f), __fmul2_rn(ip0, g)), g2);     // w d2 G0
-  const float2 cm1 = __fadd2_rn(c, m1);
-  const float2 ke = __fmul2_rn(f2(-kap2), e);
-  if (ADJ) {
-    // out_pot += y3 wa - t2 (eps c - 1) wb, out_dpdn += y0 wb - t1 (c/eps - 1) wa
-    acc0 = __ffma2_rn(dd, cm1, acc0);
-    acc0 = __ffma2_rn(ke, u, acc0);
-    acc0 = __ffma2_rn(__fmul2_rn(t2, __ffma2_rn(f2(-eps), c, one)), wb, acc0);
-    acc1 = __ffma2_rn(y0, wb, acc1);
-    acc1 = __ffma2_rn(t1, __ffma2_rn(f2(-ieps), c, one), acc1);
-  } else {
-    // out_pot += y0 wa + y1 wb, out_dpdn += y2 wa + y3 wb
-    acc0 = __ffma2_rn(y0, wa, acc0);
-    acc0 = __ffma2_rn(t1, __ffma2_rn(f2(eps), c, m1), acc0);
-    acc1 = __ffma2_rn(__fmul2_rn(t2, __ffma2_rn(f2(ieps), c, m1)), wa, acc1);
-    acc1 = __ffma2_rn(dd, cm1, acc1);
-    acc1 = __ffma2_rn(ke, u, acc1);
-  }
-}
-
-// one staged tile of up to 32 sources (np packed source pairs) for a target
-#ifndef FB_NEAR_UNROLL
-#define FB_NEAR_UNROLL 4
-#endif
-constexpr int kNearUnroll = FB_NEAR_UNROLL;
-template <bool ADJ, bool SELF>
-__device__ __forceinline__ void near_tile2(const float4 (*sP)[4], int np, int k, int sub, float2 tx, float2 ty,
-                                           float2 tz, float2 tnx, float2 tny, float2 tnz, float kappa, float kexp,
-                                           float eps, float ieps, float kap2, float2 &acc0, float2 &acc1) {
-  if (k == 1) {   // warp-uniform: a full group
-#pragma unroll kNearUnroll
-    for (int q = 0; q < np; q++)
-      near_pair2<ADJ, SELF>(sP[q][0], sP[q][1], sP[q][2], sP[q][3], tx, ty, tz, tnx, tny, tnz, kappa, kexp, eps,
-                            ieps, kap2, acc0, acc1);
-  } else {
-#pragma unroll kNearUnroll
-    for (int q = sub; q < np; q += k)
-      near_pair2<ADJ, SELF>(sP[q][0], sP[q][1], sP[q][2], sP[q][3], tx, ty, tz, tnx, tny, tnz, kappa, kexp, eps,
-                            ieps, kap2, acc0, acc1);
-  }
-}
-
 template <bool ADJ>
-__global__ void __launch_bounds__(kNearWarps * 32, FB_NEAR_MIN_BLOCKS)
-near_apply_f2_kernel(int nWork, const int2 *__restrict__ work, const int *__restrict__ leafStart,
-                     const int *__restrict__ leafCount, const int *__restrict__ nearOff,
-                     const int *__restrict__ nearSrc, const double *__restrict__ leafCtr,
+__global__ void __launch_bounds__(kNearWarps * 32)
+near_apply_f2_kernel(const int2 *__restrict__ work, const int *__restrict__ leafStart,
+                     const int *__restrict__ leafCount, const int *__restrict__ ordOff,
+                     const int *__restrict__ ordSrc, const double *__restrict__ leafCtr,
                      const float4 *__restrict__ tgtP, const float4 *__restrict__ tgtN,
-                     const float4 *__restrict__ srcA, const float4 *__restrict__ srcB,
                      const int *__restrict__ spOff, const int *__restrict__ spSrc, const double4 *__restrict__ spK,
-                     const double *__restrict__ sgm, const double *__restrict__ area, int n, float kappa, float kexp,
-                     float eps, float ieps, float kap2, double coef, int accumulate, double *out,
-                     const int *__restrict__ symOff, const float2 *__restrict__ symScr) {
+                     const double *__restrict__ sgm, const double *__restrict__ area, int n, NearConstF K,
+                     double coef, int accumulate, double *out, const int *__restrict__ gatOff,
+                     const int *__restrict__ gatSlot, const float2 *__restrict__ scr) {
   __shared__ float4 sP[kNearWarps][16][4];
-  __shared__ float sR[kNearWarps][2][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * kNearWarps + warp;
-  if (task >= nWork) return;  // warp-uniform
-  const int2 wk = work[task];
+  const int2 wk = work[blockIdx.x];
   const int L = wk.x;
   const int base = leafStart[L], cnt = leafCount[L];
   const int g0 = 32 * wk.y;
@@ -447,415 +590,107 @@ near_apply_f2_kernel(int nWork, const int2 *__restrict__ work, const int *__rest
   const bool valid = t < mt;
   const int X = base + g0 + (valid ? t : 0);
   const float4 tp = tgtP[X], tn = tgtN[X];
-  const float2 tnx = f2(tn.x), tny = f2(tn.y), tnz = f2(tn.z);
+  NearTargetsF2<1> tg;
+  tg.nx[0] = f2(tn.x); tg.ny[0] = f2(tn.y); tg.nz[0] = f2(tn.z);
   const double cx = leafCtr[3 * L], cy = leafCtr[3 * L + 1], cz = leafCtr[3 * L + 2];
   float2 acc0 = f2(0.f), acc1 = f2(0.f);
   float *pf = reinterpret_cast<float *>(&sP[warp][lane >> 1][0]) + (lane & 1);
-  const int pBeg = nearOff[L], p1 = nearOff[L + 1];
-  // the leaf pairs of the symmetric kernel: their sums for this target are in the scratch
-  if (symOff)
-    sym_scratch_sums<float>(pBeg, p1, lane, valid && sub == 0, X - base, symOff,
-                            reinterpret_cast<const float *>(symScr), acc0.x, acc1.x);
-  // the other near leaves
-  for (int p = pBeg; p < p1; p++) {
-    if (symOff && symOff[p] >= 0) continue;   // warp-uniform: summed above
-    const int S = nearSrc[p];
-    const int sb = leafStart[S], sc = leafCount[S];
-    const float2 tx = f2(tp.x + (float)(cx - leafCtr[3 * S]));
-    const float2 ty = f2(tp.y + (float)(cy - leafCtr[3 * S + 1]));
-    const float2 tz = f2(tp.z + (float)(cz - leafCtr[3 * S + 2]));
-    for (int j0 = 0; j0 < sc; j0 += 32) {
-      const int m = min(32, sc - j0);
-      float4 a = make_float4(-1e4f, -1e4f, -1e4f, 0.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int p1 = ordOff[L + 1], p0 = ordOff[L];
+  const bool byLeaf = p1 - p0 >= kNearWarps;
+  for (int p = p0 + (byLeaf ? warp : 0); p < p1; p += byLeaf ? kNearWarps : 1) {
+    const int S = ordSrc[p], sb = leafStart[S];
+    int jb, je;
+    near_share(warp, byLeaf, leafCount[S], jb, je);
+    tg.x[0] = f2(tp.x + (float)(cx - leafCtr[3 * S]));
+    tg.y[0] = f2(tp.y + (float)(cy - leafCtr[3 * S + 1]));
+    tg.z[0] = f2(tp.z + (float)(cz - leafCtr[3 * S + 2]));
+    for (int j0 = jb; j0 < je; j0 += 32) {
+      const int m = min(32, je - j0);
+      float4 a = make_float4(1e4f, 1e4f, 1e4f, 0.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
       if (lane < m) {
-        a = srcA[sb + j0 + lane];
-        b = srcB[sb + j0 + lane];
+        near_record<float>(sb + j0 + lane, n, tgtP, tgtN, area, sgm, a, b);
       }
       pf[0] = -a.x; pf[2] = -a.y; pf[4] = -a.z; pf[6] = a.w;
-      pf[8] = b.x; pf[10] = b.y; pf[12] = b.z; pf[14] = b.w;
+      pf[8] = b.x; pf[10] = b.y; pf[12] = b.z; pf[14] = ADJ ? -b.w : b.w;
       __syncwarp();
       const int np = (m + 1) >> 1;
-      if (S == L)   // warp-uniform
-        near_tile2<ADJ, true>(sP[warp], np, k, sub, tx, ty, tz, tnx, tny, tnz, kappa, kexp, eps, ieps, kap2, acc0,
-                              acc1);
-      else
-        near_tile2<ADJ, false>(sP[warp], np, k, sub, tx, ty, tz, tnx, tny, tnz, kappa, kexp, eps, ieps, kap2, acc0,
-                               acc1);
-      __syncwarp();
-    }
-  }
-  float s0 = acc0.x + acc0.y, s1 = acc1.x + acc1.y;
-  if (k > 1) {   // warp-uniform: add the k partial sums of each target
-    sR[warp][0][lane] = s0;
-    sR[warp][1][lane] = s1;
-    __syncwarp();
-    if (valid && sub == 0)
-      for (int i = 1; i < k; i++) {
-        s0 += sR[warp][0][lane + i];
-        s1 += sR[warp][1][lane + i];
-      }
-  }
-  if (!valid || sub != 0) return;
-  double e0 = 0.0, e1 = 0.0;
-  special_sums(X, n, spOff, spSrc, spK, sgm, e0, e1);
-  const double AX = area[X] * kFourPiI;
-  const double v0 = coef * (AX * (double)s0 + e0), v1 = coef * (AX * (double)s1 + e1);
-  out[X] = accumulate ? out[X] + v0 : v0;   // each output has exactly one writer
-  out[X + n] = accumulate ? out[X + n] + v1 : v1;
-}
-
-// ---------------------------------------------------------------------------
-// Symmetric near field (FP32, packed f32x2; mixed contexts; forward and transposed operator).
-// The one-point pair term of K(X, Y) and that of K(Y, X) share r, 1/r,
-// e^{-kappa r}, (kappa r + 1) e^{-kappa r}, n_X.n_Y and the double-layer
-// factors; with d = x_X - x_Y, swapping the panels negates d, so
-//   t1(Y,X) = -t2(X,Y),  t2(Y,X) = -t1(X,Y),  u, dd, y0, y3 unchanged,
-//   K(Y,X): out_pot  += y0 wa_X - t2 (eps c - 1) wb_X,
-//           out_dpdn += -t1 (c/eps - 1) wa_X + y3 wb_X.
-// So every unordered pair of distinct near leaves (R, T) is evaluated once
-// for both directions.  One warp per leaf pair: the 32-panel groups of R in
-// registers (lane = target), T in tiles of 32 staged in shared memory.  In
-// step s of a tile, lane t takes the tile's sources (t + s) and (t + s + 16)
-// (mod 32), so at every step the 32 lanes hold 32 distinct sources and each
-// source's contribution from the lane's target goes to the lane that owns that
-// source by two shuffles; after 16 steps every source has had all 32 targets.
-// The sums go to a scratch slot per (ordered leaf pair, panel); the ordered
-// near-field kernel adds them, in its near-list order, to its own FP32 sums
-// (deterministic: no atomics).  Self pairs and pairs with a small leaf stay in
-// the ordered kernel.  ADJ: the transposed operator, with the transposed
-// blocks of the two directions (near_pair's ADJ terms and their swap).
-// ---------------------------------------------------------------------------
-#ifndef FB_NEAR_SYM_MIN_BLOCKS
-#define FB_NEAR_SYM_MIN_BLOCKS 6
-#endif
-// leaf pairs whose smaller leaf has fewer panels go to the half-warp kernel (mixed
-// contexts, down to FB_NEAR_SYM16_MIN_LEAF panels; larger pairs too where its
-// padding saves more than its overhead) or stay in the ordered kernel (FP64)
-#ifndef FB_NEAR_SYM_MIN_LEAF
-#define FB_NEAR_SYM_MIN_LEAF 48
-#endif
-#ifndef FB_NEAR_SYM16_MIN_LEAF
-#define FB_NEAR_SYM16_MIN_LEAF 4
-#endif
-#ifndef FB_NEAR_SYM16_COST
-#define FB_NEAR_SYM16_COST 125
-#endif
-#ifndef FB_NEAR_SYM_UNROLL
-#define FB_NEAR_SYM_UNROLL 4
-#endif
-constexpr int kSymUnroll = FB_NEAR_SYM_UNROLL;
-constexpr int kSymWarps = 4;
-
-template <bool ADJ>
-__device__ __forceinline__ void near_sym_pair2(const float4 A, const float4 B, const float4 C, const float4 D,
-                                               float2 tx, float2 ty, float2 tz, float2 tnx, float2 tny, float2 tnz,
-                                               float2 wat, float2 wbt, float2 watn, float2 wbtn, float kappa,
-                                               float kexp, float eps, float ieps, float kap2, float2 &acc0,
-                                               float2 &acc1, float2 &s0, float2 &s1) {
-  const float2 one = f2(1.f), m1 = f2(-1.f);
-  const float2 dx = __fadd2_rn(tx, make_float2(A.x, A.y));
-  const float2 dy = __fadd2_rn(ty, make_float2(A.z, A.w));
-  const float2 dz = __fadd2_rn(tz, make_float2(B.x, B.y));
-  const float2 wa = make_float2(B.z, B.w), wb = make_float2(D.z, D.w);
-  const float2 nx = make_float2(C.x, C.y), ny = make_float2(C.z, C.w), nz = make_float2(D.x, D.y);
-  const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-  float2 g;   // distinct leaves: distinct panel centroids, r > 0
-  g.x = rsqrt_t(r2.x);
-  g.y = rsqrt_t(r2.y);
-  const float2 r = __fmul2_rn(r2, g);
-  const float2 ea = __fmul2_rn(f2(kexp), r);
-  float2 e;
-  e.x = expneg_t(1.f, ea.x);
-  e.y = expneg_t(1.f, ea.y);
-  const float2 c = __fmul2_rn(__ffma2_rn(f2(kappa), r, one), e);    // (kappa r + 1) e^{-kappa r}
-  const float2 g2 = __fmul2_rn(g, g), h = __fmul2_rn(g2, g);
-  const float2 ipX = __ffma2_rn(tnz, dz, __ffma2_rn(tny, dy, __fmul2_rn(tnx, dx)));   // n_X.d
-  const float2 ipY = __ffma2_rn(nz, dz, __ffma2_rn(ny, dy, __fmul2_rn(nx, dx)));      // n_Y.d
-  const float2 ip0 = __ffma2_rn(tnz, nz, __ffma2_rn(tny, ny, __fmul2_rn(tnx, nx)));   // n_X.n_Y
-  const float2 t1 = __fmul2_rn(ipY, h), t2 = __fmul2_rn(ipX, h), u = __fmul2_rn(ipX, t1);
-  const float2 y0 = __ffma2_rn(make_float2(-e.x, -e.y), g, g);                       // G0 - Gk
-  const float2 dd = __fmul2_rn(__ffma2_rn(u, f2(-3.f), __fmul2_rn(ip0, g)), g2);     // d2 G0
-  const float2 y3 = __ffma2_rn(dd, __fadd2_rn(c, m1), __fmul2_rn(__fmul2_rn(f2(-kap2), e), u));
-  const float2 fe = __ffma2_rn(f2(eps), c, m1), fi = __ffma2_rn(f2(ieps), c, m1);    // eps c - 1, c/eps - 1
-  const float2 t1fe = __fmul2_rn(t1, fe), t2fi = __fmul2_rn(t2, fi);
-  const float2 t2fe = __fmul2_rn(t2, fe), t1fi = __fmul2_rn(t1, fi);
-  if (ADJ) {
-    // the transposed blocks (near_pair's ADJ terms): K(Y,X)^T to the target X, K(X,Y)^T to the sources
-    acc0 = __ffma2_rn(y3, wa, acc0);
-    acc0 = __ffma2_rn(make_float2(-t2fe.x, -t2fe.y), wb, acc0);
-    acc1 = __ffma2_rn(y0, wb, acc1);
-    acc1 = __ffma2_rn(make_float2(-t1fi.x, -t1fi.y), wa, acc1);
-    s0 = __ffma2_rn(t1fe, wbt, __fmul2_rn(y3, wat));
-    s1 = __ffma2_rn(t2fi, wat, __fmul2_rn(y0, wbt));
-  } else {
-    // K(X, Y): the target X of this lane, sources Y
-    acc0 = __ffma2_rn(y0, wa, acc0);
-    acc0 = __ffma2_rn(t1fe, wb, acc0);
-    acc1 = __ffma2_rn(t2fi, wa, acc1);
-    acc1 = __ffma2_rn(y3, wb, acc1);
-    // K(Y, X): the two sources as targets of this lane's panel
-    s0 = __ffma2_rn(t2fe, wbtn, __fmul2_rn(y0, wat));
-    s1 = __ffma2_rn(t1fi, watn, __fmul2_rn(y3, wbt));
-  }
-}
-
-template <bool ADJ>
-__global__ void __launch_bounds__(kSymWarps * 32, FB_NEAR_SYM_MIN_BLOCKS)
-near_sym_f2_kernel(int nTasks, const int4 *__restrict__ tasks, const int *__restrict__ leafStart,
-                   const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
-                   const float4 *__restrict__ recA, const float4 *__restrict__ recB, float kappa, float kexp,
-                   float eps, float ieps, float kap2, float2 *scr) {
-  // per warp, component-major: sQ[k][m] holds component k of the tile's sources m and (m + 16) mod 32,
-  // interleaved (first, second, first, second), read by lane t at step s from slot (t + s) mod 32
-  __shared__ float4 sQ[kSymWarps][4][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * kSymWarps + warp;
-  if (task >= nTasks) return;  // warp-uniform
-  const int4 tk = tasks[task];
-  const int R = tk.x, T = tk.y;
-  const int rb = leafStart[R], rc = leafCount[R], tb = leafStart[T], tc = leafCount[T];
-  const float sx = (float)(leafCtr[3 * R] - leafCtr[3 * T]);
-  const float sy = (float)(leafCtr[3 * R + 1] - leafCtr[3 * T + 1]);
-  const float sz = (float)(leafCtr[3 * R + 2] - leafCtr[3 * T + 2]);
-  float4(*Q)[32] = sQ[warp];
-  for (int g0 = 0; g0 < rc; g0 += 32) {
-    const int t = g0 + lane;
-    const bool valid = t < rc;
-    // a lane past the group's end: far away, zero weights (its terms vanish, its sums are dropped)
-    const float4 a = valid ? recA[rb + t] : make_float4(1e4f, 1e4f, 1e4f, 0.f);
-    const float4 b = valid ? recB[rb + t] : make_float4(0.f, 0.f, 1.f, 0.f);
-    const float2 tx = f2(a.x + sx), ty = f2(a.y + sy), tz = f2(a.z + sz);
-    const float2 tnx = f2(b.x), tny = f2(b.y), tnz = f2(b.z);
-    const float2 wat = f2(a.w), wbt = f2(b.w), watn = f2(-a.w), wbtn = f2(-b.w);
-    float2 acc0 = f2(0.f), acc1 = f2(0.f);
-    for (int j0 = 0; j0 < tc; j0 += 32) {
-      const int m = min(32, tc - j0);
-      // stage the tile: source j0+lane, or a padding source far away with zero weights
-      float4 sa = make_float4(-1e4f, -1e4f, -1e4f, 0.f), sb = make_float4(0.f, 0.f, 1.f, 0.f);
-      if (lane < m) {
-        sa = recA[tb + j0 + lane];
-        sb = recB[tb + j0 + lane];
-      }
-      // slot m holds source m first and source m + 16 (mod 32, the lane m ^ 16) second
-      const float ox = __shfl_xor_sync(0xffffffffu, sa.x, 16), oy = __shfl_xor_sync(0xffffffffu, sa.y, 16);
-      const float oz = __shfl_xor_sync(0xffffffffu, sa.z, 16), ow = __shfl_xor_sync(0xffffffffu, sa.w, 16);
-      const float px = __shfl_xor_sync(0xffffffffu, sb.x, 16), py = __shfl_xor_sync(0xffffffffu, sb.y, 16);
-      const float pz = __shfl_xor_sync(0xffffffffu, sb.z, 16), pw = __shfl_xor_sync(0xffffffffu, sb.w, 16);
-      __syncwarp();   // the previous tile's reads are done
-      Q[0][lane] = make_float4(-sa.x, -ox, -sa.y, -oy);
-      Q[1][lane] = make_float4(-sa.z, -oz, sa.w, ow);
-      Q[2][lane] = make_float4(sb.x, px, sb.y, py);
-      Q[3][lane] = make_float4(sb.z, pz, sb.w, pw);
-      __syncwarp();
-      float2 own = f2(0.f);   // this lane's source j0+lane: (pot, dpdn) from the group's 32 targets
-#pragma unroll kSymUnroll
-      for (int st = 0; st < 16; st++) {
-        const int slot = (lane + st) & 31;
-        float2 s0, s1;
-        near_sym_pair2<ADJ>(Q[0][slot], Q[1][slot], Q[2][slot], Q[3][slot], tx, ty, tz, tnx, tny, tnz, wat, wbt,
-                            watn, wbtn, kappa, kexp, eps, ieps, kap2, acc0, acc1, s0, s1);
-        // this lane's source was the first source of lane (lane - st) and the second of lane (lane - st - 16)
-        const int l1 = (lane - st) & 31, l2 = (lane - st - 16) & 31;
-        const float a0 = __shfl_sync(0xffffffffu, s0.x, l1), a1 = __shfl_sync(0xffffffffu, s1.x, l1);
-        const float b0 = __shfl_sync(0xffffffffu, s0.y, l2), b1 = __shfl_sync(0xffffffffu, s1.y, l2);
-        own = __fadd2_rn(own, __fadd2_rn(make_float2(a0, a1), make_float2(b0, b1)));
-      }
-      if (lane < m) {   // the tile side's slot: written by the first group, added to by the next
-        float2 *q = scr + tk.w + j0 + lane;
-        const float2 prev = g0 == 0 ? f2(0.f) : *q;
-        *q = __fadd2_rn(prev, own);
-      }
-    }
-    if (valid) scr[tk.z + t] = make_float2(acc0.x + acc0.y, acc1.x + acc1.y);
-  }
-}
-
-// The symmetric scheme for leaf pairs that pad badly into 32-panel groups
-// (mixed contexts; every pair whose smaller leaf has fewer than
-// FB_NEAR_SYM_MIN_LEAF panels, and larger ones where 16-panel padding saves
-// more than this kernel's per-tile overhead): each half-warp takes its own
-// leaf pair with 16-panel groups and 16-source tiles, so a pair of 46-panel
-// leaves fills 92% of the lanes instead of the 52% of 32-wide tiles.  In step
-// s of a tile, lane t of the half takes sources (t + s) and (t + s + 8)
-// (mod 16); after 8 steps every source has had all 16 targets.  Shuffles and
-// warp barriers take the half's lane mask, so the two halves may run
-// different trip counts.
-template <bool ADJ>
-__global__ void __launch_bounds__(kSymWarps * 32, FB_NEAR_SYM_MIN_BLOCKS)
-near_sym16_f2_kernel(int nTasks, const int4 *__restrict__ tasks, const int *__restrict__ leafStart,
-                     const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
-                     const float4 *__restrict__ recA, const float4 *__restrict__ recB, float kappa, float kexp,
-                     float eps, float ieps, float kap2, float2 *scr) {
-  __shared__ float4 sQ[kSymWarps][2][4][16];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
-  const unsigned hm = 0xffffu << (16 * half);
-  const int task = (blockIdx.x * kSymWarps + warp) * 2 + half;
-  if (task >= nTasks) return;  // uniform over the half
-  const int4 tk = tasks[task];
-  const int R = tk.x, T = tk.y;
-  const int rb = leafStart[R], rc = leafCount[R], tb = leafStart[T], tc = leafCount[T];
-  const float sx = (float)(leafCtr[3 * R] - leafCtr[3 * T]);
-  const float sy = (float)(leafCtr[3 * R + 1] - leafCtr[3 * T + 1]);
-  const float sz = (float)(leafCtr[3 * R + 2] - leafCtr[3 * T + 2]);
-  float4(*Q)[16] = sQ[warp][half];
-  for (int g0 = 0; g0 < rc; g0 += 16) {
-    const int t = g0 + hl;
-    const bool valid = t < rc;
-    // a lane past the group's end: far away, zero weights (its terms vanish, its sums are dropped)
-    const float4 a = valid ? recA[rb + t] : make_float4(1e4f, 1e4f, 1e4f, 0.f);
-    const float4 b = valid ? recB[rb + t] : make_float4(0.f, 0.f, 1.f, 0.f);
-    const float2 tx = f2(a.x + sx), ty = f2(a.y + sy), tz = f2(a.z + sz);
-    const float2 tnx = f2(b.x), tny = f2(b.y), tnz = f2(b.z);
-    const float2 wat = f2(a.w), wbt = f2(b.w), watn = f2(-a.w), wbtn = f2(-b.w);
-    float2 acc0 = f2(0.f), acc1 = f2(0.f);
-    // the tile's source j0+hl, or a padding source far away with zero weights; one tile ahead
-    float4 na = make_float4(-1e4f, -1e4f, -1e4f, 0.f), nb = make_float4(0.f, 0.f, 1.f, 0.f);
-    if (hl < tc) {
-      na = recA[tb + hl];
-      nb = recB[tb + hl];
-    }
-    for (int j0 = 0; j0 < tc; j0 += 16) {
-      const int m = min(16, tc - j0);
-      const float4 sa = na, sb = nb;
-      na = make_float4(-1e4f, -1e4f, -1e4f, 0.f);
-      nb = make_float4(0.f, 0.f, 1.f, 0.f);
-      if (j0 + 16 + hl < tc) {
-        na = recA[tb + j0 + 16 + hl];
-        nb = recB[tb + j0 + 16 + hl];
-      }
-      const int js = j0 + (hl < m ? hl : 0);
-      const float2 prev = hl < m && g0 > 0 ? scr[tk.w + js] : f2(0.f);
-      // slot m holds source m first and source m + 8 (mod 16, the lane m ^ 8) second
-      const float ox = __shfl_xor_sync(hm, sa.x, 8), oy = __shfl_xor_sync(hm, sa.y, 8);
-      const float oz = __shfl_xor_sync(hm, sa.z, 8), ow = __shfl_xor_sync(hm, sa.w, 8);
-      const float px = __shfl_xor_sync(hm, sb.x, 8), py = __shfl_xor_sync(hm, sb.y, 8);
-      const float pz = __shfl_xor_sync(hm, sb.z, 8), pw = __shfl_xor_sync(hm, sb.w, 8);
-      __syncwarp(hm);   // the previous tile's reads are done
-      Q[0][hl] = make_float4(-sa.x, -ox, -sa.y, -oy);
-      Q[1][hl] = make_float4(-sa.z, -oz, sa.w, ow);
-      Q[2][hl] = make_float4(sb.x, px, sb.y, py);
-      Q[3][hl] = make_float4(sb.z, pz, sb.w, pw);
-      __syncwarp(hm);
-      float2 own = f2(0.f);   // this lane's source j0+hl: (pot, dpdn) from the group's 16 targets
+      if (S == L) {   // warp-uniform
 #pragma unroll 4
-      for (int st = 0; st < 8; st++) {
-        const int slot = (hl + st) & 15;
-        float2 s0, s1;
-        near_sym_pair2<ADJ>(Q[0][slot], Q[1][slot], Q[2][slot], Q[3][slot], tx, ty, tz, tnx, tny, tnz, wat, wbt,
-                            watn, wbtn, kappa, kexp, eps, ieps, kap2, acc0, acc1, s0, s1);
-        // this lane's source was the first source of lane (hl - st) and the second of lane (hl - st - 8)
-        const int l1 = (hl - st) & 15, l2 = (hl - st - 8) & 15;
-        const float a0 = __shfl_sync(hm, s0.x, l1, 16), a1 = __shfl_sync(hm, s1.x, l1, 16);
-        const float b0 = __shfl_sync(hm, s0.y, l2, 16), b1 = __shfl_sync(hm, s1.y, l2, 16);
-        own = __fadd2_rn(own, __fadd2_rn(make_float2(a0, a1), make_float2(b0, b1)));
-      }
-      if (hl < m) scr[tk.w + js] = __fadd2_rn(prev, own);   // written by the first group, added to by the next
-    }
-    if (valid) scr[tk.z + t] = make_float2(acc0.x + acc0.y, acc1.x + acc1.y);
-  }
-}
-
-// The same symmetric scheme in scalar arithmetic (FP64 contexts): lane t
-// takes source (t + s) mod 32 in step s of 32; the source's term from the
-// lane's target goes to the owning lane by shuffle.
-template <typename T, bool ADJ>
-__device__ __forceinline__ void near_sym_pair(const typename Vec4<T>::t a, const typename Vec4<T>::t b, T tx, T ty,
-                                              T tz, T tnx, T tny, T tnz, T wat, T wbt, T kappa, T kexp, T eps,
-                                              T ieps, T kap2, T &acc0, T &acc1, T &s0, T &s1) {
-  const T dx = tx - a.x, dy = ty - a.y, dz = tz - a.z;
-  const T r2 = dx * dx + dy * dy + dz * dz;
-  const T g = rsqrt_t(r2);   // distinct leaves: r > 0
-  const T r = r2 * g;
-  const T e = expneg_t(kexp, r);
-  const T c = (kappa * r + (T)1) * e;
-  const T g2 = g * g, h = g2 * g;
-  const T ipX = tnx * dx + tny * dy + tnz * dz;
-  const T ipY = b.x * dx + b.y * dy + b.z * dz;
-  const T ip0 = tnx * b.x + tny * b.y + tnz * b.z;
-  const T t1 = ipY * h, t2 = ipX * h, u = ipX * t1;
-  const T y0 = g - g * e;
-  const T dd = (ip0 * g - (T)3 * u) * g2;
-  const T y3 = dd * (c - (T)1) - kap2 * e * u;
-  const T fe = eps * c - (T)1, fi = c * ieps - (T)1;
-  if (ADJ) {   // the transposed blocks, as near_pair's ADJ terms
-    acc0 += y3 * a.w - t2 * fe * b.w;
-    acc1 += y0 * b.w - t1 * fi * a.w;
-    s0 = y3 * wat + t1 * fe * wbt;
-    s1 = y0 * wbt + t2 * fi * wat;
-  } else {
-    acc0 += y0 * a.w + t1 * fe * b.w;
-    acc1 += t2 * fi * a.w + y3 * b.w;
-    s0 = y0 * wat - t2 * fe * wbt;
-    s1 = y3 * wbt - t1 * fi * wat;
-  }
-}
-
-template <typename T, bool ADJ>
-__global__ void __launch_bounds__(kSymWarps * 32, sizeof(T) == 8 ? 2 : FB_NEAR_SYM_MIN_BLOCKS)
-near_sym_kernel(int nTasks, const int4 *__restrict__ tasks, const int *__restrict__ leafStart,
-                const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
-                const typename Vec4<T>::t *__restrict__ recA, const typename Vec4<T>::t *__restrict__ recB, T kappa,
-                T kexp, T eps, T ieps, T kap2, T *scr) {
-  typedef typename Vec4<T>::t V;
-  __shared__ V sA[kSymWarps][32], sB[kSymWarps][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * kSymWarps + warp;
-  if (task >= nTasks) return;  // warp-uniform
-  const int4 tk = tasks[task];
-  const int R = tk.x, Tl = tk.y;
-  const int rb = leafStart[R], rc = leafCount[R], tb = leafStart[Tl], tc = leafCount[Tl];
-  const T sx = (T)(leafCtr[3 * R] - leafCtr[3 * Tl]);
-  const T sy = (T)(leafCtr[3 * R + 1] - leafCtr[3 * Tl + 1]);
-  const T sz = (T)(leafCtr[3 * R + 2] - leafCtr[3 * Tl + 2]);
-  for (int g0 = 0; g0 < rc; g0 += 32) {
-    const int t = g0 + lane;
-    const bool valid = t < rc;
-    V a, b;
-    if (valid) {
-      a = recA[rb + t];
-      b = recB[rb + t];
-    } else {   // far away, zero weights
-      a.x = a.y = a.z = (T)1e4; a.w = (T)0;
-      b.x = b.y = (T)0; b.z = (T)1; b.w = (T)0;
-    }
-    const T tx = a.x + sx, ty = a.y + sy, tz = a.z + sz;
-    T acc0 = (T)0, acc1 = (T)0;
-    for (int j0 = 0; j0 < tc; j0 += 32) {
-      const int m = min(32, tc - j0);
-      V pa, pb;
-      if (lane < m) {
-        pa = recA[tb + j0 + lane];
-        pb = recB[tb + j0 + lane];
+        for (int q = sub; q < np; q += k)
+          near_pair2<ADJ, true>(sP[warp][q][0], sP[warp][q][1], sP[warp][q][2], sP[warp][q][3], tg, K, acc0,
+                                acc1);
       } else {
-        pa.x = pa.y = pa.z = (T)-1e4; pa.w = (T)0;
-        pb.x = pb.y = (T)0; pb.z = (T)1; pb.w = (T)0;
+#pragma unroll 4
+        for (int q = sub; q < np; q += k)
+          near_pair2<ADJ, false>(sP[warp][q][0], sP[warp][q][1], sP[warp][q][2], sP[warp][q][3], tg, K, acc0,
+                                 acc1);
       }
       __syncwarp();
-      sA[warp][lane] = pa;
-      sB[warp][lane] = pb;
-      __syncwarp();
-      T own0 = (T)0, own1 = (T)0;
-#pragma unroll 2
-      for (int st = 0; st < 32; st++) {
-        const int j = (lane + st) & 31;
-        T s0, s1;
-        near_sym_pair<T, ADJ>(sA[warp][j], sB[warp][j], tx, ty, tz, b.x, b.y, b.z, a.w, b.w, kappa, kexp, eps, ieps,
-                              kap2, acc0, acc1, s0, s1);
-        const int from = (lane - st) & 31;   // the lane whose source this step is this lane's
-        own0 += __shfl_sync(0xffffffffu, s0, from);
-        own1 += __shfl_sync(0xffffffffu, s1, from);
-      }
-      if (lane < m) {
-        T *q = scr + 2 * (size_t)(tk.w + j0 + lane);
-        q[0] = (g0 == 0 ? (T)0 : q[0]) + own0;
-        q[1] = (g0 == 0 ? (T)0 : q[1]) + own1;
-      }
-    }
-    if (valid) {
-      scr[2 * (size_t)(tk.z + t)] = acc0;
-      scr[2 * (size_t)(tk.z + t) + 1] = acc1;
     }
   }
+  float s0 = acc0.x + acc0.y, s1 = ADJ ? -(acc1.x + acc1.y) : acc1.x + acc1.y;
+  NearPartial p{0.0, 0.0, 0.0, 0.0};
+  if (valid) {
+    const int first = warp * k + sub, step = kNearWarps * k;
+    if (gatOff) near_gather(gatOff[L], gatOff[L + 1], first, step, X - base, gatSlot, scr, s0, s1);
+    special_sums(X, n, first, step, spOff, spSrc, spK, sgm, p.e0, p.e1);
+  }
+  p.s0 = (double)s0;
+  p.s1 = (double)s1;
+  p = near_partials(p, mt, k);
+  if ((int)threadIdx.x < mt) near_store(base + g0 + threadIdx.x, n, p, area, coef, accumulate, out);
+}
+
+template <bool ADJ>
+__global__ void __launch_bounds__(kNearWarps * 32)
+near_apply_kernel(const int2 *__restrict__ work, const int *__restrict__ leafStart,
+                  const int *__restrict__ leafCount, const int *__restrict__ ordOff,
+                  const int *__restrict__ ordSrc, const double *__restrict__ leafCtr,
+                  const double4 *__restrict__ tgtP, const double4 *__restrict__ tgtN,
+                  const int *__restrict__ spOff, const int *__restrict__ spSrc, const double4 *__restrict__ spK,
+                  const double *__restrict__ sgm, const double *__restrict__ area, int n, NearConstD K, double coef,
+                  int accumulate, double *out, const int *__restrict__ gatOff, const int *__restrict__ gatSlot,
+                  const double2 *__restrict__ scr) {
+  __shared__ double4 sA[kNearWarps][32], sB[kNearWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int2 wk = work[blockIdx.x];
+  const int L = wk.x;
+  const int base = leafStart[L], cnt = leafCount[L];
+  const int g0 = 32 * wk.y;
+  const int mt = min(32, cnt - g0);   // targets in this group
+  const int k = 32 / mt;              // lanes per target
+  const int t = lane / k, sub = lane - t * k;
+  const bool valid = t < mt;
+  const int X = base + g0 + (valid ? t : 0);
+  const double4 tp = tgtP[X], tn = tgtN[X];
+  const double cx = leafCtr[3 * L], cy = leafCtr[3 * L + 1], cz = leafCtr[3 * L + 2];
+  NearPartial p{0.0, 0.0, 0.0, 0.0};
+  const int p1 = ordOff[L + 1], p0 = ordOff[L];
+  const bool byLeaf = p1 - p0 >= kNearWarps;
+  for (int q = p0 + (byLeaf ? warp : 0); q < p1; q += byLeaf ? kNearWarps : 1) {
+    const int S = ordSrc[q], sb = leafStart[S];
+    int jb, je;
+    near_share(warp, byLeaf, leafCount[S], jb, je);
+    const double tx = tp.x + (cx - leafCtr[3 * S]), ty = tp.y + (cy - leafCtr[3 * S + 1]),
+                 tz = tp.z + (cz - leafCtr[3 * S + 2]);
+    for (int j0 = jb; j0 < je; j0 += 32) {
+      const int m = min(32, je - j0);
+      if (lane < m)
+        near_record<double>(sb + j0 + lane, n, tgtP, tgtN, area, sgm, sA[warp][lane], sB[warp][lane]);
+      __syncwarp();
+#pragma unroll 4
+      for (int jj = sub; jj < m; jj += k)
+        near_pair<ADJ>(sA[warp][jj], sB[warp][jj], tx, ty, tz, tn, K, p.s0, p.s1);
+      __syncwarp();
+    }
+  }
+  if (valid) {
+    const int first = warp * k + sub, step = kNearWarps * k;
+    if (gatOff) near_gather(gatOff[L], gatOff[L + 1], first, step, X - base, gatSlot, scr, p.s0, p.s1);
+    special_sums(X, n, first, step, spOff, spSrc, spK, sgm, p.e0, p.e1);
+  }
+  p = near_partials(p, mt, k);
+  if ((int)threadIdx.x < mt) near_store(base + g0 + threadIdx.x, n, p, area, coef, accumulate, out);
 }
 
 // FP64 correction for every special pair: exact panelIA0 minus the
@@ -1289,11 +1124,8 @@ bool setup_near(Context &c) {
     w.nearOff[w.nLeaves] = (int)w.nearSrc.size();
     if (!c.arena.upload(&c.d_nearOff, w.nearOff, s) || !c.arena.upload(&c.d_nearSrc, w.nearSrc, s)) return false;
   }
-  // warp tasks: (leaf, group of 32 targets), the most expensive first so the
-  // last wave of the grid holds the short tasks (a warp's time ~ sources / k,
-  // k = lanes per target)
+  // the finishing kernel's blocks: (leaf, group of 32 targets), the largest leaves first
   std::vector<int2> work;
-  std::vector<long long> cost;
   c.maxLeaf = 0;
   c.nearPanelPairs = 0;
   for (int L = 0; L < pt.nLeaves; L++) {
@@ -1302,19 +1134,10 @@ bool setup_near(Context &c) {
     long long srcs = 0;
     for (int p = pt.nearOff[L]; p < pt.nearOff[L + 1]; p++) srcs += pt.leafCount[pt.nearSrc[p]];
     c.nearPanelPairs += srcs * cnt;
-    for (int g = 0; g * 32 < cnt; g++) {
-      work.push_back(make_int2(L, g));
-      cost.push_back(srcs / (32 / std::min(32, cnt - 32 * g)));
-    }
+    for (int g = 0; g * 32 < cnt; g++) work.push_back(make_int2(L, g));
   }
-  {
-    std::vector<int> ord(work.size());
-    for (size_t i = 0; i < ord.size(); i++) ord[i] = (int)i;
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    std::vector<int2> sorted(work.size());
-    for (size_t i = 0; i < ord.size(); i++) sorted[i] = work[ord[i]];
-    work.swap(sorted);
-  }
+  std::stable_sort(work.begin(), work.end(),
+                   [&](const int2 &a, const int2 &b) { return pt.leafCount[a.x] > pt.leafCount[b.x]; });
   c.nWork = (int)work.size();
   if (!c.arena.upload(&c.d_work, work, s)) return false;
 
@@ -1435,73 +1258,100 @@ static bool special_pairs_host(Context &c, const std::vector<int> &nearSortedFla
   return true;
 }
 
-// The symmetric kernels' leaf pairs (FMM operator, both precisions): every
-// unordered pair of distinct near leaves whose smaller leaf has at least
-// FB_NEAR_SYM_MIN_LEAF panels, the larger leaf on the register side; a scratch
-// slot of 2 floats per (ordered pair, target panel); costliest pairs first.
-// FABIPB_B200_NEAR_SYM=0 turns it off (every pair in the ordered kernel).
+// The symmetric near field's tasks: every unordered pair of distinct near
+// leaves whose smaller leaf has at least FB_NEAR_SYM_MIN_LEAF panels, the larger
+// leaf on the register side, largest tasks first.  FABIPB_B200_NEAR_SYM=0 turns
+// them off (every pair in the finishing kernel).
+#ifndef FB_NEAR_SYM_MIN_LEAF
+#define FB_NEAR_SYM_MIN_LEAF 4
+#endif
+// FP64 pairs with a smaller leaf stay in the finishing kernel (32-wide tiles only)
+#ifndef FB_NEAR_SYM_MIN_LEAF64
+#define FB_NEAR_SYM_MIN_LEAF64 48
+#endif
+// cost of a padded pair on a half-warp, percent of that on a warp
+#ifndef FB_NEAR_SYM16_COST
+#define FB_NEAR_SYM16_COST 110
+#endif
 static bool setup_near_sym(Context &c) {
   c.nSymTasks = 0;
-  const char *env = getenv("FABIPB_B200_NEAR_SYM");
-  if (c.dense || (env && atoi(env) == 0)) return true;
   const PanelTree &pt = c.pt;
-  const size_t nEnt = pt.nearSrc.size();
-  std::vector<int> symOff(nEnt, -1);
-  std::vector<int4> tasks;
-  std::vector<long long> cost;
-  std::vector<char> half;   // a pair with a small leaf: near_sym16_f2_kernel
-  long long tot = 0, pairs = 0;
-  for (int L = 0; L < pt.nLeaves; L++)
-    for (int p = pt.nearOff[L]; p < pt.nearOff[L + 1]; p++) {
-      const int S = pt.nearSrc[p];
-      if (S <= L) continue;
-      const int cl = pt.leafCount[L], cs = pt.leafCount[S];
-      const int mn = std::min(cl, cs);
-      if (mn < (c.mixed ? FB_NEAR_SYM16_MIN_LEAF : FB_NEAR_SYM_MIN_LEAF)) continue;
-      // mixed contexts: the half-warp kernel where its padding to 16-panel groups and tiles saves
-      // more than its larger per-tile overhead (FB_NEAR_SYM16_COST percent of the 32-wide cost
-      // per padded pair), which always holds below FB_NEAR_SYM_MIN_LEAF
-      const long long p32 = (long long)((cl + 31) / 32) * ((cs + 31) / 32) * 1024;
-      const long long p16 = (long long)((cl + 15) / 16) * ((cs + 15) / 16) * 256;
-      const bool small = c.mixed && (mn < FB_NEAR_SYM_MIN_LEAF || p16 * FB_NEAR_SYM16_COST < p32 * 100);
-      int q = -1;   // the mirror entry (S <- L)
-      for (int k = pt.nearOff[S]; k < pt.nearOff[S + 1]; k++)
-        if (pt.nearSrc[k] == L) { q = k; break; }
-      if (q < 0) continue;   // not mirrored: both directions stay ordered
-      const bool lReg = cl >= cs;
-      const int R = lReg ? L : S, T = lReg ? S : L, pR = lReg ? p : q, pT = lReg ? q : p;
-      FB_CHECK(tot + cl + cs < 2147483647LL, "symmetric near-field scratch above 2^31 slots");
-      symOff[pR] = (int)tot;
-      tot += pt.leafCount[R];
-      symOff[pT] = (int)tot;
-      tot += pt.leafCount[T];
-      tasks.push_back(make_int4(R, T, symOff[pR], symOff[pT]));
-      cost.push_back((long long)cl * cs);
-      half.push_back(small);
-      pairs += (long long)cl * cs;
-    }
-  if (tasks.empty()) return true;
-  // the 32-wide tasks first, then the half-warp ones, each by decreasing cost
-  std::vector<int> ord(tasks.size());
-  for (size_t i = 0; i < ord.size(); i++) ord[i] = (int)i;
-  std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
-    return half[a] != half[b] ? half[b] != 0 : cost[a] > cost[b];
-  });
-  std::vector<int4> sorted(tasks.size());
-  int n32 = 0;
-  for (size_t i = 0; i < ord.size(); i++) {
-    sorted[i] = tasks[ord[i]];
-    n32 += half[ord[i]] ? 0 : 1;
-  }
   cudaStream_t s = c.stream;
-  const size_t esz = c.mixed ? sizeof(float) : sizeof(double);   // scratch element; records are 4 of them
-  if (!c.arena.upload(&c.d_symTask, sorted, s) || !c.arena.upload(&c.d_symOff, symOff, s) ||
-      !c.arena.alloc(&c.d_symScr, 2 * esz * (size_t)tot) || !c.arena.alloc(&c.d_symA, 4 * esz * (size_t)c.n) ||
-      !c.arena.alloc(&c.d_symB, 4 * esz * (size_t)c.n))
-    return false;
-  c.nSymTasks = (int)sorted.size();
-  c.nSym32 = n32;
-  c.symPanelPairs = pairs;
+  const char *env = getenv("FABIPB_B200_NEAR_SYM");
+  std::vector<NearTask> tasks;
+  std::vector<std::vector<int>> slots(pt.nLeaves);   // per leaf, the slots of its sums
+  std::vector<int> ordOff(pt.nLeaves + 1, 0), ordSrc;
+  if (!c.dense && !(env && atoi(env) == 0)) {
+    const int minLeaf = c.mixed ? FB_NEAR_SYM_MIN_LEAF : FB_NEAR_SYM_MIN_LEAF64;
+    auto on_tasks = [&](int a, int b) { return a != b && std::min(pt.leafCount[a], pt.leafCount[b]) >= minLeaf; };
+    // panels of R per task: whole leaves up to 256 panels; 64 when that leaves fewer padded 32 x 32
+    // tiles than eight for each of the chip's 2,368 resident warps (a task is one warp's serial work)
+    long long tiles = 0;
+    for (int L = 0; L < pt.nLeaves; L++)
+      for (int p = pt.nearOff[L]; p < pt.nearOff[L + 1]; p++)
+        if (pt.nearSrc[p] > L) tiles += (long long)((pt.leafCount[L] + 31) / 32) * ((pt.leafCount[pt.nearSrc[p]] + 31) / 32);
+    const int chunk = tiles < 8 * 2368 ? 64 : 256;
+    std::vector<long long> cost;
+    std::vector<char> half;
+    long long tot = 0;
+    for (int L = 0; L < pt.nLeaves; L++)
+      for (int p = pt.nearOff[L]; p < pt.nearOff[L + 1]; p++) {
+        const int S = pt.nearSrc[p];
+        if (S <= L || !on_tasks(L, S)) continue;
+        const int R = pt.leafCount[L] >= pt.leafCount[S] ? L : S, T = R == L ? S : L;
+        const int cr = pt.leafCount[R], ct = pt.leafCount[T];
+        // the half-warp where its padding to 16-panel groups and tiles saves more than its cost
+        const long long p32 = (long long)((cr + 31) / 32) * ((ct + 31) / 32) * 1024;
+        const long long p16 = (long long)((cr + 15) / 16) * ((ct + 15) / 16) * 256;
+        const bool small = c.mixed && p16 * FB_NEAR_SYM16_COST < p32 * 100;
+        const int nch = (cr + chunk - 1) / chunk;
+        FB_CHECK(tot + cr + (long long)nch * ct < 2147483647LL, "symmetric near-field scratch above 2^31 slots");
+        const int scrR = (int)tot;
+        tot += cr;
+        slots[R].push_back(scrR);
+        for (int k = 0; k < nch; k++) {
+          const int r0 = k * chunk, r1 = std::min(cr, r0 + chunk);
+          tasks.push_back(NearTask{R, T, r0, r1, scrR, (int)tot});
+          slots[T].push_back((int)tot);
+          tot += ct;
+          cost.push_back((long long)(r1 - r0) * ct);
+          half.push_back(small);
+        }
+      }
+    // the warp tasks first, then the half-warp ones, each by decreasing cost
+    std::vector<int> ord(tasks.size());
+    for (size_t i = 0; i < ord.size(); i++) ord[i] = (int)i;
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+      return half[a] != half[b] ? half[b] != 0 : cost[a] > cost[b];
+    });
+    std::vector<NearTask> sorted(tasks.size());
+    for (size_t i = 0; i < ord.size(); i++) sorted[i] = tasks[ord[i]];
+    c.nSymTasks = (int)sorted.size();
+    c.nSym32 = (int)std::count(half.begin(), half.end(), 0);
+    if (c.nSymTasks > 0) {
+      std::vector<int> gatOff(pt.nLeaves + 1, 0), gatSlot;
+      for (int L = 0; L < pt.nLeaves; L++) {
+        gatSlot.insert(gatSlot.end(), slots[L].begin(), slots[L].end());
+        gatOff[L + 1] = (int)gatSlot.size();
+      }
+      const size_t esz = c.mixed ? sizeof(float2) : sizeof(double2);
+      if (!c.arena.upload(&c.d_symTask, sorted, s) || !c.arena.upload(&c.d_gatOff, gatOff, s) ||
+          !c.arena.upload(&c.d_gatSlot, gatSlot, s) || !c.arena.alloc(&c.d_symScr, esz * (size_t)tot) ||
+          !c.arena.alloc(&c.d_recA, 2 * esz * (size_t)c.n) || !c.arena.alloc(&c.d_recB, 2 * esz * (size_t)c.n))
+        return false;
+      for (int L = 0; L < pt.nLeaves; L++) {
+        for (int p = pt.nearOff[L]; p < pt.nearOff[L + 1]; p++)
+          if (!on_tasks(L, pt.nearSrc[p])) ordSrc.push_back(pt.nearSrc[p]);
+        ordOff[L + 1] = (int)ordSrc.size();
+      }
+      if (!c.arena.upload(&c.d_ordOff, ordOff, s) || !c.arena.upload(&c.d_ordSrc, ordSrc, s)) return false;
+      FB_CUDA(cudaStreamSynchronize(s));   // the host vectors go out of scope
+    }
+  }
+  if (c.nSymTasks == 0) {   // every pair in the finishing kernel
+    c.d_ordOff = c.d_nearOff;
+    c.d_ordSrc = c.d_nearSrc;
+  }
   return true;
 }
 
@@ -1510,9 +1360,7 @@ static bool setup_near_targets(Context &c) {
   const int n = c.n;
   cudaStream_t s = c.stream;
   size_t vb = c.mixed ? sizeof(float4) : sizeof(double4);
-  if (!c.arena.alloc(&c.d_tgtP, vb * n) || !c.arena.alloc(&c.d_tgtN, vb * n) ||
-      !c.arena.alloc(&c.d_srcA, vb * n) || !c.arena.alloc(&c.d_srcB, vb * n))
-    return false;
+  if (!c.arena.alloc(&c.d_tgtP, vb * n) || !c.arena.alloc(&c.d_tgtN, vb * n)) return false;
   if (c.mixed) {
     near_targets_kernel<float><<<ceil_div(n, 256), 256, 0, s>>>(
         n, c.d_vtx, c.d_nrm, c.d_area, c.d_leafOfPanel, c.d_leafCtr, (float4 *)c.d_tgtP, (float4 *)c.d_tgtN);
@@ -1524,61 +1372,49 @@ static bool setup_near_targets(Context &c) {
   return setup_near_sym(c);
 }
 
-template <typename T, bool ADJ>
-static void launch_near_t(Context &c, const void *tgtP, const void *tgtN, void *srcA, void *srcB, const double *sgm,
-                          double coef, double *out, cudaStream_t s, bool accumulate) {
-  typedef typename Vec4<T>::t V;
-  const int n = c.n;
+template <bool ADJ>
+static void launch_near_f32(Context &c, const double *sgm, double coef, double *out, cudaStream_t s, bool accumulate) {
   const double kap = c.prm.kappa, eps = c.epsilon;
-  const unsigned grid = ceil_div(c.nWork, kNearWarps);
-  const double kexp = sizeof(T) == 4 ? -kap * 1.4426950408889634 : -kap;   // float: exp2 argument
-  const bool packed = sizeof(T) == 4 && FB_NEAR_PACKED;
-  near_pack_kernel<T><<<ceil_div(n, 256), 256, 0, s>>>(n, (const V *)tgtP, (const V *)tgtN, c.d_area, sgm, (V *)srcA,
-                                                       (V *)srcB, packed ? (ADJ ? 2 : 1) : 0);
-  if (packed) {
-    const bool sym = c.nSymTasks > 0 && tgtP == c.d_tgtP;
-    if (sym) {   // unordered leaf pairs of the symmetric kernel first, into the scratch
-      near_pack_kernel<float><<<ceil_div(n, 256), 256, 0, s>>>(n, (const float4 *)tgtP, (const float4 *)tgtN,
-                                                               c.d_area, sgm, (float4 *)c.d_symA, (float4 *)c.d_symB, 0);
-      if (c.nSym32 > 0) {
-        near_sym_f2_kernel<ADJ><<<ceil_div(c.nSym32, kSymWarps), kSymWarps * 32, 0, s>>>(
-            c.nSym32, c.d_symTask, c.d_leafStart, c.d_leafCount, c.d_leafCtr, (const float4 *)c.d_symA,
-            (const float4 *)c.d_symB, (float)kap, (float)kexp, (float)eps, (float)(1.0 / eps), (float)(kap * kap),
-            (float2 *)c.d_symScr);
-        c.launches += 1;
-      }
-      if (c.nSymTasks > c.nSym32) {
-        near_sym16_f2_kernel<ADJ><<<ceil_div(c.nSymTasks - c.nSym32, 2 * kSymWarps), kSymWarps * 32, 0, s>>>(
-            c.nSymTasks - c.nSym32, c.d_symTask + c.nSym32, c.d_leafStart, c.d_leafCount, c.d_leafCtr,
-            (const float4 *)c.d_symA, (const float4 *)c.d_symB, (float)kap, (float)kexp, (float)eps,
-            (float)(1.0 / eps), (float)(kap * kap), (float2 *)c.d_symScr);
-        c.launches += 1;
-      }
-      c.launches += 1;
-    }
-    near_apply_f2_kernel<ADJ><<<grid, kNearWarps * 32, 0, s>>>(
-        c.nWork, c.d_work, c.d_leafStart, c.d_leafCount, c.d_nearOff, c.d_nearSrc, c.d_leafCtr,
-        (const float4 *)tgtP, (const float4 *)tgtN, (const float4 *)srcA, (const float4 *)srcB, c.d_spOff, c.d_spSrc,
-        ADJ ? c.d_spKT : c.d_spK, sgm, c.d_area, n, (float)kap, (float)kexp, (float)eps, (float)(1.0 / eps),
-        (float)(kap * kap), coef, accumulate ? 1 : 0, out, sym ? c.d_symOff : nullptr,
-        (const float2 *)c.d_symScr);
-    return;
-  }
-  // the symmetric kernel for the context's own records (not the FP64 residual records of a mixed context)
-  const bool sym = c.nSymTasks > 0 && tgtP == c.d_tgtP && (sizeof(T) == 8) == !c.mixed;
-  if (sym) {
-    near_pack_kernel<T><<<ceil_div(n, 256), 256, 0, s>>>(n, (const V *)tgtP, (const V *)tgtN, c.d_area, sgm,
-                                                         (V *)c.d_symA, (V *)c.d_symB, 0);
-    near_sym_kernel<T, ADJ><<<ceil_div(c.nSymTasks, kSymWarps), kSymWarps * 32, 0, s>>>(
-        c.nSymTasks, c.d_symTask, c.d_leafStart, c.d_leafCount, c.d_leafCtr, (const V *)c.d_symA,
-        (const V *)c.d_symB, (T)kap, (T)kexp, (T)eps, (T)(1.0 / eps), (T)(kap * kap), (T *)c.d_symScr);
+  const NearConstF K{(float)kap, (float)(-kap * 1.4426950408889634), (float)eps, (float)(1.0 / eps),
+                     (float)(kap * kap)};
+  const float4 *tgtP = (const float4 *)c.d_tgtP, *tgtN = (const float4 *)c.d_tgtN;
+  float4 *recA = (float4 *)c.d_recA, *recB = (float4 *)c.d_recB;
+  if (c.nSymTasks > 0) {
+    near_pack_kernel<float><<<ceil_div(c.n, 256), 256, 0, s>>>(c.n, tgtP, tgtN, c.d_area, sgm, recA, recB);
+    const unsigned blocks = ceil_div(c.nSym32, kSymWarps) + ceil_div(c.nSymTasks - c.nSym32, 2 * kSymWarps);
+    near_sym_f2_kernel<ADJ><<<blocks, kSymWarps * 32, 0, s>>>(c.nSym32, c.nSymTasks, c.d_symTask, c.d_leafStart,
+                                                              c.d_leafCount, c.d_leafCtr, recA, recB, K,
+                                                              (float2 *)c.d_symScr);
     c.launches += 2;
   }
-  near_apply_kernel<T, ADJ><<<grid, kNearWarps * 32, 0, s>>>(
-      c.nWork, c.d_work, c.d_leafStart, c.d_leafCount, c.d_nearOff, c.d_nearSrc, c.d_leafCtr, (const V *)tgtP,
-      (const V *)tgtN, (const V *)srcA, (const V *)srcB, c.d_spOff, c.d_spSrc, ADJ ? c.d_spKT : c.d_spK, sgm,
-      c.d_area, n, (T)kap, (T)kexp, (T)eps, (T)(1.0 / eps), (T)(kap * kap), coef, accumulate ? 1 : 0, out,
-      sym ? c.d_symOff : nullptr, (const T *)c.d_symScr);
+  near_apply_f2_kernel<ADJ><<<c.nWork, kNearWarps * 32, 0, s>>>(
+      c.d_work, c.d_leafStart, c.d_leafCount, c.d_ordOff, c.d_ordSrc, c.d_leafCtr, tgtP, tgtN, c.d_spOff, c.d_spSrc,
+      ADJ ? c.d_spKT : c.d_spK, sgm, c.d_area, c.n, K, coef, accumulate ? 1 : 0, out, c.d_gatOff, c.d_gatSlot,
+      (const float2 *)c.d_symScr);
+  c.launches += 1;
+}
+
+// FP64 contexts, and the FP64 residuals of a mixed context (its own records; the scratch is FP32
+// there, so every pair goes to the finishing kernel)
+template <bool ADJ>
+static void launch_near_f64(Context &c, const double *sgm, double coef, double *out, cudaStream_t s, bool accumulate) {
+  const double kap = c.prm.kappa, eps = c.epsilon;
+  const NearConstD K{kap, -kap, eps, 1.0 / eps, kap * kap};
+  const bool own = !c.mixed, sym = own && c.nSymTasks > 0;
+  const double4 *tgtP = (const double4 *)(own ? c.d_tgtP : c.d_tgtP64);
+  const double4 *tgtN = (const double4 *)(own ? c.d_tgtN : c.d_tgtN64);
+  if (sym) {
+    double4 *recA = (double4 *)c.d_recA, *recB = (double4 *)c.d_recB;
+    near_pack_kernel<double><<<ceil_div(c.n, 256), 256, 0, s>>>(c.n, tgtP, tgtN, c.d_area, sgm, recA, recB);
+    near_sym_kernel<ADJ><<<ceil_div(c.nSymTasks, kSymWarps), kSymWarps * 32, 0, s>>>(
+        c.nSymTasks, c.d_symTask, c.d_leafStart, c.d_leafCount, c.d_leafCtr, recA, recB, K, (double2 *)c.d_symScr);
+    c.launches += 2;
+  }
+  near_apply_kernel<ADJ><<<c.nWork, kNearWarps * 32, 0, s>>>(
+      c.d_work, c.d_leafStart, c.d_leafCount, own ? c.d_ordOff : c.d_nearOff, own ? c.d_ordSrc : c.d_nearSrc,
+      c.d_leafCtr, tgtP, tgtN, c.d_spOff, c.d_spSrc, ADJ ? c.d_spKT : c.d_spK, sgm, c.d_area, c.n, K, coef,
+      accumulate ? 1 : 0, out, sym ? c.d_gatOff : nullptr, c.d_gatSlot, (const double2 *)c.d_symScr);
+  c.launches += 1;
 }
 
 // FP64 records in a mixed context, for the FP64 residuals of iterative
@@ -1587,9 +1423,7 @@ static bool setup_near_fp64(Context &c) {
   if (c.d_tgtP64) return true;
   const int n = c.n;
   const size_t vb = sizeof(double4) * (size_t)n;
-  if (!c.arena.alloc(&c.d_tgtP64, vb) || !c.arena.alloc(&c.d_tgtN64, vb) || !c.arena.alloc(&c.d_srcA64, vb) ||
-      !c.arena.alloc(&c.d_srcB64, vb))
-    return false;
+  if (!c.arena.alloc(&c.d_tgtP64, vb) || !c.arena.alloc(&c.d_tgtN64, vb)) return false;
   near_targets_kernel<double><<<ceil_div(n, 256), 256, 0, c.stream>>>(n, c.d_vtx, c.d_nrm, c.d_area, c.d_leafOfPanel,
                                                                       c.d_leafCtr, (double4 *)c.d_tgtP64,
                                                                       (double4 *)c.d_tgtN64);
@@ -1665,18 +1499,14 @@ bool launch_near(Context &c, const double *sgm, double coef, double *out, bool a
     FB_CUDA(cudaGetLastError());
     return true;
   }
-  if (c.mixed && fp64) {
-    if (!setup_near_fp64(c)) return false;
-    if (adjoint) launch_near_t<double, true>(c, c.d_tgtP64, c.d_tgtN64, c.d_srcA64, c.d_srcB64, sgm, coef, out, s, acc);
-    else launch_near_t<double, false>(c, c.d_tgtP64, c.d_tgtN64, c.d_srcA64, c.d_srcB64, sgm, coef, out, s, acc);
-  } else if (c.mixed) {
-    if (adjoint) launch_near_t<float, true>(c, c.d_tgtP, c.d_tgtN, c.d_srcA, c.d_srcB, sgm, coef, out, s, acc);
-    else launch_near_t<float, false>(c, c.d_tgtP, c.d_tgtN, c.d_srcA, c.d_srcB, sgm, coef, out, s, acc);
+  if (c.mixed && !fp64) {
+    if (adjoint) launch_near_f32<true>(c, sgm, coef, out, s, acc);
+    else launch_near_f32<false>(c, sgm, coef, out, s, acc);
   } else {
-    if (adjoint) launch_near_t<double, true>(c, c.d_tgtP, c.d_tgtN, c.d_srcA, c.d_srcB, sgm, coef, out, s, acc);
-    else launch_near_t<double, false>(c, c.d_tgtP, c.d_tgtN, c.d_srcA, c.d_srcB, sgm, coef, out, s, acc);
+    if (c.mixed && !setup_near_fp64(c)) return false;
+    if (adjoint) launch_near_f64<true>(c, sgm, coef, out, s, acc);
+    else launch_near_f64<false>(c, sgm, coef, out, s, acc);
   }
-  c.launches += 2;
   FB_CUDA(cudaGetLastError());
   return true;
 }

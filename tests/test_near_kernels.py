@@ -48,3 +48,25 @@ def test_quadrature_near_field(panels, depth, q):
 def test_quadrature_near_field_screening(kappa):
     """No screening, and so much that e^{-kappa r} underflows for most pairs."""
     check(*both(cut_sphere(200), lib.FP64, order=3, depth=3, quad_order=2, kappa=kappa), 1e-12)
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-12), (lib.MIXED, 5e-6)])
+@pytest.mark.parametrize("panels,depth", [(2, 2), (33, 2), (319, 1), (641, 1), (1279, 2), (1280, 3)])
+def test_near_field_tiles(panels, depth, precision, tol):
+    """Leaves of one panel up to several tiles: groups and tiles that end anywhere, tasks on warps and half-warps, leaves
+    below the tasks' least size, whole leaves split over tasks."""
+    check(*both(cut_sphere(panels, seed=panels), precision, order=3, depth=depth, height=min(2, depth)), tol)
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-12), (lib.MIXED, 5e-6)])
+@pytest.mark.parametrize("kappa", [0.0, 40.0])
+def test_near_field_screening(kappa, precision, tol):
+    check(*both(cut_sphere(900), precision, order=3, depth=2, kappa=kappa), tol)
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-12), (lib.MIXED, 5e-6)])
+def test_near_field_zero_densities(precision, tol):
+    """A density with one half zero, and one of a single panel."""
+    s, o = both(cut_sphere(700), precision, order=3, depth=2)
+    for v in (np.r_[np.zeros(s.n), np.ones(s.n)], np.r_[np.ones(s.n), np.zeros(s.n)], np.eye(2 * s.n)[3]):
+        assert rel_l2(s.apply(v, part=lib.NEAR), o.near_apply(v)) < tol
