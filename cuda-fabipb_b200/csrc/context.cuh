@@ -33,8 +33,13 @@ struct Context {
   int *d_leafStart = nullptr, *d_leafCount = nullptr, *d_leafOfPanel = nullptr;
   int *d_nearOff = nullptr, *d_nearSrc = nullptr;
   double *d_leafCtr = nullptr;             // 3 per leaf: enclosing-box centre
+  // the near-field kernels' parts: the leaves, or in an FP64 direct context equal runs of panels
+  // (first panel, count, centre, part of panel)
+  std::vector<int> partStart, partCount;
+  int *d_partStart = nullptr, *d_partCount = nullptr, *d_partOf = nullptr;
+  double *d_partCtr = nullptr;
   int nWork = 0;                           // blocks of the near field's finishing kernel
-  int2 *d_work = nullptr;                  // (leaf, 32-target group)
+  int2 *d_work = nullptr;                  // (part, 32-target group)
   long long nearPanelPairs = 0;
   int maxLeaf = 0;
 
@@ -48,8 +53,8 @@ struct Context {
   double4 *d_spKT = nullptr;                   // the same for the transposed operator
   void *d_tgtP64 = nullptr, *d_tgtN64 = nullptr;   // FP64 records of a mixed context (refinement residuals)
   // the symmetric near field: its tasks (the first nSym32 on a warp, the rest on a half-warp), the
-  // scratch slots of their sums (two floats or doubles each) listed by leaf for the finishing kernel,
-  // and by leaf the source leaves that no task covers
+  // scratch slots of their sums (two floats or doubles each) listed by part for the finishing kernel,
+  // and by part the source parts that no task covers
   int nSymTasks = 0, nSym32 = 0;
   NearTask *d_symTask = nullptr;
   int *d_gatOff = nullptr, *d_gatSlot = nullptr;

@@ -70,3 +70,14 @@ def test_near_field_zero_densities(precision, tol):
     s, o = both(cut_sphere(700), precision, order=3, depth=2)
     for v in (np.r_[np.zeros(s.n), np.ones(s.n)], np.r_[np.ones(s.n), np.zeros(s.n)], np.eye(2 * s.n)[3]):
         assert rel_l2(s.apply(v, part=lib.NEAR), o.near_apply(v)) < tol
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-12), (lib.MIXED, 5e-6)])
+@pytest.mark.parametrize("panels,depth", [(3, 2), (127, 2), (129, 3), (641, 2), (1279, 3)])
+def test_direct_operator_parts(panels, depth, precision, tol):
+    """The direct context's parts (runs of 128 panels in FP64, leaves in mixed contexts) against the oracle with no far
+    field: an acceptance ratio so small that every leaf pair is near."""
+    pan = cut_sphere(panels, seed=panels)
+    opts = dict(order=3, depth=depth, sep_ratio=1e-9)
+    s = lib.Surface(pan, lib.params(precision=precision, **opts), direct=True)
+    check(s, O.Oracle(pan, O.make_params(**opts)), tol)
