@@ -12,15 +12,16 @@
 //                          Givens rotations, x0 = initial guess)
 //
 // B200 design: the block matrices are assembled by a kernel in FP64 (the
-// exact panelIA0 cases), factored with cuSOLVER at setup, and replaced by
-// their explicit inverses, so each preconditioner apply is one block-diagonal
-// GEMV kernel streaming the inverses from HBM instead of ~3 launches per
-// block.  The Krylov vectors live on the device; the Gram-Schmidt dot
-// products are reduced deterministically into a device array and only the
-// (restart+1)-long Hessenberg column crosses to the host per iteration, where
-// the Givens rotations run in FP64 exactly as in the reference.
+// exact panelIA0 cases) and replaced by their explicit inverses, so each
+// preconditioner apply is one block-diagonal GEMV kernel streaming the
+// inverses from HBM instead of ~3 launches per block; the inverses are formed
+// by size class in thread-block clusters (cuSOLVER above the last class).  The
+// Krylov vectors, the Hessenberg columns and the Givens rotations live on the
+// device, with deterministic reductions; a status record crosses to the host
+// once per step.
 #include <cusolverDn.h>
 
+#include <climits>
 #include <cmath>
 #include <vector>
 
@@ -40,6 +41,7 @@ struct PrecondDev {
   int *d_start = nullptr, *d_size = nullptr;
   int2 *d_tiles = nullptr;   // (block, first row) tiles of the apply
   int *d_colSrc = nullptr;   // per block (offset 2*start): input component of each stored column
+  int *d_rowDst = nullptr;   // output component of each stored row
   int nTiles = 0;
   long long *d_off = nullptr;
   double *d_inv = nullptr;
@@ -141,10 +143,10 @@ __global__ void pc_special_kernel(int nBlocks, const int *__restrict__ bStart, c
   }
 }
 
-// the listed blocks of I := identity, and their column index the identity
+// the listed blocks of I := identity, and their column and row indices the identity
 __global__ void identity_kernel(int nList, const int *__restrict__ list, const int *__restrict__ bStart,
                                 const int *__restrict__ bSize, const long long *__restrict__ bOff, double *I,
-                                int *colSrc) {
+                                int *colSrc, int *rowDst) {
   for (int li = blockIdx.y; li < nList; li += gridDim.y) {   // (y extent capped at 65535)
     const int b = list[li];
     const int M = 2 * bSize[b];
@@ -153,15 +155,307 @@ __global__ void identity_kernel(int nList, const int *__restrict__ list, const i
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < e; p += (long long)gridDim.x * blockDim.x)
       Ib[p] = ((p / M) == (p % M)) ? 1.0 : 0.0;
     if (blockIdx.x == 0)
-      for (int c = threadIdx.x; c < M; c += blockDim.x) colSrc[2LL * bStart[b] + c] = c;
+      for (int c = threadIdx.x; c < M; c += blockDim.x)
+        colSrc[2LL * bStart[b] + c] = rowDst[2LL * bStart[b] + c] = c;
   }
 }
 
-// In-place inversion of the preconditioner blocks by blocked Gauss-Jordan
-// elimination with partial (row) pivoting, all blocks in one launch per size
-// class (a library LU costs tens of small launches per block).  A block is
-// inverted by a cluster of CS thread blocks (CS = 1 for small blocks).  Per
-// panel of NB columns:
+// In-place inversion of the preconditioner blocks of up to 1,536 rows by
+// blocked Gauss-Jordan elimination with partial pivoting, all blocks of a size
+// class in one launch; a block is inverted by a cluster of CS thread blocks.
+// Per panel of NB columns:
+//   * every CTA of the cluster eliminates the panel in its shared memory (the
+//     same data, so the same result), eight columns at a time with its rows in
+//     registers (row i belongs to thread i mod 256), one barrier per pivot: the
+//     warps' candidates (largest |a| among the rows not yet taken) carry their
+//     rows along; each eight columns are then a rank-8 update of the panel's rest;
+//   * each CTA takes its share of the other columns, dealt in tiles:
+//     A(:, j) = A(:, j) without the pivot rows + Panel * A(pivot rows, j).
+// Rows are never interchanged: perm[k] is the row that column k was eliminated
+// with, stored column c multiplies input component colSrc[c] = perm[c], and
+// stored row perm[k] is output component rowDst[perm[k]] = k.
+//
+// 2 M^3 operations; bound by the blocks' traffic in the updates (every panel
+// reads and writes a whole block, and the blocks in work exceed the L2) and by
+// the pivots' latency in the panels, so panels are as wide as shared memory
+// allows and two CTAs share an SM.  A panel of 32 columns of a 575-row block on
+// two CTAs: 46 us of pivots and in-panel updates, 26 gathering the pivot rows,
+// 115 updating.  With interchanged rows, panels of 16 eliminated in shared
+// memory with two barriers per pivot, the interchange list formed by one thread
+// and the classes side by side, the 1,127 blocks of the 204,800-panel star
+// surface (mean 363 rows) took 52 ms in FP32; 27.5 now.
+constexpr int kInvSub = 8;   // columns eliminated in registers
+
+template <typename TV>
+struct InvShape;   // quads of rows and columns per thread in the update
+template <>
+struct InvShape<float> {
+  static constexpr int QR = 2;
+  typedef float4 V4;
+};
+template <>
+struct InvShape<double> {
+  static constexpr int QR = 1;
+  typedef double4 V4;
+};
+
+template <typename TV, int NB, int QC>
+__host__ __device__ constexpr size_t inv_smem_bytes(int maxM) {
+  return sizeof(TV) * ((size_t)NB * ((maxM + 3) & ~3) + (size_t)NB * 64 * QC) + (size_t)maxM * (sizeof(int) + 1);
+}
+
+// the largest value of the warp and the lowest index among the lanes that hold it (v >= 0, or -1 for none)
+__device__ __forceinline__ int warp_first_max(float v, int i) {
+  const unsigned b = v < 0.f ? 0u : __float_as_uint(v) + 1u;
+  const unsigned m = __reduce_max_sync(0xffffffffu, b);
+  return __reduce_min_sync(0xffffffffu, b == m ? i : INT_MAX);
+}
+__device__ __forceinline__ int warp_first_max(double v, int i) {
+  const unsigned hi = v < 0.0 ? 0u : (unsigned)__double2hiint(v) + 1u;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)__double2loint(v) : 0u;
+  const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+  return __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? i : INT_MAX);
+}
+
+template <typename TV, int NB, int CS, int RPT, int QC, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+pc_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart, const int *__restrict__ bSize,
+                 const long long *__restrict__ bOff, TV *inv, int *colSrc, int *rowDst, int *info) {
+  typedef typename Vec2<TV>::t V2;
+  typedef typename InvShape<TV>::V4 V4;
+  constexpr int QR = InvShape<TV>::QR, TR = 64 * QR, TC = 64 * QC;
+  constexpr int W = NT / 32;
+  extern __shared__ double4 invSmem[];
+  __shared__ TV cVal[2][W], cRow[2][W][kInvSub], sY[NB][kInvSub];
+  __shared__ int cIdx[2][W];
+  const int rank = (CS > 1) ? (int)(blockIdx.x % CS) : 0;
+  const int b = list[blockIdx.x / CS];
+  const int M = 2 * bSize[b], Mp = (M + 3) & ~3;
+  TV *A = inv + bOff[b];
+  TV *P = reinterpret_cast<TV *>(invSmem);       // the panel, [NB][Mp]
+  TV *Yt = P + (size_t)NB * Mp;                  // the pivot rows of a column tile, [NB][TC]
+  int *perm = reinterpret_cast<int *>(Yt + (size_t)NB * TC);   // [M]
+  unsigned char *flag = reinterpret_cast<unsigned char *>(perm + M);   // [M]: a pivot row of this panel
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int grp = t / 256, tr = t % 16, tc = (t % 256) / 16;   // groups of 256 threads take the row tiles in turn
+  unsigned used = 0;   // of this thread's rows
+  int bad = 0;
+  for (int k0 = 0; k0 < M; k0 += NB) {
+    const int nb = min(NB, M - k0);
+    if (CS > 1) {   // the owners' updates of these columns are complete and visible
+      __threadfence();
+      cooperative_groups::this_cluster().sync();
+    } else {
+      __syncthreads();
+    }
+    for (int i = t; i < M; i += NT) {
+      flag[i] = 0;
+      const TV *src = A + (size_t)k0 * M + i;
+#pragma unroll 16
+      for (int c = 0; c < nb; c++) P[c * Mp + i] = src[(size_t)c * M];
+    }
+    // (row i of P and of flag: written and read by thread i mod 256 until the next barrier)
+    for (int c0 = 0; c0 < nb; c0 += kInvSub) {
+      const int sb = min(kInvSub, nb - c0);
+      TV v[RPT][kInvSub];
+      unsigned sub = 0;   // pivot rows of these columns
+#pragma unroll
+      for (int r = 0; r < RPT; r++) {
+        const int i = t + r * NT;
+#pragma unroll
+        for (int c = 0; c < kInvSub; c++) v[r][c] = i < M && c < sb ? P[(c0 + c) * Mp + i] : (TV)0;
+      }
+#pragma unroll
+      for (int kk = 0; kk < kInvSub; kk++) {
+        if (kk >= sb) break;   // uniform
+        TV best = (TV)-1;
+        int bi = INT_MAX;
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+          const int i = t + r * NT;
+          const TV a = fabs(v[r][kk]);
+          if (i < M && !((used >> r) & 1u) && a > best) {
+            best = a;
+            bi = i;
+          }
+        }
+        const int wi = warp_first_max(best, bi), par = kk & 1;
+        if (wi == INT_MAX) {   // no row left in this warp
+          if (lane == 0) {
+            cVal[par][warp] = (TV)-1;
+            cIdx[par][warp] = INT_MAX;
+          }
+        } else if (bi == wi) {
+          cVal[par][warp] = best;
+          cIdx[par][warp] = wi;
+#pragma unroll
+          for (int r = 0; r < RPT; r++)
+            if (t + r * NT == wi)
+#pragma unroll
+              for (int c = 0; c < kInvSub; c++) cRow[par][warp][c] = v[r][c];
+        }
+        __syncthreads();   // (two buffers: a step's writes cannot meet the previous step's reads)
+        const int ci = lane < W ? cIdx[par][lane] : INT_MAX;
+        const int pv = warp_first_max(lane < W ? cVal[par][lane] : (TV)-1, ci);
+        const int pw = __ffs(__ballot_sync(0xffffffffu, ci == pv)) - 1;
+        const TV piv = cRow[par][pw][kk];
+        const TV d = piv != (TV)0 ? (TV)1 / piv : (TV)0;
+        if (piv == (TV)0) bad = bad ? bad : k0 + c0 + kk + 1;
+        if (t == 0) perm[k0 + c0 + kk] = pv;
+        TV row[kInvSub];
+#pragma unroll
+        for (int c = 0; c < kInvSub; c++) row[c] = c == kk ? d : cRow[par][pw][c] * d;
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+          const TV f = v[r][kk];
+          if (t + r * NT == pv) {
+            used |= 1u << r;
+            sub |= 1u << r;
+            flag[pv] = 1;
+#pragma unroll
+            for (int c = 0; c < kInvSub; c++) v[r][c] = row[c];
+          } else {
+#pragma unroll
+            for (int c = 0; c < kInvSub; c++) v[r][c] = c == kk ? -f * d : v[r][c] - f * row[c];
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < RPT; r++) {
+        const int i = t + r * NT;
+        if (i < M)
+#pragma unroll
+          for (int c = 0; c < kInvSub; c++)
+            if (c < sb) P[(c0 + c) * Mp + i] = v[r][c];
+      }
+      if (nb > kInvSub) {   // the panel's other columns
+        __syncthreads();    // perm, and the previous rows' columns, are written
+        for (int e = t; e < nb * kInvSub; e += NT) {
+          const int c = e / kInvSub, kk = e % kInvSub;
+          sY[c][kk] = kk < sb && (c < c0 || c >= c0 + sb) ? P[c * Mp + perm[k0 + c0 + kk]] : (TV)0;
+        }
+        __syncthreads();
+        for (int c = 0; c < nb; c++) {
+          if (c >= c0 && c < c0 + sb) continue;
+          TV y[kInvSub];
+#pragma unroll
+          for (int kk = 0; kk < kInvSub; kk++) y[kk] = sY[c][kk];
+#pragma unroll
+          for (int r = 0; r < RPT; r++) {
+            const int i = t + r * NT;
+            if (i < M) {
+              TV s = (sub >> r) & 1u ? (TV)0 : P[c * Mp + i];
+#pragma unroll
+              for (int kk = 0; kk < kInvSub; kk++) s += v[r][kk] * y[kk];
+              P[c * Mp + i] = s;
+            }
+          }
+        }
+      }
+    }
+    if (CS > 1) cooperative_groups::this_cluster().sync();   // every CTA has read the panel's columns
+    else __syncthreads();
+    if (rank == 0)
+      for (int c = 0; c < nb; c++)
+        for (int i = t; i < M; i += NT) A[(size_t)(k0 + c) * M + i] = P[c * Mp + i];
+    for (int jt = TC * rank; jt < M; jt += TC * CS) {
+      __syncthreads();   // the previous tile's reads of Yt are done
+#pragma unroll 8
+      for (int e = t; e < nb * TC; e += NT) {
+        const int kk = e / TC, j = jt + e % TC;
+        Yt[e] = j < M ? A[(size_t)j * M + perm[k0 + kk]] : (TV)0;
+      }
+      __syncthreads();
+      // row tiles, the next one's values loaded while the current one is computed
+      auto load_tile = [&](int it, TV (&v)[QC * 4][QR * 4]) {
+#pragma unroll
+        for (int q = 0; q < QR; q++) {
+          const int i0 = it + 64 * q + 4 * tr;
+          const bool in = i0 < M, hi = i0 + 2 < M;   // M is even: a row quad is full or holds two rows
+#pragma unroll
+          for (int c = 0; c < QC * 4; c++) {
+            const int j = jt + 64 * (c / 4) + 4 * tc + c % 4;
+            V2 a{(TV)0, (TV)0}, z{(TV)0, (TV)0};
+            if (in && j < M) {
+              const V2 *src = reinterpret_cast<const V2 *>(A + (size_t)j * M + i0);
+              a = src[0];
+              if (hi) z = src[1];
+            }
+            v[c][4 * q] = a.x;
+            v[c][4 * q + 1] = a.y;
+            v[c][4 * q + 2] = z.x;
+            v[c][4 * q + 3] = z.y;
+          }
+        }
+      };
+      constexpr int kStep = TR * (NT / 256);
+      TV nxt[QC * 4][QR * 4];
+      if (TR * grp < M) load_tile(TR * grp, nxt);
+      for (int it = TR * grp; it < M; it += kStep) {
+        TV acc[QC * 4][QR * 4];
+        int ir[QR];
+#pragma unroll
+        for (int q = 0; q < QR; q++) {
+          const int i0 = it + 64 * q + 4 * tr;
+          ir[q] = i0 < M ? i0 : -1;
+#pragma unroll
+          for (int r = 0; r < 4; r++) {
+            const bool f = i0 + r < M && flag[i0 + r];   // a pivot row starts from zero
+#pragma unroll
+            for (int c = 0; c < QC * 4; c++) acc[c][4 * q + r] = f ? (TV)0 : nxt[c][4 * q + r];
+          }
+        }
+        if (it + kStep < M) load_tile(it + kStep, nxt);
+#pragma unroll 2
+        for (int kk = 0; kk < nb; kk++) {
+          V4 w[QR], y[QC];
+#pragma unroll
+          for (int q = 0; q < QR; q++) w[q] = *reinterpret_cast<const V4 *>(P + (size_t)kk * Mp + (ir[q] < 0 ? 0 : ir[q]));
+#pragma unroll
+          for (int q = 0; q < QC; q++) y[q] = *reinterpret_cast<const V4 *>(Yt + kk * TC + 64 * q + 4 * tc);
+#pragma unroll
+          for (int c = 0; c < QC * 4; c++) {
+            const V4 &yq = y[c / 4];
+            const TV yc = c % 4 == 0 ? yq.x : c % 4 == 1 ? yq.y : c % 4 == 2 ? yq.z : yq.w;
+#pragma unroll
+            for (int q = 0; q < QR; q++) {
+              acc[c][4 * q] += w[q].x * yc;
+              acc[c][4 * q + 1] += w[q].y * yc;
+              acc[c][4 * q + 2] += w[q].z * yc;
+              acc[c][4 * q + 3] += w[q].w * yc;
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < QC * 4; c++) {
+          const int j = jt + 64 * (c / 4) + 4 * tc + c % 4;
+          if (j >= M || (j >= k0 && j < k0 + nb)) continue;
+#pragma unroll
+          for (int q = 0; q < QR; q++)
+            if (ir[q] >= 0) {
+              V2 *dst = reinterpret_cast<V2 *>(A + (size_t)j * M + ir[q]);
+              dst[0] = V2{acc[c][4 * q], acc[c][4 * q + 1]};
+              if (ir[q] + 2 < M) dst[1] = V2{acc[c][4 * q + 2], acc[c][4 * q + 3]};
+            }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (rank == 0) {
+    int *cs = colSrc + 2 * bStart[b], *rd = rowDst + 2 * bStart[b];
+    for (int k = t; k < M; k += NT) {
+      cs[k] = perm[k];
+      rd[perm[k]] = k;
+    }
+    if (t == 0) info[b] = bad;
+  }
+}
+
+// The same for larger blocks, whose panel's rows do not fit in registers: the
+// panel eliminated in shared memory, with row interchanges.  Per panel of NB
+// columns:
 //   * every CTA of the cluster eliminates the panel in its shared memory (the
 //     same data, so the same result; pivot = first largest |a| at or below
 //     the diagonal, as idamax) and rank 0 writes it back;
@@ -172,8 +466,8 @@ __global__ void identity_kernel(int nList, const int *__restrict__ list, const i
 //   * a cluster barrier before the next panel, whose columns some CTA owns.
 // The column interchanges that end Gauss-Jordan are not carried out:
 // colSrc[c] records which input component stored column c multiplies, and
-// the apply kernels gather through it.  info[b] = k+1 for an exactly zero
-// pivot k.
+// the apply kernels gather through it (rowDst is the identity).  info[b] = k+1
+// for an exactly zero pivot k.
 constexpr int kGjThreads = 256;
 
 template <typename TV, int NB>
@@ -190,7 +484,7 @@ template <typename TV, int NB, int CS>
 __global__ void __launch_bounds__(kGjThreads, sizeof(TV) == 4 ? FB_GJ_MIN_BLOCKS : 1)
 pc_gj_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart, const int *__restrict__ bSize,
                     const long long *__restrict__ bOff, const long long *__restrict__ yOff, TV *inv, TV *yAll,
-                    int *colSrc, int *info) {
+                    int *colSrc, int *rowDst, int *info) {
   typedef typename Vec2<TV>::t V2;
   extern __shared__ double gjSmemD[];
   TV *gjSmem = reinterpret_cast<TV *>(gjSmemD);
@@ -412,6 +706,7 @@ pc_gj_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart
     // invert: colSrc[sigma[j]] = j
     for (int j = 0; j < M; j++) perm[cs[j]] = j;
     for (int c = 0; c < M; c++) cs[c] = perm[c];
+    for (int c = 0; c < M; c++) rowDst[2 * bStart[b] + c] = c;
     info[b] = bad;
   }
   if (CS > 1) cooperative_groups::this_cluster().sync();   // no CTA leaves while others may still read
@@ -440,8 +735,8 @@ constexpr int kPcRows = 32 * kPcRpl, kPcWarps = 8, kPcChunk = 2048;
 template <typename TI>
 __global__ void __launch_bounds__(kPcWarps * 32)
 pc_apply_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ bStart, const int *__restrict__ bSize,
-                const long long *__restrict__ bOff, const int *__restrict__ colSrc, const TI *__restrict__ inv,
-                const double *__restrict__ rhs, double *x) {
+                const long long *__restrict__ bOff, const int *__restrict__ colSrc, const int *__restrict__ rowDst,
+                const TI *__restrict__ inv, const double *__restrict__ rhs, double *x) {
   typedef typename Vec2<TI>::t V2;
   __shared__ double xs[kPcChunk];
   __shared__ double red[kPcWarps][kPcRows];
@@ -491,8 +786,9 @@ pc_apply_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ b
       double t = red[0][i];
 #pragma unroll
       for (int w = 1; w < kPcWarps; w++) t += red[w][i];
-      if (rr < hm) x[st + rr] = t;
-      else x[n + st + rr - hm] = t;
+      const int g = rowDst[2 * (size_t)st + rr];
+      if (g < hm) x[st + g] = t;
+      else x[n + st + g - hm] = t;
     }
   }
 }
@@ -504,8 +800,8 @@ pc_apply_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ b
 template <typename TI>
 __global__ void __launch_bounds__(kPcWarps * 32)
 pc_apply_t_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ bStart, const int *__restrict__ bSize,
-                  const long long *__restrict__ bOff, const int *__restrict__ colSrc, const TI *__restrict__ inv,
-                  const double *__restrict__ rhs, double *x) {
+                  const long long *__restrict__ bOff, const int *__restrict__ colSrc, const int *__restrict__ rowDst,
+                  const TI *__restrict__ inv, const double *__restrict__ rhs, double *x) {
   typedef typename Vec2<TI>::t V2;
   __shared__ double xs[kPcChunk];
   const int2 tl = tiles[blockIdx.x];
@@ -521,8 +817,8 @@ pc_apply_t_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__
     const int kn = min(kPcChunk, M - k0);
     __syncthreads();
     for (int i = threadIdx.x; i < kn; i += blockDim.x) {
-      const int rr = k0 + i;
-      xs[i] = (rr < hm) ? rhs[st + rr] : rhs[n + st + rr - hm];
+      const int g = rowDst[2 * (size_t)st + k0 + i];
+      xs[i] = (g < hm) ? rhs[st + g] : rhs[n + st + g - hm];
     }
     __syncthreads();
 #pragma unroll
@@ -591,7 +887,8 @@ static bool factor_cusolver(Context &c, PrecondDev &p, const std::vector<int> &b
   FB_CUDA(cudaMalloc((void **)&d_list, blocks.size() * sizeof(int)));
   FB_CUDA(cudaMemcpyAsync(d_list, blocks.data(), blocks.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   dim3 grid(64, (unsigned)std::min<size_t>(blocks.size(), 65535));
-  identity_kernel<<<grid, 256, 0, s>>>((int)blocks.size(), d_list, p.d_start, p.d_size, p.d_off, p.d_inv, p.d_colSrc);
+  identity_kernel<<<grid, 256, 0, s>>>((int)blocks.size(), d_list, p.d_start, p.d_size, p.d_off, p.d_inv, p.d_colSrc,
+                                  p.d_rowDst);
   cudaEvent_t evA = nullptr;
   bool ok = cudaEventCreateWithFlags(&evA, cudaEventDisableTiming) == cudaSuccess;
   ok = ok && cudaEventRecord(evA, s) == cudaSuccess;
@@ -656,11 +953,6 @@ static bool factor_cusolver(Context &c, PrecondDev &p, const std::vector<int> &b
 #ifndef FB_PC_GJ_MAXM
 #define FB_PC_GJ_MAXM 11000
 #endif
-// CTAs per block for blocks of 385-768 rows (1 or 2; larger blocks use 8)
-#ifndef FB_PC_GJ_MIDCS
-#define FB_PC_GJ_MIDCS 2
-#endif
-
 template <typename TV, int NB, int CS>
 static bool launch_gj_t(int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p, const long long *d_yOff,
                         TV *inv, TV *d_y, int *d_info) {
@@ -689,37 +981,74 @@ static bool launch_gj_t(int nList, int maxM, cudaStream_t st, const int *d_list,
   cfg.numAttrs = 1;
   FB_CUDA(cudaLaunchKernelEx(&cfg, pc_gj_invert_kernel<TV, NB, CS>, d_list, (const int *)p.d_start,
                              (const int *)p.d_size, (const long long *)p.d_off, d_yOff, inv, d_y, p.d_colSrc,
-                             d_info));
+                             p.d_rowDst, d_info));
   return true;
 }
 
 template <typename TV>
-static bool launch_gj(int nb, int cs, int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p,
+static bool launch_gj(int nb, int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p,
                       const long long *d_yOff, TV *inv, TV *d_y, int *d_info) {
-  if (nb == 16 && cs == 1) return launch_gj_t<TV, 16, 1>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
-  if (nb == 16 && cs == 2) return launch_gj_t<TV, 16, 2>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
-  if (nb == 16 && cs == 8) return launch_gj_t<TV, 16, 8>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
-  if (nb == 8 && cs == 8) return launch_gj_t<TV, 8, 8>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
-  if constexpr (sizeof(TV) == 4) return launch_gj_t<TV, 4, 8>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
-  set_error("no Gauss-Jordan class with panel width %d", nb);
-  return false;
+  if constexpr (sizeof(TV) == 4) {
+    if (nb == 16) return launch_gj_t<TV, 16, 8>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
+    if (nb == 4) return launch_gj_t<TV, 4, 8>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
+  }
+  return launch_gj_t<TV, 8, 8>(nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
 }
 
-// Size classes of the Gauss-Jordan kernel per precision: rows up to, panel
-// width NB, CTAs per block (the panel of NB columns and the pivot record fit
-// in shared memory).  Blocks above the last class go to cuSOLVER (FP64).
-struct GjCls { int hi, nb, cs; };
+template <typename TV, int NB, int CS, int RPT, int QC, int NT>
+static bool launch_inv_t(int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p, TV *inv,
+                         int *d_info) {
+  FB_CHECK(maxM <= RPT * NT, "inversion class of %d rows given %d", RPT * NT, maxM);
+  const size_t shm = inv_smem_bytes<TV, NB, QC>(maxM);
+  FB_CUDA(cudaFuncSetAttribute(pc_invert_kernel<TV, NB, CS, RPT, QC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)shm));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nList * CS));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = shm;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  FB_CUDA(cudaLaunchKernelEx(&cfg, pc_invert_kernel<TV, NB, CS, RPT, QC, NT>, d_list, (const int *)p.d_start,
+                             (const int *)p.d_size, (const long long *)p.d_off, inv, p.d_colSrc, p.d_rowDst,
+                             d_info));
+  return true;
+}
+
+// Size classes per precision: rows up to, panel width.  Blocks of up to 1,536
+// rows go to pc_invert_kernel on one, two or four CTAs of 256 threads, two per
+// SM, so that one's pivots hide behind the other's updates (FP64 above 768
+// rows: 512 threads, one per SM); larger ones to pc_gj_invert_kernel; blocks
+// above the last class go to cuSOLVER (FP64).  FP32, 422 blocks of 385 to 768
+// rows: 11.7 ms on two CTAs, 14.6 on four, 21.9 on eight (each CTA repeats the
+// pivots), 13.7 with 512 threads; 91 blocks of 769 to 1,226 rows, panels of
+// 16: 15.0 ms on four, 21.7 on two, 18.1 on eight; panels of 32: 15.7 and more
+// (one CTA per SM).  FP64, the same 91: 37.4 ms, 53 on eight.
+struct GjCls { int hi, nb; };
 template <typename TV>
 static const GjCls *gj_classes(int *count) {
   // FP64 stops at 3200 rows: above it cuSOLVER's factorisation of a single
   // large block (all SMs) beats the kernel's narrow panels (measured on a
   // 2.1M-panel surface: 7.9 s against 9.8 s for the whole inversion)
-  // (the NB = 16 FP64 panel of 1536 rows plus the kernel's static shared
-  // memory is the largest that fits in the 227 KiB a block may use)
-  static const GjCls d64[4] = {{384, 16, 1}, {768, 16, FB_PC_GJ_MIDCS}, {1536, 16, 8}, {3200, 8, 8}};
-  static const GjCls d32[5] = {{384, 16, 1}, {768, 16, FB_PC_GJ_MIDCS}, {3200, 16, 8}, {6000, 8, 8}, {11000, 4, 8}};
-  *count = sizeof(TV) == 8 ? 4 : 5;
+  static const GjCls d64[4] = {{384, 16}, {768, 16}, {1536, 16}, {3200, 8}};
+  static const GjCls d32[6] = {{384, 32}, {768, 32}, {1536, 16}, {3200, 16}, {6000, 8}, {11000, 4}};
+  *count = sizeof(TV) == 8 ? 4 : 6;
   return sizeof(TV) == 8 ? d64 : d32;
+}
+
+template <typename TV>
+static bool launch_inversion(int ci, int nb, int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p,
+                             const long long *d_yOff, TV *inv, TV *d_y, int *d_info) {
+  constexpr bool f = sizeof(TV) == 4;
+  if (ci == 0) return launch_inv_t<TV, f ? 32 : 16, 1, 2, 1, 256>(nList, maxM, st, d_list, p, inv, d_info);
+  if (ci == 1) return launch_inv_t<TV, f ? 32 : 16, 2, 3, 1, 256>(nList, maxM, st, d_list, p, inv, d_info);
+  if (ci == 2) return launch_inv_t<TV, 16, 4, f ? 6 : 3, 1, f ? 256 : 512>(nList, maxM, st, d_list, p, inv, d_info);
+  return launch_gj<TV>(nb, nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
 }
 
 template <typename TV>
@@ -729,9 +1058,8 @@ static int gj_max_rows() {
   return std::min(c[n - 1].hi, FB_PC_GJ_MAXM);
 }
 
-// Gauss-Jordan inversion of every block of inv (assembled there), size
-// classes on their own streams so the large blocks start at once; blocks
-// above the kernel's size limit (FP64 only) go to cuSOLVER meanwhile.
+// Gauss-Jordan inversion of every block of inv (assembled there), class by
+// class; blocks above the kernels' size limit (FP64 only) go to cuSOLVER.
 template <typename TV>
 static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   cudaStream_t s = c.stream;
@@ -746,7 +1074,7 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   long long ytot = 0;
   for (int b = 0; b < p.nBlocks; b++) {
     yOff[b] = ytot;
-    ytot += 16LL * 2 * p.hSize[b];
+    if (2 * p.hSize[b] > cls[2].hi) ytot += 16LL * 2 * p.hSize[b];   // only pc_gj_invert_kernel uses it
   }
   long long *d_yOff = nullptr;
   TV *d_y = nullptr;
@@ -756,12 +1084,10 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
       !tmp.alloc_n(&d_info, (size_t)p.nBlocks))
     return false;
   FB_CUDA(cudaMemsetAsync(d_info, 0, (size_t)p.nBlocks * sizeof(int), s));
-  cudaEvent_t evA = nullptr;
-  FB_CUDA(cudaEventCreateWithFlags(&evA, cudaEventDisableTiming));
-  FB_CUDA(cudaEventRecord(evA, s));
-  std::vector<cudaStream_t> ss;
+  // the classes one after the other, the largest blocks first: side by side they push each other's blocks out of
+  // the L2, and a cluster waits for free SMs (the star's three classes: 59 ms side by side, 31.7 in turn)
   bool ok = true;
-  for (int ci = 0; ci < ncls; ci++) {
+  for (int ci = ncls - 1; ok && ci >= 0; ci--) {
     const GjCls &k = cls[ci];
     const int lo = ci ? cls[ci - 1].hi : 0, hi = std::min(k.hi, cut);
     std::vector<int> list;
@@ -776,42 +1102,17 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
     if (list.empty()) continue;
     std::stable_sort(list.begin(), list.end(), [&](int a, int b) { return p.hSize[a] > p.hSize[b]; });
     int *d_list = nullptr;
-    cudaStream_t st = nullptr;
-    ok = ok && tmp.upload(&d_list, list, s) && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
-    if (!ok) break;
-    ss.push_back(st);
-    cudaEvent_t evL = nullptr;   // the list upload and the assembly on s come first
-    ok = cudaEventCreateWithFlags(&evL, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(evL, s) == cudaSuccess &&
-         cudaStreamWaitEvent(st, evL, 0) == cudaSuccess;
-    if (evL) cudaEventDestroy(evL);
-    if (!ok) break;
-    if (!launch_gj<TV>(k.nb, k.cs, (int)list.size(), maxM, st, d_list, p, d_yOff, inv, d_y, d_info)) {
-      ok = false;
-      break;
-    }
+    ok = tmp.upload(&d_list, list, s) && launch_inversion<TV>(ci, k.nb, (int)list.size(), maxM, s, d_list, p, d_yOff, inv, d_y, d_info);
     c.launches += 1;
-    ok = cudaGetLastError() == cudaSuccess;
+    ok = ok && cudaGetLastError() == cudaSuccess;
   }
-  // the large blocks meanwhile, through cuSOLVER on its own streams
+  // the large blocks through cuSOLVER on its own streams
   if (ok && !big.empty()) {
     if constexpr (sizeof(TV) == 8) ok = factor_cusolver(c, p, big);
-  }
-  for (cudaStream_t st : ss) {
-    cudaEvent_t ev = nullptr;
-    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
-      cudaEventRecord(ev, st);
-      cudaStreamWaitEvent(s, ev, 0);
-      cudaEventDestroy(ev);
-    }
   }
   std::vector<int> info(p.nBlocks, 0);
   if (ok) ok = cudaMemcpyAsync(info.data(), d_info, info.size() * sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess;
   if (ok) ok = cudaStreamSynchronize(s) == cudaSuccess;
-  for (cudaStream_t st : ss) {
-    cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
-  }
-  cudaEventDestroy(evA);
   tmp.release();
   FB_CHECK(ok, "preconditioner inversion failed: %s", cudaGetErrorString(cudaGetLastError()));
   for (int b = 0; b < p.nBlocks; b++)
@@ -851,7 +1152,7 @@ bool precond_setup(Context &c, int mode) {
   StageTimer tm("precond_setup", s);
   if (!p.arena.upload(&p.d_start, p.hStart, s) || !p.arena.upload(&p.d_size, p.hSize, s) ||
       !p.arena.upload(&p.d_tiles, tiles, s) || !p.arena.upload(&p.d_off, p.hOff, s) ||
-      !p.arena.alloc_n(&p.d_colSrc, 2 * (size_t)c.n))
+      !p.arena.alloc_n(&p.d_colSrc, 2 * (size_t)c.n) || !p.arena.alloc_n(&p.d_rowDst, 2 * (size_t)c.n))
     return false;
   // FP64 contexts invert in FP64; mixed contexts assemble and invert in FP32
   // (the preconditioner only steers GMRES; its inverse is stored in FP32)
@@ -891,17 +1192,17 @@ bool precond_apply(Context &c, const double *b, double *x, bool adjoint) {
   if (p.mode == 2 && adjoint) {
     if (p.d_invF)
       pc_apply_t_kernel<float><<<p.nTiles, kPcWarps * 32, 0, c.stream>>>(c.n, p.d_tiles, p.d_start, p.d_size,
-                                                                             p.d_off, p.d_colSrc, p.d_invF, b, x);
+                                                                             p.d_off, p.d_colSrc, p.d_rowDst, p.d_invF, b, x);
     else
       pc_apply_t_kernel<double><<<p.nTiles, kPcWarps * 32, 0, c.stream>>>(c.n, p.d_tiles, p.d_start, p.d_size,
-                                                                              p.d_off, p.d_colSrc, p.d_inv, b, x);
+                                                                              p.d_off, p.d_colSrc, p.d_rowDst, p.d_inv, b, x);
   } else if (p.mode == 2) {
     if (p.d_invF)
       pc_apply_kernel<float><<<p.nTiles, kPcWarps * 32, 0, c.stream>>>(c.n, p.d_tiles, p.d_start, p.d_size,
-                                                                           p.d_off, p.d_colSrc, p.d_invF, b, x);
+                                                                           p.d_off, p.d_colSrc, p.d_rowDst, p.d_invF, b, x);
     else
       pc_apply_kernel<double><<<p.nTiles, kPcWarps * 32, 0, c.stream>>>(c.n, p.d_tiles, p.d_start, p.d_size,
-                                                                             p.d_off, p.d_colSrc, p.d_inv, b, x);
+                                                                             p.d_off, p.d_colSrc, p.d_rowDst, p.d_inv, b, x);
   } else if (p.mode == 3) {
     pc_diag_kernel<<<ceil_div(c.n, 256), 256, 0, c.stream>>>(c.n, c.d_area, (1.0 + c.epsilon) / 2.0,
                                                             (1.0 + 1.0 / c.epsilon) / 2.0, b, x);

@@ -1,0 +1,55 @@
+"""Preconditioner kernels at the sizes where their dispatch changes, against the FP64
+restatement oracle.
+
+Tolerances: FP64 operators 1e-12 and block inverses 1e-11 relative L2, as for the golden cases; block inverses of mixed
+contexts 1e-4 (FP32 inverses of well-conditioned blocks: rows * 2^-24 <= 1536 * 6e-8); mixed operators 5e-6.
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from fabipb_b200 import lib, meshgen, meshio
+from oracle import oracle as O
+from test_near_kernels import cut_sphere
+
+pytestmark = pytest.mark.gpu
+
+
+def patch_and_far_panel(panels):
+    """`panels` faces around a pole of the 5,120-panel sphere and one face far away: at depth 1 the patch is one leaf."""
+    unit, faces = meshgen.icosphere(4)
+    pan = meshio.build_panels(20.0 * unit, unit, faces)
+    z = pan.vtx[:, :, 2].mean(1)
+    keep = np.sort(np.argsort(-z)[:panels])
+    far = int(np.argmin(z))
+    vtx = np.concatenate([pan.vtx[keep], pan.vtx[far:far + 1] + np.array([300.0, 300.0, -300.0])])
+    keep = np.r_[keep, far]
+    return meshio.PanelSet(vtx, pan.normal[keep], pan.area[keep], pan.face_index[keep])
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-11), (lib.MIXED, 1e-4)])
+@pytest.mark.parametrize("panels", [1, 3, 4, 8, 9, 17, 191, 192, 193, 384, 385, 768, 769])
+def test_block_inverse_classes(panels, precision, tol):
+    """Blocks of 2 * panels rows on both sides of every class of the inversion, and of every batch of the application."""
+    pan = patch_and_far_panel(panels)
+    opts = dict(order=2, depth=1, height=1)
+    s, o = lib.Surface(pan, lib.params(precision=precision, **opts)), O.Oracle(pan, O.make_params(**opts))
+    assert sorted(s.leaf_layout()[1]) == [1, panels]
+    s.precond_setup(2)
+    o.precond_setup(2)
+    b = np.random.default_rng(panels).standard_normal(2 * s.n)
+    assert rel_l2(s.precond_apply(b), o.precond_apply(b)) < tol
+
+
+@pytest.mark.parametrize("panels,depth", [(5, 2), (331, 2), (643, 1)])
+def test_adjoint_block_application(panels, depth):
+    """The energy is quadratic in the charges, so q . dE/dq = 2 E; the transposed solve takes the forward one's steps."""
+    pan = cut_sphere(panels, seed=panels)
+    rng = np.random.default_rng(panels)
+    ch = meshio.ChargeSet(rng.uniform(-5, 5, (7, 3)), rng.standard_normal(7), np.ones(7))
+    s = lib.Surface(pan, lib.params(order=3, depth=depth, height=min(depth, 2), precision=lib.FP64), charges=ch)
+    s.precond_setup(2)
+    e, it, _, info = s.forward(restart=20, maxit=200, tol=1e-12)
+    dq, _, it_t, _, info_t = s.backward(1.0, restart=20, maxit=200, tol=1e-12)
+    assert info == 0 and info_t == 0 and abs(it - it_t) <= max(2, it // 4)
+    assert abs(dq @ ch.q - 2 * e) <= 1e-9 * abs(2 * e)
