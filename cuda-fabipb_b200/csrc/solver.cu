@@ -759,17 +759,26 @@ pc_apply_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ b
     __syncthreads();
     if (r < M) {
       const TI *col = Ib + (size_t)k0 * M + r;
-#pragma unroll 8
-      for (int c = warp; c < kn; c += kPcWarps) {
-        const V2 a = *reinterpret_cast<const V2 *>(col + (size_t)c * M);
-        const double xc = xs[c];
-        y0 += (double)a.x * xc;
-        y1 += (double)a.y * xc;
-        if (kPcRpl == 4 && q2) {
-          const V2 a2 = *reinterpret_cast<const V2 *>(col + (size_t)c * M + 2);
-          y2 += (double)a2.x * xc;
-          y3 += (double)a2.y * xc;
-        }
+      for (int c = warp; c < kn; c += 8 * kPcWarps) {
+        V2 lo[8], hi[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (c + u * kPcWarps < kn) {   // warp-uniform
+            const V2 *src = reinterpret_cast<const V2 *>(col + (size_t)(c + u * kPcWarps) * M);
+            lo[u] = src[0];
+            if (kPcRpl == 4 && q2) hi[u] = src[1];
+          }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (c + u * kPcWarps < kn) {
+            const double xc = xs[c + u * kPcWarps];
+            y0 += (double)lo[u].x * xc;
+            y1 += (double)lo[u].y * xc;
+            if (kPcRpl == 4 && q2) {
+              y2 += (double)hi[u].x * xc;
+              y3 += (double)hi[u].y * xc;
+            }
+          }
       }
     }
   }
@@ -795,8 +804,8 @@ pc_apply_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ b
 
 // Transposed block-diagonal apply (adjoint solves): output c of a block is
 // column c of its inverse dotted with the block's input.  Tiles of kPcRows
-// outputs; the block's input is staged in shared memory in chunks, a warp per
-// output column, each lane two consecutive rows per step.
+// outputs; the block's input is staged in shared memory in chunks, a warp takes
+// four output columns at a time, each lane two consecutive rows per step.
 template <typename TI>
 __global__ void __launch_bounds__(kPcWarps * 32)
 pc_apply_t_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__ bStart, const int *__restrict__ bSize,
@@ -821,18 +830,22 @@ pc_apply_t_kernel(int n, const int2 *__restrict__ tiles, const int *__restrict__
       xs[i] = (g < hm) ? rhs[st + g] : rhs[n + st + g - hm];
     }
     __syncthreads();
+    // four columns at a time: their loads overlap and share the staged input
 #pragma unroll
-    for (int q = 0; q < kCols; q++) {
-      const int c = c0 + warp + q * kPcWarps;
-      if (c < M) {
-        const TI *col = Ib + (size_t)c * M + k0;
-        double acc = 0.0;
-#pragma unroll 4
-        for (int i = 2 * lane; i < kn; i += 64) {   // kn is even
-          const V2 a = *reinterpret_cast<const V2 *>(col + i);
-          acc += (double)a.x * xs[i] + (double)a.y * xs[i + 1];
+    for (int q = 0; q < kCols; q += 4) {
+      if (c0 + warp + q * kPcWarps >= M) break;   // warp-uniform
+      const TI *col[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)   // (a column past the block: the last one again, dropped below)
+        col[u] = Ib + (size_t)min(c0 + warp + (q + u) * kPcWarps, M - 1) * M + k0;
+#pragma unroll 2
+      for (int i = 2 * lane; i < kn; i += 64) {   // kn is even
+        const double x0 = xs[i], x1 = xs[i + 1];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const V2 a = *reinterpret_cast<const V2 *>(col[u] + i);
+          y[q + u] += (double)a.x * x0 + (double)a.y * x1;
         }
-        y[q] += acc;
       }
     }
   }
