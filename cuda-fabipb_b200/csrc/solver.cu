@@ -51,6 +51,7 @@ struct PrecondDev {
   int restart = 0;
   double *d_V = nullptr, *d_r = nullptr, *d_av = nullptr, *d_w = nullptr;
   double *d_h = nullptr, *d_part = nullptr, *d_y = nullptr;
+  double *d_G = nullptr;                    // Gram entries of the current cycle's basis (row k: j < k)
   double *d_H = nullptr, *d_sv = nullptr;   // Hessenberg (+ cs, sn columns) and rotated residual vector
   void *d_status = nullptr;                 // GmresStatus on the device
   void *h_status = nullptr;                 // pinned host copy (and two host-read norms)
@@ -1320,38 +1321,113 @@ __device__ __forceinline__ void block_store_partial(double acc, double *red, dou
   if (threadIdx.x == 0) partOut[blockIdx.x] = red[0];
 }
 
-// One modified Gram-Schmidt column (gmres.c's ddot + daxpy pair) as a single
-// launch on kRedBlocks blocks: every block reduces the partials of
-// h_k = w.v_k in the same order, block 0 stores h_k, each block updates its
-// grid-stride share w -= h_k v_k and leaves its partial of the next product,
-// w.v_next (or w.w when v_next is null).  The grid partition is that of
-// dot_partial_kernel, so the values equal the separate dot/axpy sequence.
+// Modified Gram-Schmidt of one Arnoldi step (gmres.c's ddot + daxpy pairs) in
+// two passes over the basis whatever its length.  MGS takes h_k = v_k.(w -
+// sum_{j<k} h_j v_j); with the products c_k = v_k.w and the basis' own Gram
+// entries L_kj = v_k.v_j (j < k; rounding-sized, kept for the cycle) that is the
+// triangular solve (I + L) h = c, the one-reduction form of MGS of Swirydowicz,
+// Langou, Ananthan, Yang and Thomas (Numer. Linear Algebra Appl. 28, 2021).
+// gs_dots_kernel takes all products at once (and the newest column's Gram row),
+// gs_update_kernel solves and subtracts, mgs_norm_scale_kernel normalises and
+// takes the Givens step: three launches per step.  One launch per column
+// took 5.3 us each (20,000 panels: 529 us for the 19 steps of two solves); these
+// take 4.6, 4.7 and 5.0 us (271 us).
+constexpr int kGsCols = 8;   // columns per pass over w in gs_dots_kernel
+
+// part[k][block] = partial of w.v_k (k < i), part[i + k][block] = partial of v_{i-1}.v_k (k < i - 1)
 __global__ void __launch_bounds__(kRedThreads)
-mgs_step_kernel(long long n, const double *__restrict__ partIn, double *hk, const double *__restrict__ vk,
-                const double *__restrict__ vnext, double *w, double *partOut) {
-  __shared__ double red[kRedThreads];
-  const double h = block_sum_partials(partIn, red);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *hk = h;
-  const double a = -h;
-  double acc = 0.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double wi = w[i] + a * vk[i];
-    w[i] = wi;
-    acc += wi * (vnext ? vnext[i] : wi);
+gs_dots_kernel(long long n, int i, const double *__restrict__ V, const double *__restrict__ w, double *part) {
+  __shared__ double red[2 * kGsCols][kRedThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double *last = V + (size_t)(i - 1) * n;
+  for (int k0 = 0; k0 < i; k0 += kGsCols) {
+    double c[kGsCols], g[kGsCols];
+#pragma unroll
+    for (int q = 0; q < kGsCols; q++) c[q] = g[q] = 0.0;
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+      const double we = w[e], le = last[e];
+#pragma unroll
+      for (int q = 0; q < kGsCols; q++)
+        if (k0 + q < i) {   // uniform
+          const double v = V[(size_t)(k0 + q) * n + e];
+          c[q] += we * v;
+          g[q] += le * v;
+        }
+    }
+    __syncthreads();   // the previous columns' sums are read
+#pragma unroll
+    for (int q = 0; q < kGsCols; q++) {
+      for (int o = 16; o > 0; o >>= 1) {
+        c[q] += __shfl_xor_sync(0xffffffffu, c[q], o);
+        g[q] += __shfl_xor_sync(0xffffffffu, g[q], o);
+      }
+      if (lane == 0) {
+        red[q][warp] = c[q];
+        red[kGsCols + q][warp] = g[q];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kGsCols) {
+      const int q = threadIdx.x % kGsCols, gram = threadIdx.x / kGsCols;
+      if (k0 + q < i - gram) {
+        double s = 0.0;
+        for (int v = 0; v < kRedThreads / 32; v++) s += red[threadIdx.x][v];
+        part[(size_t)(gram * i + k0 + q) * gridDim.x + blockIdx.x] = s;
+      }
+    }
   }
-  block_store_partial(acc, red, partOut);
 }
 
-// h_i = sqrt(w.w) from the partials; v_i = w / h_i (w itself when h_i is 0)
+// every block: the sums of the partials in the same order, h from (I + L) h = c (block 0 stores h and the
+// newest Gram row), its share of w -= V h and the partial of w.w.  Dynamic shared memory: gs_smem(i) bytes; the
+// older Gram rows are read there up to kGsStage columns, from global memory above.
+constexpr int kGsStage = 64;
+static size_t gs_smem(int i) { return sizeof(double) * (i <= kGsStage ? (size_t)i * (i + 1) : 2 * (size_t)i); }
 __global__ void __launch_bounds__(kRedThreads)
-mgs_norm_scale_kernel(long long n, const double *__restrict__ partIn, double *hi, const double *__restrict__ w,
-                      double *v) {
+gs_update_kernel(long long n, int i, int ldg, const double *__restrict__ V, const double *__restrict__ part,
+                 double *G, double *hOut, double *w, double *partOut) {
+  extern __shared__ double gsSmem[];
   __shared__ double red[kRedThreads];
-  const double d = sqrt(block_sum_partials(partIn, red));
-  if (blockIdx.x == 0 && threadIdx.x == 0) *hi = d;
-  const double sc = (d > 0.0) ? 1.0 / d : 1.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    v[i] = (d > 0.0) ? w[i] * sc : w[i];
+  double *h = gsSmem, *row = gsSmem + i, *L = row + i;   // [i], the newest Gram row, the others [i - 1][i] (row k: j < k)
+  const bool staged = i <= kGsStage;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (staged)
+    for (int e = threadIdx.x; e < (i - 1) * i; e += blockDim.x) {
+      const int k = e / i, j = e % i;
+      if (j < k) L[e] = G[(size_t)k * ldg + j];
+    }
+  for (int q = warp; q < 2 * i - 1; q += kRedThreads / 32) {
+    double s = 0.0;
+    for (int b = lane; b < kRedBlocks; b += 32) s += part[(size_t)q * kRedBlocks + b];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      if (q < i) h[q] = s;
+      else row[q - i] = s;
+    }
+  }
+  __syncthreads();
+  if (warp == 0)   // forward substitution, column by column
+    for (int k = 0; k < i; k++) {
+      const double hk = h[k];
+      for (int j = k + 1 + lane; j < i; j += 32)
+        h[j] -= hk * (j == i - 1 ? row[k] : staged ? L[j * i + k] : G[(size_t)j * ldg + k]);
+      __syncwarp();
+    }
+  __syncthreads();
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < i; k += blockDim.x) {
+      hOut[k] = h[k];
+      if (k < i - 1) G[(size_t)(i - 1) * ldg + k] = row[k];
+    }
+  double acc = 0.0;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    double we = w[e];
+#pragma unroll 8
+    for (int k = 0; k < i; k++) we -= h[k] * V[(size_t)k * n + e];
+    w[e] = we;
+    acc += we * we;
+  }
+  block_store_partial(acc, red, partOut);
 }
 
 static bool dot_dev(Context &c, long long n, const double *x, const double *y, double *out, bool sq) {
@@ -1450,21 +1526,42 @@ __global__ void gmres_cycle_start_kernel(const double *__restrict__ part, int nP
   }
 }
 
-// One Givens step for column i (1-based, as src/gmres.c): H(:, i-1) = h,
-// previous rotations, the new rotation, s rotated, residual estimate.  A step
-// queued after the cycle ended (state != 0) changes nothing.
-__global__ void gmres_givens_kernel(const double *__restrict__ h, double *H, int ldh, int restrt, double *sv,
-                                    int i, int iters, int maxit, double bnrm2, double tol, GmresStatus *st) {
-  if (threadIdx.x != 0 || st->state != 0) return;
+// h_i = sqrt(w.w) from the partials; v_i = w / h_i (w itself when h_i is 0); then, in block 0, the Givens step
+// of column i (1-based, as src/gmres.c): H(:, i-1) = h, previous rotations, the new rotation, s rotated, residual
+// estimate.  A step queued after the cycle ended (state != 0) changes nothing in H and the status.
+__global__ void __launch_bounds__(kRedThreads)
+mgs_norm_scale_kernel(long long n, const double *__restrict__ partIn, const double *__restrict__ h,
+                      const double *__restrict__ w, double *v, double *H, int ldh, int restrt, double *sv, int i,
+                      int iters, int maxit, double bnrm2, double tol, GmresStatus *st) {
+  __shared__ double red[kRedThreads];
+  const double d = sqrt(block_sum_partials(partIn, red));
+  const double sc = (d > 0.0) ? 1.0 / d : 1.0;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+    v[e] = (d > 0.0) ? w[e] * sc : w[e];
+  if (blockIdx.x != 0 || threadIdx.x != 0 || st->state != 0) return;
   double *cs = H + (size_t)restrt * ldh, *sn = H + (size_t)(restrt + 1) * ldh;
   double *hc = H + (size_t)(i - 1) * ldh;
-  for (int k = 0; k <= i; k++) hc[k] = h[k];
-  for (int k = 0; k < i - 1; k++) drot_d(&hc[k], &hc[k + 1], cs[k], sn[k]);
-  double aa = hc[i - 1], bb = hc[i];
-  drotg_d(&aa, &bb, &cs[i - 1], &sn[i - 1]);
-  drot_d(&hc[i - 1], &hc[i], cs[i - 1], sn[i - 1]);
-  drot_d(&sv[i - 1], &sv[i], cs[i - 1], sn[i - 1]);
-  const double res = fabs(sv[i]) / bnrm2;
+  double cur = h[0];   // the rotated column's running entry
+  for (int k = 0; k < i - 1; k++) {
+    double nxt = h[k + 1];
+    drot_d(&cur, &nxt, cs[k], sn[k]);
+    hc[k] = cur;
+    cur = nxt;
+  }
+  double aa = cur, bb = d, cc, ss;
+  drotg_d(&aa, &bb, &cc, &ss);
+  cs[i - 1] = cc;
+  sn[i - 1] = ss;
+  double x = cur, y = d;
+  drot_d(&x, &y, cc, ss);
+  hc[i - 1] = x;
+  hc[i] = y;
+  x = sv[i - 1];
+  y = sv[i];
+  drot_d(&x, &y, cc, ss);
+  sv[i - 1] = x;
+  sv[i] = y;
+  const double res = fabs(y) / bnrm2;
   st->resid = res;
   st->i = i;
   st->iters = iters;
@@ -1549,8 +1646,8 @@ bool gmres_solve(Context &c, const double *b, double *x, int restrt, int maxit, 
     p.restart = restrt;
     if (!p.arena.alloc_n(&p.d_V, (size_t)n2 * (restrt + 1)) || !p.arena.alloc_n(&p.d_r, (size_t)n2) ||
         !p.arena.alloc_n(&p.d_av, (size_t)n2) || !p.arena.alloc_n(&p.d_w, (size_t)n2) ||
-        !p.arena.alloc_n(&p.d_h, (size_t)ldh + 1) || !p.arena.alloc_n(&p.d_part, 2 * (size_t)kRedBlocks + 2) ||
-        !p.arena.alloc_n(&p.d_y, (size_t)restrt + 1) || !p.arena.alloc_n(&p.d_H, (size_t)ldh * (restrt + 2)) ||
+        !p.arena.alloc_n(&p.d_h, (size_t)ldh + 1) || !p.arena.alloc_n(&p.d_part, (2 * (size_t)restrt + 2) * kRedBlocks + 2) ||
+        !p.arena.alloc_n(&p.d_G, (size_t)restrt * restrt) || !p.arena.alloc_n(&p.d_y, (size_t)restrt + 1) || !p.arena.alloc_n(&p.d_H, (size_t)ldh * (restrt + 2)) ||
         !p.arena.alloc_n(&p.d_sv, (size_t)restrt + 2) || !p.arena.alloc(&p.d_status, sizeof(GmresStatus)))
       return false;
     if (!p.h_status) FB_CUDA(cudaMallocHost(&p.h_status, 4 * sizeof(GmresStatus)));
@@ -1619,20 +1716,14 @@ bool gmres_solve(Context &c, const double *b, double *x, int restrt, int maxit, 
       *steps = it;
       if (!op_matvec(c, 1.0, p.d_V + (size_t)(i - 1) * n2, 0.0, p.d_av, adjoint)) return false;
       if (!precond_apply(c, p.d_av, p.d_w, adjoint)) return false;
-      // modified Gram-Schmidt: h[k] = w.v_k; w -= h[k] v_k, one launch per
-      // column with the partial sums ping-ponged between two buffers
-      double *partA = p.d_part, *partB = p.d_part + kRedBlocks;
-      dot_partial_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, p.d_w, p.d_V, partA);
-      for (int k = 0; k < i; k++) {
-        const double *vnext = (k + 1 < i) ? p.d_V + (size_t)(k + 1) * n2 : nullptr;
-        mgs_step_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, partA, p.d_h + k, p.d_V + (size_t)k * n2, vnext,
-                                                           p.d_w, partB);
-        std::swap(partA, partB);
-      }
-      mgs_norm_scale_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, partA, p.d_h + i, p.d_w,
-                                                               p.d_V + (size_t)i * n2);
-      gmres_givens_kernel<<<1, 32, 0, s>>>(p.d_h, p.d_H, ldh, restrt, p.d_sv, i, it, maxit, bnrm2, tol, d_st);
-      c.launches += i + 3;
+      // modified Gram-Schmidt of w against v_0 .. v_{i-1}, then the Givens step
+      double *norm = p.d_part + 2 * (size_t)restrt * kRedBlocks;
+      gs_dots_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, i, p.d_V, p.d_w, p.d_part);
+      gs_update_kernel<<<kRedBlocks, kRedThreads, gs_smem(i), s>>>(n2, i, restrt, p.d_V, p.d_part, p.d_G, p.d_h, p.d_w,
+                                                                 norm);
+      mgs_norm_scale_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, norm, p.d_h, p.d_w, p.d_V + (size_t)i * n2, p.d_H,
+                                                               ldh, restrt, p.d_sv, i, it, maxit, bnrm2, tol, d_st);
+      c.launches += 3;
       FB_CUDA(cudaGetLastError());
       if (!read_status(c, d_st, h_st)) return false;
       *resid = h_st->resid;

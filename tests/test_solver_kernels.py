@@ -1,4 +1,4 @@
-"""Preconditioner kernels at the sizes where their dispatch changes, against the FP64
+"""Preconditioner and GMRES kernels at the sizes where their dispatch changes, against the FP64
 restatement oracle.
 
 Tolerances: FP64 operators 1e-12 and block inverses 1e-11 relative L2, as for the golden cases; block inverses of mixed
@@ -53,3 +53,31 @@ def test_adjoint_block_application(panels, depth):
     dq, _, it_t, _, info_t = s.backward(1.0, restart=20, maxit=200, tol=1e-12)
     assert info == 0 and info_t == 0 and abs(it - it_t) <= max(2, it // 4)
     assert abs(dq @ ch.q - 2 * e) <= 1e-9 * abs(2 * e)
+
+
+def graded_spheres():
+    """Five 80-panel spheres whose panel areas span 1 to 0.1: without a preconditioner a hundred steps and more."""
+    unit, faces = meshgen.icosphere(1)
+    parts = []
+    for i in range(5):
+        at = np.array([60 * np.cos(0.7 * i), 60 * np.sin(0.7 * i), 10 * i]) * 0.75 ** i
+        parts.append(meshio.build_panels(20 * 0.75 ** i * unit + at, unit, faces))
+    return meshio.PanelSet(*(np.concatenate([getattr(p, f) for p in parts])
+                             for f in ("vtx", "normal", "area", "face_index")))
+
+
+@pytest.mark.parametrize("restart", [1, 2, 10, 63, 64, 65, 90])
+def test_gmres_restart_lengths(restart):
+    """A hundred steps in cycles of one column, of a few and of more than one staged group of columns, ended before they
+    converge: the oracle's iterate.  A relative change of 1e-16 in the right-hand side moves it by 1e-10 at restart 1 and
+    by 1e-12 above; operators that agree to 1e-15 leave it within 1e-8."""
+    pan = graded_spheres()
+    opts = dict(order=3, depth=3, height=2)
+    s, o = lib.Surface(pan, lib.params(precision=lib.FP64, **opts)), O.Oracle(pan, O.make_params(**opts))
+    b = np.random.default_rng(3).standard_normal(2 * s.n)
+    s.precond_setup(-1)
+    o.precond_setup(-1)
+    x, it, res, info = s.solve(b, b.copy(), restart=restart, maxit=100, tol=1e-14)
+    xr, itr, resr, infor = o.gmres(b, b.copy(), restart, 100, 1e-14)
+    assert (it, info) == (itr, infor) and abs(res - resr) <= 1e-6 * resr
+    assert rel_l2(x, xr) < 1e-8
