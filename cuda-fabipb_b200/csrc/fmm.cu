@@ -20,7 +20,6 @@
 #include <cmath>
 #include <vector>
 
-#include <type_traits>
 #include <utility>
 
 #include "context.cuh"
@@ -37,9 +36,6 @@ __constant__ double c_ifact3[kTabN];
 __constant__ double c_sgn3[kTabN];
 __constant__ double c_fact[kTabOrder + 4];
 __constant__ double c_ifact[kTabOrder + 4];
-// copies for reads at an index that differs from lane to lane
-__device__ int g_mi[kTabN];             // i1 | i2 << 8 | i3 << 16 | (i1 + i2 + i3) << 24
-__device__ double g_ifact3[kTabN];
 
 __device__ __forceinline__ int IDX(int a, int b, int c) { return c_idx3[(a * kTabDim + b) * kTabDim + c]; }
 
@@ -78,10 +74,6 @@ static bool upload_tables() {
   FB_CUDA(cudaMemcpyToSymbol(c_idx3, h.idx3.data(), h.idx3.size() * sizeof(short)));
   FB_CUDA(cudaMemcpyToSymbol(c_mi, h.mi.data(), h.mi.size() * sizeof(char4)));
   FB_CUDA(cudaMemcpyToSymbol(c_ifact3, h.ifact3.data(), h.ifact3.size() * sizeof(double)));
-  std::vector<int> mi(h.mi.size());
-  for (size_t k = 0; k < mi.size(); k++) mi[k] = h.mi[k].x | h.mi[k].y << 8 | h.mi[k].z << 16 | h.mi[k].w << 24;
-  FB_CUDA(cudaMemcpyToSymbol(g_mi, mi.data(), mi.size() * sizeof(int)));
-  FB_CUDA(cudaMemcpyToSymbol(g_ifact3, h.ifact3.data(), h.ifact3.size() * sizeof(double)));
   FB_CUDA(cudaMemcpyToSymbol(c_sgn3, h.sgn3.data(), h.sgn3.size() * sizeof(double)));
   FB_CUDA(cudaMemcpyToSymbol(c_fact, h.fact.data(), h.fact.size() * sizeof(double)));
   FB_CUDA(cudaMemcpyToSymbol(c_ifact, h.ifact.data(), h.ifact.size() * sizeof(double)));
@@ -239,26 +231,6 @@ __global__ void leaf_moments_kernel(int n, int order, const double *__restrict__
 // per-matvec passes
 // ------------------------------------------------------------------------
 
-// Lane l ends with the warp total of v[(l >> 1) & 15]: one butterfly over
-// sixteen values (8 + 4 + 2 + 1 + 1 shuffles), whose first stages carry
-// several independent shuffles each.
-template <typename T>
-__device__ __forceinline__ T warp_sum16(const T (&v)[16], int lane) {
-  const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
-  T w[8], x[4], y[2];
-#pragma unroll
-  for (int i = 0; i < 8; i++)
-    w[i] = (h16 ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[i + 8], 16);
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-    x[i] = (h8 ? w[i + 4] : w[i]) + __shfl_xor_sync(0xffffffffu, h8 ? w[i] : w[i + 4], 8);
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-    y[i] = (h4 ? x[i + 2] : x[i]) + __shfl_xor_sync(0xffffffffu, h4 ? x[i] : x[i + 2], 4);
-  T z = (h2 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, h2 ? y[0] : y[1], 2);
-  return z + __shfl_xor_sync(0xffffffffu, z, 1);
-}
-
 // Q2M: one block per leaf, warp w sums rows m = w, w+8, ... over the leaf panels
 // swap = 1 reads the two halves of sgm exchanged (the adjoint of L2P:
 // momPot <- Q1 . second half, momDpdn <- Q0 . first half).
@@ -295,29 +267,7 @@ __global__ void q2m_kernel(int nLeaves, int n, int NMleaf, int NM, const int *__
 // w, w + 8, ... when a cube had more than eight), lanes over the output
 // coefficients; the warps' shifted moments are added in warp order.
 // L2L: one warp per child cube, eight cubes per block.
-// Both are chains of dependent loads and a few hundred FMAs per cube: the
-// shift vector's powers are formed once per warp, the tables read at lane-varying
-// indices come from global memory (constant memory serialises them), and the
-// term loops have known bounds, so that their loads overlap.  Before: SHIFT_BEFORE; now SHIFT_AFTER.
 constexpr int kShiftWarps = 8;
-
-// a[e] = t^g / g! over the multi-indices g of e < ne (setupConVect, src/moments.c:390-410); one warp,
-// which synchronises before its first use; pw: 3 x (kMaxOrder + 1) values of its own
-__device__ __forceinline__ void warp_conv_entries(const double *t, int order, int ne, int lane, double *pw, double *a) {
-  if (lane < 3) {
-    double f = 1.0;
-    for (int k = 0; k <= order; k++) {
-      pw[lane * (kMaxOrder + 1) + k] = f;
-      f *= t[lane];
-    }
-  }
-  __syncwarp();
-  for (int e = lane; e < ne; e += 32) {
-    const int m = g_mi[e];
-    a[e] = pw[m & 255] * pw[kMaxOrder + 1 + ((m >> 8) & 255)] * pw[2 * (kMaxOrder + 1) + ((m >> 16) & 255)] *
-           g_ifact3[e];
-  }
-}
 
 __global__ void __launch_bounds__(kShiftWarps * 32)
 m2m_kernel(int first, int count, int NM, int ordOut, int ordIn, const int *__restrict__ kidFirst,
@@ -326,7 +276,6 @@ m2m_kernel(int first, int count, int NM, int ordOut, int ordIn, const int *__res
   // per warp: shift entries a, child moments b1, b2, and the child's shifted
   // contribution o1, o2 (nOut each); then the term list (offsets, entries)
   extern __shared__ double sm[];
-  __shared__ double pw[kShiftWarps][3 * (kMaxOrder + 1)];
   if ((int)blockIdx.x >= count) return;
   const int f = first + blockIdx.x;
   const int nOut = nmom(ordOut), nIn = nmom(ordIn);
@@ -343,17 +292,15 @@ m2m_kernel(int first, int count, int NM, int ordOut, int ordIn, const int *__res
     const double t[3] = {ctr[3 * kid] - ctr[3 * f], ctr[3 * kid + 1] - ctr[3 * f + 1],
                          ctr[3 * kid + 2] - ctr[3 * f + 2]};
     __syncwarp();   // the previous child's reads of a, b1, b2 are done
-    warp_conv_entries(t, ordOut, nOut, lane, pw[warp], a);
     for (int e = lane; e < nOut; e += 32) {
+      a[e] = conv_entry(t, e);
       b1[e] = (e < nIn) ? momPot[(size_t)kid * NM + e] : 0.0;
       b2[e] = (e < nIn) ? momDpdn[(size_t)kid * NM + e] : 0.0;
     }
     __syncwarp();
     for (int al = lane; al < nOut; al += 32) {
       double s1 = 0.0, s2 = 0.0;
-      const int q1 = lstOff[al + 1];
-#pragma unroll 4
-      for (int q = lstOff[al]; q < q1; q++) {
+      for (int q = lstOff[al]; q < lstOff[al + 1]; q++) {
         const int ent = lst[q];
         const int ia = ent & 1023, ib = (ent >> 10) & 1023;
         s1 += a[ia] * b1[ib];
@@ -720,6 +667,14 @@ struct M2LTensors<PM, TV, true> {
 // bank conflicts.
 __device__ __forceinline__ int m2l_slot(int e, int j) { return e * 32 + (j ^ (e & 31)); }
 
+// One (alpha, beta) entry.  FULL: the cube's order is PM, every entry counts.
+// The four sums of a coefficient are reduced over the lanes (component v's
+// total lands in lane 8v) and added to the warp's shared sums sAcc[v][alpha].
+template <typename TV>
+struct M2LSumsT {
+  TV s1, s2, s3, s4;
+};
+
 // Moment readers of the conv.  M2LColMoments: the XOR-swizzled columns staged
 // by plain loads.  M2LRowMoments: the lane's source row of (pot, dpdn) float2
 // entries staged by bulk copies, read as float4 (entries IB, IB+1) at even IB;
@@ -747,21 +702,66 @@ struct M2LRowMoments {
   }
 };
 
-// One (alpha, beta) step of the conv.  FULL: the cube's order is PM, every entry counts.  The four sums of four
-// consecutive output coefficients are reduced together by warp_sum16 (16 shuffles for 16 sums instead of 24, and
-// independent shuffle chains), lane 2j (j = 4 slot + component) adding sum j to the warp's shared sums sAcc[j & 3][alpha].
-template <typename TV>
-struct M2LSums16 {
-  TV s1, s2, s3, s4;
-  TV b[16];   // [slot of alpha mod 4][component]
-};
 template <int PM, int Q, bool FULL, bool ADJ, typename TV, typename TT, typename TM>
-__device__ __forceinline__ void m2l_step16(M2LSums16<TV> &S, TM &M, const TT &T, int lane, int order, double *sAcc) {
+__device__ __forceinline__ void m2l_step(M2LSumsT<TV> &S, TM &M, const TT &T, int lane, int order, double *sAcc) {
   constexpr M2LEntry E = m2l_entry<PM>(Q);
   if (E.first) S.s1 = S.s2 = S.s3 = S.s4 = (TV)0;
   if (FULL || E.dsum <= order) {
     const typename Vec2<TV>::t mo = M.template get<E.ib>();
     const typename Vec2<TV>::t d = T.get(E.ig, lane);
+    if ((ADJ ? E.dal : E.dsum - E.dal) & 1) {   // (-1)^|input|, or (-1)^|output| transposed
+      S.s1 -= mo.y * d.x; S.s2 -= mo.y * d.y; S.s3 -= mo.x * d.x; S.s4 -= mo.x * d.y;
+    } else {
+      S.s1 += mo.y * d.x; S.s2 += mo.y * d.y; S.s3 += mo.x * d.x; S.s4 += mo.x * d.y;
+    }
+  }
+  if (E.last && (FULL || E.dal <= order)) {
+    const TV t = warp_sum4<TV>(S.s1, S.s2, S.s3, S.s4, lane);
+    if ((lane & 7) == 0) sAcc[(lane >> 3) * nmom_c(PM) + E.al] += (double)t;
+  }
+}
+
+template <int PM, bool FULL, bool ADJ, typename TV, typename TT, typename TM, int... Q>
+__device__ __forceinline__ void m2l_steps(std::integer_sequence<int, Q...>, M2LSumsT<TV> &S, TM &M, const TT &T,
+                                          int lane, int order, double *sAcc) {
+  (m2l_step<PM, Q, FULL, ADJ, TV, TT, TM>(S, M, T, lane, order, sAcc), ...);
+}
+
+// Lane l ends with the warp total of v[(l >> 1) & 15]: one butterfly over
+// sixteen values (8 + 4 + 2 + 1 + 1 shuffles), whose first stages carry
+// several independent shuffles each.
+__device__ __forceinline__ float warp_sum16(const float (&v)[16], int lane) {
+  const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
+  float w[8], x[4], y[2];
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+    w[i] = (h16 ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[i + 8], 16);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    x[i] = (h8 ? w[i + 4] : w[i]) + __shfl_xor_sync(0xffffffffu, h8 ? w[i] : w[i + 4], 8);
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+    y[i] = (h4 ? x[i + 2] : x[i]) + __shfl_xor_sync(0xffffffffu, h4 ? x[i] : x[i + 2], 4);
+  float z = (h2 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, h2 ? y[0] : y[1], 2);
+  return z + __shfl_xor_sync(0xffffffffu, z, 1);
+}
+
+// The bulk-staged M2L's (alpha, beta) step: the conv of m2l_step (FP32), with
+// the four sums of four consecutive output coefficients reduced together by
+// warp_sum16 (16 shuffles for 16 sums instead of 24, and independent shuffle
+// chains), lane 2j (j = 4 slot + component) adding sum j to its coefficient.
+struct M2LSums16 {
+  float s1, s2, s3, s4;
+  float b[16];   // [slot of alpha mod 4][component]
+};
+template <int PM, int Q, bool FULL, bool ADJ, typename TT>
+__device__ __forceinline__ void m2l_step16(M2LSums16 &S, M2LRowMoments &M, const TT &T, int lane, int order,
+                                           double *sAcc) {
+  constexpr M2LEntry E = m2l_entry<PM>(Q);
+  if (E.first) S.s1 = S.s2 = S.s3 = S.s4 = 0.f;
+  if (FULL || E.dsum <= order) {
+    const float2 mo = M.template get<E.ib>();
+    const float2 d = T.get(E.ig, lane);
     if ((ADJ ? E.dal : E.dsum - E.dal) & 1) {   // (-1)^|input|, or (-1)^|output| transposed
       S.s1 -= mo.y * d.x; S.s2 -= mo.y * d.y; S.s3 -= mo.x * d.x; S.s4 -= mo.x * d.y;
     } else {
@@ -776,16 +776,16 @@ __device__ __forceinline__ void m2l_step16(M2LSums16<TV> &S, TM &M, const TT &T,
     S.b[4 * slot + 3] = S.s4;
     if constexpr (slot == 3 || E.al == nmom_c(PM) - 1) {
       // a last group of fewer than four: the slots past E.al are reduced, not written
-      const TV t = warp_sum16<TV>(S.b, lane);
+      const float t = warp_sum16(S.b, lane);
       const int j = (lane >> 1) & 15, al = (E.al & ~3) + (j >> 2);
       if (!(lane & 1) && al <= E.al && (FULL || c_mi[al].w <= order)) sAcc[(j & 3) * nmom_c(PM) + al] += (double)t;
     }
   }
 }
-template <int PM, bool FULL, bool ADJ, typename TV, typename TT, typename TM, int... Q>
-__device__ __forceinline__ void m2l_steps16(std::integer_sequence<int, Q...>, M2LSums16<TV> &S, TM &M, const TT &T,
-                                            int lane, int order, double *sAcc) {
-  (m2l_step16<PM, Q, FULL, ADJ, TV, TT, TM>(S, M, T, lane, order, sAcc), ...);
+template <int PM, bool FULL, bool ADJ, typename TT, int... Q>
+__device__ __forceinline__ void m2l_steps16(std::integer_sequence<int, Q...>, M2LSums16 &S, M2LRowMoments &M,
+                                            const TT &T, int lane, int order, double *sAcc) {
+  (m2l_step16<PM, Q, FULL, ADJ, TT>(S, M, T, lane, order, sAcc), ...);
 }
 
 // The lane's FP32 M2L tensor (packed D^e G0, D^e Gk) from its pair's offset x =
@@ -815,9 +815,7 @@ __device__ __forceinline__ void m2l_gen_tensor(const float x[3], bool live, floa
 // ADJ: the transposed interaction, as for m2l_kernel.  TV = float: tensors
 // (float2) and staged moments in FP32, each batch's per-coefficient sums in
 // FP32, accumulated over the batches in FP64.
-// SPLIT (few cubes): a block takes one cube, its warps the cube's batches in turn, and their sums are added at the
-// end; else a warp takes a cube.
-template <int PM, bool ADJ, typename TV, bool SPLIT>
+template <int PM, bool ADJ, typename TV>
 __global__ void __launch_bounds__(M2LUnrolledShape<PM, TV>::W * 32,
                                   PM >= 5 ? 1 : (sizeof(TV) == 4 ? FB_M2L_MIN_BLOCKS_F32 : FB_M2L_MIN_BLOCKS))
 m2l_unrolled_kernel(int nDst, const int *__restrict__ dstList, const int *__restrict__ m2lOff,
@@ -834,14 +832,13 @@ m2l_unrolled_kernel(int nDst, const int *__restrict__ dstList, const int *__rest
   char *wbase = reinterpret_cast<char *>(m2luSmem) + (size_t)warp * Sh::warpBytes;
   V2 *sC = reinterpret_cast<V2 *>(wbase);
   double *sAcc = reinterpret_cast<double *>(wbase + Sh::colBytes);   // [4][NMP]
-  const int bi = SPLIT ? (int)blockIdx.x : (int)blockIdx.x * Sh::W + warp;
-  if (bi >= nDst) return;  // warp-uniform (block-uniform when split)
+  const int bi = blockIdx.x * Sh::W + warp;
+  if (bi >= nDst) return;  // warp-uniform
   const int f = dstList[bi];
   const int order = ordOfCube[f];
   const int o0 = m2lOff[f], o1 = m2lOff[f + 1];
   for (int e = lane; e < 4 * NMP; e += 32) sAcc[e] = 0.0;
-  constexpr int kStep = SPLIT ? 32 * Sh::W : 32;
-  for (int b0 = o0 + (SPLIT ? 32 * warp : 0); b0 < o1; b0 += kStep) {
+  for (int b0 = o0; b0 < o1; b0 += 32) {
     const int k = b0 + lane;
     const bool live = k < o1;
     const int nb = min(32, o1 - b0);
@@ -892,29 +889,20 @@ m2l_unrolled_kernel(int nDst, const int *__restrict__ dstList, const int *__rest
       for (int e = 0; e < NMP; e++) T.v[e] = tp[(size_t)e * nPairs];
     }
     __syncwarp();
-    M2LSums16<TV> S{};
+    M2LSumsT<TV> S{(TV)0, (TV)0, (TV)0, (TV)0};
     M2LColMoments<V2> M{sC, lane};
     if (order == PM)
-      m2l_steps16<PM, true, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
+      m2l_steps<PM, true, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order,
+                                   sAcc);
     else
-      m2l_steps16<PM, false, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
+      m2l_steps<PM, false, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order,
+                                    sAcc);
   }
-  if (SPLIT) __syncthreads();
-  else __syncwarp();
+  __syncwarp();
   const int nm = ((order + 1) * (order + 2) * (order + 3)) / 6;
   const double ieps = 1.0 / eps;
-  for (int e = SPLIT ? threadIdx.x : lane; e < nm; e += kStep) {
-    double S1 = 0.0, S2 = 0.0, S3 = 0.0, S4 = 0.0;
-#pragma unroll
-    for (int w = 0; w < (SPLIT ? Sh::W : 1); w++) {
-      const double *acc = SPLIT ? reinterpret_cast<const double *>(reinterpret_cast<const char *>(m2luSmem) +
-                                                                   (size_t)w * Sh::warpBytes + Sh::colBytes)
-                                : sAcc;
-      S1 += acc[e];
-      S2 += acc[NMP + e];
-      S3 += acc[2 * NMP + e];
-      S4 += acc[3 * NMP + e];
-    }
+  for (int e = lane; e < nm; e += 32) {
+    const double S1 = sAcc[e], S2 = sAcc[NMP + e], S3 = sAcc[2 * NMP + e], S4 = sAcc[3 * NMP + e];
     const size_t o = (size_t)f * NM + e;
     if (ADJ) {   // sign already folded in
       lec1[o] += eps * S2 - S1 - S3 + S4;
@@ -1017,25 +1005,21 @@ __device__ __forceinline__ void m2l_bulk_issue(int nb, int sj, int lane, const f
   if (lane < nb) bulk_g2s(buf + lane * Sh::RS, momF + (size_t)sj * Sh::NMS, Sh::NMS * sizeof(float2), bar);
 }
 
-// NW warps per destination cube, which take its batches in turn (several when there are few cubes)
-template <int PM, bool ADJ, int NW>
-__global__ void __launch_bounds__(32 * NW, M2LBulkShape<PM>::MINB / NW < 1 ? 1 : M2LBulkShape<PM>::MINB / NW)
+template <int PM, bool ADJ>
+__global__ void __launch_bounds__(32, M2LBulkShape<PM>::MINB)
 m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff, const int *__restrict__ m2lSrc,
                 const int *__restrict__ ordOfCube, const double *__restrict__ ctr, float kappa, int NM, double eps,
                 const float2 *__restrict__ momF, double *lec1, double *lec2, double *lec3, double *lec4) {
   typedef M2LBulkShape<PM> Sh;
   constexpr int NMP = Sh::NMP;
   extern __shared__ __align__(16) unsigned char m2lbSmem[];
-  constexpr int kStep = 32 * NW;
-  constexpr size_t kWarpBytes = (Sh::bytes + 15) & ~(size_t)15;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char *base = m2lbSmem + warp * kWarpBytes;
-  float2 *buf = reinterpret_cast<float2 *>(base);   // [2][32][RS]
-  double *sAcc = reinterpret_cast<double *>(base + Sh::accOff);   // [4][NMP]
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(base + Sh::barOff);
+  float2 *buf = reinterpret_cast<float2 *>(m2lbSmem);   // [2][32][RS]
+  double *sAcc = reinterpret_cast<double *>(m2lbSmem + Sh::accOff);   // [4][NMP]
+  unsigned long long *bar = reinterpret_cast<unsigned long long *>(m2lbSmem + Sh::barOff);
+  const int lane = threadIdx.x;
   const int f = dstList[blockIdx.x];
   const int order = ordOfCube[f];
-  const int oBeg = m2lOff[f], o0 = oBeg + 32 * warp, o1 = m2lOff[f + 1];
+  const int o0 = m2lOff[f], o1 = m2lOff[f + 1];
   for (int e = lane; e < 4 * NMP; e += 32) sAcc[e] = 0.0;
   if (lane == 0) {
     mbar_init(&bar[0], 1);
@@ -1046,18 +1030,18 @@ m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff,
   const double cf0 = ctr[3 * f], cf1 = ctr[3 * f + 1], cf2 = ctr[3 * f + 2];
   // batch 0 in flight; batch 1's sources and batch 0's centres loaded
   int srcCur = o0 + lane < o1 ? m2lSrc[o0 + lane] : 0;
-  if (o0 < o1) m2l_bulk_issue<PM>(min(32, o1 - o0), srcCur, lane, momF, buf, &bar[0]);   // warp-uniform
-  int srcNext = o0 + kStep + lane < o1 ? m2lSrc[o0 + kStep + lane] : 0;
+  m2l_bulk_issue<PM>(min(32, o1 - o0), srcCur, lane, momF, buf, &bar[0]);
+  int srcNext = o0 + 32 + lane < o1 ? m2lSrc[o0 + 32 + lane] : 0;
   double cs0 = ctr[3 * srcCur], cs1 = ctr[3 * srcCur + 1], cs2 = ctr[3 * srcCur + 2];
   unsigned phase = 0;   // bit s: the parity to wait for on bar[s]
   bool bad = false;
   int it = 0;
-  for (int b0 = o0; b0 < o1; b0 += kStep, it++) {
+  for (int b0 = o0; b0 < o1; b0 += 32, it++) {
     const int s = it & 1;
     const bool live = b0 + lane < o1;
-    const bool more = b0 + kStep < o1;
-    if (more) m2l_bulk_issue<PM>(min(32, o1 - b0 - kStep), srcNext, lane, momF, buf + (s ^ 1) * 32 * Sh::RS, &bar[s ^ 1]);
-    const int srcNext2 = b0 + 2 * kStep + lane < o1 ? m2lSrc[b0 + 2 * kStep + lane] : 0;
+    const bool more = b0 + 32 < o1;
+    if (more) m2l_bulk_issue<PM>(min(32, o1 - b0 - 32), srcNext, lane, momF, buf + (s ^ 1) * 32 * Sh::RS, &bar[s ^ 1]);
+    const int srcNext2 = b0 + 64 + lane < o1 ? m2lSrc[b0 + 64 + lane] : 0;
     const double cn0 = ctr[3 * srcNext], cn1 = ctr[3 * srcNext + 1], cn2 = ctr[3 * srcNext + 2];
     // the lane's tensor from the pair's offset (forward: x_dst - x_src; transposed: the
     // forward pair's cubes, x_src - x_dst here)
@@ -1082,21 +1066,20 @@ m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff,
     }
     // a lane past the batch reads row 0 (finite moments) with its zero tensor
     M2LRowMoments M{buf + s * 32 * Sh::RS + (live ? lane : 0) * Sh::RS, make_float4(0.f, 0.f, 0.f, 0.f)};
-    M2LSums16<float> S{};
+    M2LSums16 S{};
     if (order == PM)
-      m2l_steps16<PM, true, ADJ, float>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
+      m2l_steps16<PM, true, ADJ>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
     else
-      m2l_steps16<PM, false, ADJ, float>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
+      m2l_steps16<PM, false, ADJ>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
     srcNext = srcNext2;
     cs0 = cn0; cs1 = cn1; cs2 = cn2;
   }
-  if (bad && lane == 0) atomicAdd(&g_m2lStalls, 1u);
-  if (NW > 1) bad = __syncthreads_or(bad);
-  else __syncwarp();
+  __syncwarp();
   const int nm = ((order + 1) * (order + 2) * (order + 3)) / 6;
   if (bad) {
+    if (lane == 0) atomicAdd(&g_m2lStalls, 1u);
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    for (int e = threadIdx.x; e < nm; e += kStep) {
+    for (int e = lane; e < nm; e += 32) {
       const size_t o = (size_t)f * NM + e;
       lec1[o] = nan;
       lec2[o] = nan;
@@ -1108,16 +1091,8 @@ m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff,
     return;
   }
   const double ieps = 1.0 / eps;
-  for (int e = threadIdx.x; e < nm; e += kStep) {
-    double S1 = 0.0, S2 = 0.0, S3 = 0.0, S4 = 0.0;
-#pragma unroll
-    for (int w = 0; w < NW; w++) {   // the warps' sums
-      const double *acc = reinterpret_cast<const double *>(m2lbSmem + w * kWarpBytes + Sh::accOff);
-      S1 += acc[e];
-      S2 += acc[NMP + e];
-      S3 += acc[2 * NMP + e];
-      S4 += acc[3 * NMP + e];
-    }
+  for (int e = lane; e < nm; e += 32) {
+    const double S1 = sAcc[e], S2 = sAcc[NMP + e], S3 = sAcc[2 * NMP + e], S4 = sAcc[3 * NMP + e];
     const size_t o = (size_t)f * NM + e;
     if (ADJ) {   // sign already folded in
       lec1[o] += eps * S2 - S1 - S3 + S4;
@@ -1149,7 +1124,6 @@ l2l_kernel(int first, int count, int NM, int ordIn, int ordOut, const int *__res
   // per warp: shift entries a and the parent's locals i1..i4 (nIn each); then
   // the term list (offsets, entries)
   extern __shared__ double sm[];
-  __shared__ double pw[kShiftWarps][3 * (kMaxOrder + 1)];
   const int nIn = nmom(ordIn), nOut = nmom(ordOut);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int *lstOff = reinterpret_cast<int *>(sm + (size_t)kShiftWarps * 5 * nIn), *lst = lstOff + nOut + 1;
@@ -1162,8 +1136,8 @@ l2l_kernel(int first, int count, int NM, int ordIn, int ordOut, const int *__res
   const int f = first + cube;
   const int p = parent[f];
   const double t[3] = {ctr[3 * f] - ctr[3 * p], ctr[3 * f + 1] - ctr[3 * p + 1], ctr[3 * f + 2] - ctr[3 * p + 2]};
-  warp_conv_entries(t, ordIn, nIn, lane, pw[warp], a);
   for (int e = lane; e < nIn; e += 32) {
+    a[e] = conv_entry(t, e);
     i1[e] = lec1[(size_t)p * NM + e];
     i2[e] = lec2[(size_t)p * NM + e];
     i3[e] = lec3[(size_t)p * NM + e];
@@ -1171,14 +1145,12 @@ l2l_kernel(int first, int count, int NM, int ordIn, int ordOut, const int *__res
   }
   __syncwarp();
   for (int al = lane; al < nOut; al += 32) {
-    // beta runs in graded order: those of degree up to ordIn - |alpha|
-    const int left = ordIn - (g_mi[al] >> 24);
-    const int q0 = lstOff[al], q1 = min(lstOff[al + 1], q0 + (left < 0 ? 0 : nmom(left)));
+    const int degA = c_mi[al].w;
     double t1 = 0.0, t2 = 0.0, t3 = 0.0, t4 = 0.0;
-#pragma unroll 4
-    for (int q = q0; q < q1; q++) {
+    for (int q = lstOff[al]; q < lstOff[al + 1]; q++) {
       const int ent = lst[q];
-      const int ib = ent & 1023, ig = (ent >> 10) & 1023;
+      const int ib = ent & 1023, ig = (ent >> 10) & 1023, db = ent >> 20;
+      if (db > ordIn - degA) break;
       t1 += a[ib] * i1[ig];
       t2 += a[ib] * i2[ig];
       t3 += a[ib] * i3[ig];
@@ -1230,52 +1202,6 @@ __global__ void l2p_kernel(int n, int NMleaf, int NM, const int *__restrict__ le
   out[n + i] = o1;
 }
 
-// The same with kL2pSlices threads to a panel, each over every kL2pSlices-th
-// coefficient, their sums added in order: while a thread per panel would leave
-// the chip short of warps, the loop over the coefficients is one chain of loads
-// (320 panels: 15.3 us with a thread per panel, 7.6 sliced; 20,480: 16.3 and
-// 8.1; above kL2pSliced panels the loads of a thread per panel fill HBM).
-constexpr int kL2pSlices = 8;
-constexpr int kL2pSliced = 2 * 148 * 256;
-
-template <typename TQ>
-__global__ void __launch_bounds__(256)
-l2p_sliced_kernel(int n, int NMleaf, int NM, const int *__restrict__ leafOfPanel,
-                  const int *__restrict__ leafFmm, const TQ *__restrict__ Q0,
-                  const TQ *__restrict__ Q1, const double *__restrict__ lec1,
-                  const double *__restrict__ lec2, const double *__restrict__ lec3,
-                  const double *__restrict__ lec4, double alpha, double beta, const double *__restrict__ area,
-                  const double *__restrict__ diagX, double s1, double s2, int swap,
-                  const double *__restrict__ addend, double *out) {
-  constexpr int PB = 256 / kL2pSlices;   // panels per block: one per lane of a warp
-  __shared__ double red[2][kL2pSlices][PB];
-  const int slice = threadIdx.x / PB, lane = threadIdx.x % PB;
-  const int i = blockIdx.x * PB + lane;
-  double a = 0.0, b = 0.0;
-  if (i < n) {
-    const size_t f = (size_t)leafFmm[leafOfPanel[i]] * NM;
-#pragma unroll 4
-    for (int m = slice; m < NMleaf; m += kL2pSlices) {
-      a += (double)Q0[(size_t)m * n + i] * (lec1[f + m] + lec2[f + m]);
-      b += (double)Q1[(size_t)m * n + i] * (lec3[f + m] + lec4[f + m]);
-    }
-  }
-  red[0][slice][lane] = a;
-  red[1][slice][lane] = b;
-  __syncthreads();
-  if (slice > 1 || i >= n) return;   // slice 0 the potential half, slice 1 the other
-  const int from = swap ? 1 - slice : slice;
-  double v = 0.0;
-#pragma unroll
-  for (int w = 0; w < kL2pSlices; w++) v += red[from][w][lane];
-  const size_t at = (size_t)slice * n + i;
-  double o = (beta == 0.0) ? 0.0 : beta * out[at];
-  o += alpha * v;
-  if (diagX) o += (slice ? s2 : s1) * area[i] * diagX[at];
-  if (addend) o += addend[at];
-  out[at] = o;
-}
-
 // ------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------
@@ -1290,65 +1216,41 @@ static void launch_leaf_moments(Context &c, int order) {
 // Forward: moments (d_mom) -> local expansions (4 planes of d_lec).
 // Adjoint: adjoint locals g12, g34 (planes 0, 1 of d_lec) -> adjoint moments
 // (pot, dpdn: planes 0, 1 of d_mom) over the transposed pair lists.
-// Destination cubes up to which an M2L splits a cube's batches over four warps: all four times as many warps are then
-// resident at once (16 per SM), and a cube's two to four batches run side by side instead of one after the other.
-// M2L_SPLIT
-constexpr int kM2LSplitCubes = 592;
-
-template <int PU, bool ADJ, typename TV, bool SPLIT>
-static void launch_m2l_unrolled_t(Context &c, int nDst, const int *dst, const int *off, const int *src,
-                                  const int *pairIdx, const void *tens, const double *inPot, const double *inDpdn,
-                                  double *o1, double *o2, double *o3, double *o4) {
-  typedef M2LUnrolledShape<PU, TV> Sh;
-  static bool attrDone = false;
-  if (!attrDone) {
-    cudaFuncSetAttribute(m2l_unrolled_kernel<PU, ADJ, TV, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Sh::bytes);
-    attrDone = true;
-  }
-  const unsigned grid = SPLIT ? nDst : ceil_div((long long)nDst, Sh::W);
-  m2l_unrolled_kernel<PU, ADJ, TV, SPLIT><<<grid, Sh::W * 32, Sh::bytes, c.stream>>>(
-      nDst, dst, off, src, pairIdx, c.d_ordM2L, c.nM2LPairs, (const typename Vec2<TV>::t *)tens, c.d_cubeCtr,
-      (float)c.prm.kappa, c.NM, c.epsilon, inPot, inDpdn, o1, o2, o3, o4);
-}
 template <int PU, bool ADJ, typename TV>
 static void launch_m2l_unrolled(Context &c, int nDst, const int *dst, const int *off, const int *src,
                                 const int *pairIdx, const void *tens, const double *inPot, const double *inDpdn,
                                 double *o1, double *o2, double *o3, double *o4) {
-  if (M2LUnrolledShape<PU, TV>::W > 1 && nDst <= kM2LSplitCubes)
-    launch_m2l_unrolled_t<PU, ADJ, TV, true>(c, nDst, dst, off, src, pairIdx, tens, inPot, inDpdn, o1, o2, o3, o4);
-  else
-    launch_m2l_unrolled_t<PU, ADJ, TV, false>(c, nDst, dst, off, src, pairIdx, tens, inPot, inDpdn, o1, o2, o3, o4);
+  typedef M2LUnrolledShape<PU, TV> Sh;
+  static bool attrDone = false;
+  if (!attrDone) {
+    cudaFuncSetAttribute(m2l_unrolled_kernel<PU, ADJ, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)Sh::bytes);
+    attrDone = true;
+  }
+  const unsigned grid = ceil_div((long long)nDst, Sh::W);
+  m2l_unrolled_kernel<PU, ADJ, TV><<<grid, Sh::W * 32, Sh::bytes, c.stream>>>(
+      nDst, dst, off, src, pairIdx, c.d_ordM2L, c.nM2LPairs, (const typename Vec2<TV>::t *)tens, c.d_cubeCtr,
+      (float)c.prm.kappa, c.NM, c.epsilon, inPot, inDpdn, o1, o2, o3, o4);
 }
 
 // The bulk-copy staged M2L of a mixed context: the input rows packed to FP32,
-// then NW warps per destination cube.
-template <int PU, bool ADJ, int NW>
-static void launch_m2l_bulk_t(Context &c, int nDst, const int *dst, const int *off, const int *src,
-                              const double *inPot, const double *inDpdn, double *o1, double *o2, double *o3,
-                              double *o4) {
-  typedef M2LBulkShape<PU> Sh;
-  constexpr size_t bytes = NW * ((Sh::bytes + 15) & ~(size_t)15);
-  static bool attrDone = false;
-  if (!attrDone) {
-    cudaFuncSetAttribute(m2l_bulk_kernel<PU, ADJ, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    attrDone = true;
-  }
-  const long long total = (long long)c.pt.nFmm * Sh::NMS;
-  m2l_pack_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(total, c.NM, Sh::NMS, inPot, inDpdn, c.d_momF2);
-  m2l_bulk_kernel<PU, ADJ, NW><<<nDst, 32 * NW, bytes, c.stream>>>(dst, off, src, c.d_ordM2L, c.d_cubeCtr,
-                                                                   (float)c.prm.kappa, c.NM, c.epsilon, c.d_momF2, o1,
-                                                                   o2, o3, o4);
-  c.launches += 1;   // the pack
-}
+// then one warp per destination cube.
 template <int PU, bool ADJ>
 static void launch_m2l_bulk(Context &c, int nDst, const int *dst, const int *off, const int *src,
                             const double *inPot, const double *inDpdn, double *o1, double *o2, double *o3,
                             double *o4) {
-  if (nDst <= kM2LSplitCubes)
-    launch_m2l_bulk_t<PU, ADJ, 4>(c, nDst, dst, off, src, inPot, inDpdn, o1, o2, o3, o4);
-  else
-    launch_m2l_bulk_t<PU, ADJ, 1>(c, nDst, dst, off, src, inPot, inDpdn, o1, o2, o3, o4);
+  typedef M2LBulkShape<PU> Sh;
+  static bool attrDone = false;
+  if (!attrDone) {
+    cudaFuncSetAttribute(m2l_bulk_kernel<PU, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::bytes);
+    attrDone = true;
+  }
+  const long long total = (long long)c.pt.nFmm * Sh::NMS;
+  m2l_pack_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(total, c.NM, Sh::NMS, inPot, inDpdn, c.d_momF2);
+  m2l_bulk_kernel<PU, ADJ><<<nDst, 32, Sh::bytes, c.stream>>>(dst, off, src, c.d_ordM2L, c.d_cubeCtr,
+                                                              (float)c.prm.kappa, c.NM, c.epsilon, c.d_momF2, o1,
+                                                              o2, o3, o4);
+  c.launches += 1;   // the pack
 }
 
 // Forward: moments (d_mom) -> local expansions (4 planes of d_lec).
@@ -1477,8 +1379,8 @@ bool setup_fmm(Context &c) {
       !c.arena.upload(&c.d_m2lOff, pt.m2lOff, s) || !c.arena.upload(&c.d_m2lSrc, pt.m2lSrc, s) ||
       !c.arena.upload(&c.d_m2lDst, c.h_m2lDst, s))
     return false;
-  if (!c.arena.alloc_n(&c.d_mom, 6 * (size_t)pt.nFmm * c.NM)) return false;
-  c.d_lec = c.d_mom + 2 * (size_t)pt.nFmm * c.NM;   // one buffer, zeroed by one memset per product
+  if (!c.arena.alloc_n(&c.d_mom, 2 * (size_t)pt.nFmm * c.NM) || !c.arena.alloc_n(&c.d_lec, 4 * (size_t)pt.nFmm * c.NM))
+    return false;
   StageTimer tm("fmm_setup", s);
   // M2L derivative tensors, once per geometry
   c.nM2LPairs = (long long)pt.m2lSrc.size();
@@ -1549,18 +1451,6 @@ static bool setup_m2l_adjoint(Context &c) {
   return true;
 }
 
-// the moments of `count` cubes from their children's, two planes
-static bool launch_m2m(Context &c, int first, int count, int ordOut, int ordIn, const int *kidFirst,
-                       const int *kidCount, const double *ctr, double *m1, double *m2, cudaStream_t s) {
-  const int nOut = nmom(ordOut), nLst = c.h_mOff[nOut];
-  const size_t shm = (size_t)kShiftWarps * 5 * nOut * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
-  if (shm > 44 * 1024)
-    FB_CUDA(cudaFuncSetAttribute(m2m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-  m2m_kernel<<<count, kShiftWarps * 32, shm, s>>>(first, count, c.NM, ordOut, ordIn, kidFirst, kidCount, ctr,
-                                                  c.d_mOff, c.d_mLst, nLst, m1, m2);
-  return true;
-}
-
 // Forward: Q2M, M2M, M2L, L2L; the leaves' local expansions end in d_lec.
 // Adjoint (the transposed far operator, read right to left): L2P^T (Q2M with
 // the halves exchanged) -> g12, g34 in d_lec planes 0, 1; L2L^T, which is the
@@ -1572,7 +1462,8 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
   cudaStream_t s = c.stream;
   const size_t plane = (size_t)pt.nFmm * c.NM;
   if (adjoint && !setup_m2l_adjoint(c)) return false;
-  FB_CUDA(cudaMemsetAsync(c.d_mom, 0, 6 * plane * sizeof(double), s));   // d_lec's planes follow
+  FB_CUDA(cudaMemsetAsync(c.d_mom, 0, 2 * plane * sizeof(double), s));
+  FB_CUDA(cudaMemsetAsync(c.d_lec, 0, 4 * plane * sizeof(double), s));
   c.launches += 1 + 2 * (depth - height);
   // upward arrays: moments (forward) or adjoint locals (adjoint)
   double *up1 = adjoint ? c.d_lec + plane : c.d_mom, *up2 = adjoint ? c.d_lec : c.d_mom + plane;
@@ -1584,9 +1475,13 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
                                                   c.d_leafFmm, c.d_Q0, c.d_Q1, sgm, adjoint ? 1 : 0, up1, up2);
   if (marks) cudaEventRecord(marks[0], s);
   for (int lev = depth - 1; lev >= height; lev--) {
-    if (!launch_m2m(c, pt.fmmLevelStart[lev], pt.fmmLevelCount[lev], pt.ordMom[lev], pt.ordMom[lev + 1], c.d_kidFirst,
-                    c.d_kidCount, c.d_cubeCtr, up1, up2, s))
-      return false;
+    int ordOut = pt.ordMom[lev], ordIn = pt.ordMom[lev + 1];
+    const int nOut = nmom(ordOut), nLst = c.h_mOff[nOut];
+    const size_t shm = (size_t)kShiftWarps * 5 * nOut * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
+    if (shm > 48 * 1024) cudaFuncSetAttribute(m2m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    m2m_kernel<<<pt.fmmLevelCount[lev], kShiftWarps * 32, shm, s>>>(
+        pt.fmmLevelStart[lev], pt.fmmLevelCount[lev], c.NM, ordOut, ordIn, c.d_kidFirst, c.d_kidCount, c.d_cubeCtr,
+        c.d_mOff, c.d_mLst, nLst, up1, up2);
   }
   if (marks) cudaEventRecord(marks[1], s);
   if (!launch_m2l_only(c, adjoint, fp64)) return false;
@@ -1598,7 +1493,7 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
     int ordIn = pt.ordMom[lev], ordOut = pt.ordMom[lev + 1];
     const int nOut = nmom(ordOut), nLst = c.h_lstOff[nOut];
     const size_t shm = (size_t)kShiftWarps * 5 * nmom(ordIn) * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
-    if (shm > 44 * 1024) cudaFuncSetAttribute(l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    if (shm > 48 * 1024) cudaFuncSetAttribute(l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
     l2l_kernel<<<ceil_div(pt.fmmLevelCount[lev + 1], kShiftWarps), kShiftWarps * 32, shm, s>>>(
         pt.fmmLevelStart[lev + 1], pt.fmmLevelCount[lev + 1], c.NM, ordIn, ordOut, c.d_fmmParent, c.d_cubeCtr,
         c.d_lstOff, c.d_lst, nLst, d1, d2, c.d_lec + 2 * plane, c.d_lec + 3 * plane);
@@ -1624,16 +1519,15 @@ bool launch_l2p(Context &c, double alpha, double beta, double *out, const double
   // adjoint: Q0 . (adjoint dpdn moments + 0) -> dpdn half, Q1 . (adjoint pot moments + 0) -> pot half
   const double *l1 = adjoint ? c.d_mom + plane : c.d_lec, *l2 = c.d_lec + (adjoint ? 2 : 1) * plane;
   const double *l3 = adjoint ? c.d_mom : c.d_lec + 2 * plane, *l4 = c.d_lec + 3 * plane;
-  auto run = [&](auto q0, auto q1) {
-    typedef typename std::remove_const<typename std::remove_pointer<decltype(q0)>::type>::type TQ;
-    const bool sliced = c.n <= kL2pSliced;
-    auto kern = sliced ? l2p_sliced_kernel<TQ> : l2p_kernel<TQ>;
-    kern<<<ceil_div(c.n, sliced ? 256 / kL2pSlices : 256), 256, 0, c.stream>>>(
-        c.n, c.NMleaf, c.NM, c.d_leafOfPanel, c.d_leafFmm, q0, q1, l1, l2, l3, l4, alpha, beta, c.d_area, diagX, s1,
-        s2, adjoint ? 1 : 0, addend, out);
-  };
-  if (c.d_Q0F && !fp64) run((const float *)c.d_Q0F, (const float *)c.d_Q1F);
-  else run((const double *)c.d_Q0, (const double *)c.d_Q1);
+  if (c.d_Q0F && !fp64)
+    l2p_kernel<float><<<ceil_div(c.n, 256), 256, 0, c.stream>>>(c.n, c.NMleaf, c.NM, c.d_leafOfPanel, c.d_leafFmm,
+                                                                c.d_Q0F, c.d_Q1F, l1, l2, l3, l4, alpha, beta,
+                                                                c.d_area, diagX, s1, s2, adjoint ? 1 : 0, addend, out);
+  else
+    l2p_kernel<double><<<ceil_div(c.n, 256), 256, 0, c.stream>>>(c.n, c.NMleaf, c.NM, c.d_leafOfPanel, c.d_leafFmm,
+                                                                 c.d_Q0, c.d_Q1, l1, l2, l3, l4, alpha, beta,
+                                                                 c.d_area, diagX, s1, s2, adjoint ? 1 : 0, addend,
+                                                                 out);
   FB_CUDA(cudaGetLastError());
   return true;
 }
