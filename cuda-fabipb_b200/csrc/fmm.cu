@@ -667,14 +667,6 @@ struct M2LTensors<PM, TV, true> {
 // bank conflicts.
 __device__ __forceinline__ int m2l_slot(int e, int j) { return e * 32 + (j ^ (e & 31)); }
 
-// One (alpha, beta) entry.  FULL: the cube's order is PM, every entry counts.
-// The four sums of a coefficient are reduced over the lanes (component v's
-// total lands in lane 8v) and added to the warp's shared sums sAcc[v][alpha].
-template <typename TV>
-struct M2LSumsT {
-  TV s1, s2, s3, s4;
-};
-
 // Moment readers of the conv.  M2LColMoments: the XOR-swizzled columns staged
 // by plain loads.  M2LRowMoments: the lane's source row of (pot, dpdn) float2
 // entries staged by bulk copies, read as float4 (entries IB, IB+1) at even IB;
@@ -702,37 +694,13 @@ struct M2LRowMoments {
   }
 };
 
-template <int PM, int Q, bool FULL, bool ADJ, typename TV, typename TT, typename TM>
-__device__ __forceinline__ void m2l_step(M2LSumsT<TV> &S, TM &M, const TT &T, int lane, int order, double *sAcc) {
-  constexpr M2LEntry E = m2l_entry<PM>(Q);
-  if (E.first) S.s1 = S.s2 = S.s3 = S.s4 = (TV)0;
-  if (FULL || E.dsum <= order) {
-    const typename Vec2<TV>::t mo = M.template get<E.ib>();
-    const typename Vec2<TV>::t d = T.get(E.ig, lane);
-    if ((ADJ ? E.dal : E.dsum - E.dal) & 1) {   // (-1)^|input|, or (-1)^|output| transposed
-      S.s1 -= mo.y * d.x; S.s2 -= mo.y * d.y; S.s3 -= mo.x * d.x; S.s4 -= mo.x * d.y;
-    } else {
-      S.s1 += mo.y * d.x; S.s2 += mo.y * d.y; S.s3 += mo.x * d.x; S.s4 += mo.x * d.y;
-    }
-  }
-  if (E.last && (FULL || E.dal <= order)) {
-    const TV t = warp_sum4<TV>(S.s1, S.s2, S.s3, S.s4, lane);
-    if ((lane & 7) == 0) sAcc[(lane >> 3) * nmom_c(PM) + E.al] += (double)t;
-  }
-}
-
-template <int PM, bool FULL, bool ADJ, typename TV, typename TT, typename TM, int... Q>
-__device__ __forceinline__ void m2l_steps(std::integer_sequence<int, Q...>, M2LSumsT<TV> &S, TM &M, const TT &T,
-                                          int lane, int order, double *sAcc) {
-  (m2l_step<PM, Q, FULL, ADJ, TV, TT, TM>(S, M, T, lane, order, sAcc), ...);
-}
-
 // Lane l ends with the warp total of v[(l >> 1) & 15]: one butterfly over
 // sixteen values (8 + 4 + 2 + 1 + 1 shuffles), whose first stages carry
 // several independent shuffles each.
-__device__ __forceinline__ float warp_sum16(const float (&v)[16], int lane) {
+template <typename T>
+__device__ __forceinline__ T warp_sum16(const T (&v)[16], int lane) {
   const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
-  float w[8], x[4], y[2];
+  T w[8], x[4], y[2];
 #pragma unroll
   for (int i = 0; i < 8; i++)
     w[i] = (h16 ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[i + 8], 16);
@@ -742,26 +710,26 @@ __device__ __forceinline__ float warp_sum16(const float (&v)[16], int lane) {
 #pragma unroll
   for (int i = 0; i < 2; i++)
     y[i] = (h4 ? x[i + 2] : x[i]) + __shfl_xor_sync(0xffffffffu, h4 ? x[i] : x[i + 2], 4);
-  float z = (h2 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, h2 ? y[0] : y[1], 2);
+  T z = (h2 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, h2 ? y[0] : y[1], 2);
   return z + __shfl_xor_sync(0xffffffffu, z, 1);
 }
 
-// The bulk-staged M2L's (alpha, beta) step: the conv of m2l_step (FP32), with
-// the four sums of four consecutive output coefficients reduced together by
-// warp_sum16 (16 shuffles for 16 sums instead of 24, and independent shuffle
-// chains), lane 2j (j = 4 slot + component) adding sum j to its coefficient.
+// One (alpha, beta) step of the conv.  FULL: the cube's order is PM, every entry counts.  The four sums of four
+// consecutive output coefficients are reduced together by warp_sum16 (16 shuffles for 16 sums instead of 24, and
+// independent shuffle chains), lane 2j (j = 4 slot + component) adding sum j to the warp's shared sums sAcc[j & 3][alpha].
+// In FP64 at order 4 (410,508 pairs) this takes the kernel from 269 us to 200.
+template <typename TV>
 struct M2LSums16 {
-  float s1, s2, s3, s4;
-  float b[16];   // [slot of alpha mod 4][component]
+  TV s1, s2, s3, s4;
+  TV b[16];   // [slot of alpha mod 4][component]
 };
-template <int PM, int Q, bool FULL, bool ADJ, typename TT>
-__device__ __forceinline__ void m2l_step16(M2LSums16 &S, M2LRowMoments &M, const TT &T, int lane, int order,
-                                           double *sAcc) {
+template <int PM, int Q, bool FULL, bool ADJ, typename TV, typename TT, typename TM>
+__device__ __forceinline__ void m2l_step16(M2LSums16<TV> &S, TM &M, const TT &T, int lane, int order, double *sAcc) {
   constexpr M2LEntry E = m2l_entry<PM>(Q);
-  if (E.first) S.s1 = S.s2 = S.s3 = S.s4 = 0.f;
+  if (E.first) S.s1 = S.s2 = S.s3 = S.s4 = (TV)0;
   if (FULL || E.dsum <= order) {
-    const float2 mo = M.template get<E.ib>();
-    const float2 d = T.get(E.ig, lane);
+    const typename Vec2<TV>::t mo = M.template get<E.ib>();
+    const typename Vec2<TV>::t d = T.get(E.ig, lane);
     if ((ADJ ? E.dal : E.dsum - E.dal) & 1) {   // (-1)^|input|, or (-1)^|output| transposed
       S.s1 -= mo.y * d.x; S.s2 -= mo.y * d.y; S.s3 -= mo.x * d.x; S.s4 -= mo.x * d.y;
     } else {
@@ -776,16 +744,16 @@ __device__ __forceinline__ void m2l_step16(M2LSums16 &S, M2LRowMoments &M, const
     S.b[4 * slot + 3] = S.s4;
     if constexpr (slot == 3 || E.al == nmom_c(PM) - 1) {
       // a last group of fewer than four: the slots past E.al are reduced, not written
-      const float t = warp_sum16(S.b, lane);
+      const TV t = warp_sum16<TV>(S.b, lane);
       const int j = (lane >> 1) & 15, al = (E.al & ~3) + (j >> 2);
       if (!(lane & 1) && al <= E.al && (FULL || c_mi[al].w <= order)) sAcc[(j & 3) * nmom_c(PM) + al] += (double)t;
     }
   }
 }
-template <int PM, bool FULL, bool ADJ, typename TT, int... Q>
-__device__ __forceinline__ void m2l_steps16(std::integer_sequence<int, Q...>, M2LSums16 &S, M2LRowMoments &M,
-                                            const TT &T, int lane, int order, double *sAcc) {
-  (m2l_step16<PM, Q, FULL, ADJ, TT>(S, M, T, lane, order, sAcc), ...);
+template <int PM, bool FULL, bool ADJ, typename TV, typename TT, typename TM, int... Q>
+__device__ __forceinline__ void m2l_steps16(std::integer_sequence<int, Q...>, M2LSums16<TV> &S, TM &M, const TT &T,
+                                            int lane, int order, double *sAcc) {
+  (m2l_step16<PM, Q, FULL, ADJ, TV, TT, TM>(S, M, T, lane, order, sAcc), ...);
 }
 
 // The lane's FP32 M2L tensor (packed D^e G0, D^e Gk) from its pair's offset x =
@@ -815,7 +783,9 @@ __device__ __forceinline__ void m2l_gen_tensor(const float x[3], bool live, floa
 // ADJ: the transposed interaction, as for m2l_kernel.  TV = float: tensors
 // (float2) and staged moments in FP32, each batch's per-coefficient sums in
 // FP32, accumulated over the batches in FP64.
-template <int PM, bool ADJ, typename TV>
+// SPLIT (few cubes): a block takes one cube, its warps the cube's batches in turn, and their sums are added at the
+// end; else a warp takes a cube.
+template <int PM, bool ADJ, typename TV, bool SPLIT>
 __global__ void __launch_bounds__(M2LUnrolledShape<PM, TV>::W * 32,
                                   PM >= 5 ? 1 : (sizeof(TV) == 4 ? FB_M2L_MIN_BLOCKS_F32 : FB_M2L_MIN_BLOCKS))
 m2l_unrolled_kernel(int nDst, const int *__restrict__ dstList, const int *__restrict__ m2lOff,
@@ -832,13 +802,14 @@ m2l_unrolled_kernel(int nDst, const int *__restrict__ dstList, const int *__rest
   char *wbase = reinterpret_cast<char *>(m2luSmem) + (size_t)warp * Sh::warpBytes;
   V2 *sC = reinterpret_cast<V2 *>(wbase);
   double *sAcc = reinterpret_cast<double *>(wbase + Sh::colBytes);   // [4][NMP]
-  const int bi = blockIdx.x * Sh::W + warp;
-  if (bi >= nDst) return;  // warp-uniform
+  const int bi = SPLIT ? (int)blockIdx.x : (int)blockIdx.x * Sh::W + warp;
+  if (bi >= nDst) return;  // warp-uniform (block-uniform when split)
   const int f = dstList[bi];
   const int order = ordOfCube[f];
   const int o0 = m2lOff[f], o1 = m2lOff[f + 1];
   for (int e = lane; e < 4 * NMP; e += 32) sAcc[e] = 0.0;
-  for (int b0 = o0; b0 < o1; b0 += 32) {
+  constexpr int kStep = SPLIT ? 32 * Sh::W : 32;
+  for (int b0 = o0 + (SPLIT ? 32 * warp : 0); b0 < o1; b0 += kStep) {
     const int k = b0 + lane;
     const bool live = k < o1;
     const int nb = min(32, o1 - b0);
@@ -889,20 +860,29 @@ m2l_unrolled_kernel(int nDst, const int *__restrict__ dstList, const int *__rest
       for (int e = 0; e < NMP; e++) T.v[e] = tp[(size_t)e * nPairs];
     }
     __syncwarp();
-    M2LSumsT<TV> S{(TV)0, (TV)0, (TV)0, (TV)0};
+    M2LSums16<TV> S{};
     M2LColMoments<V2> M{sC, lane};
     if (order == PM)
-      m2l_steps<PM, true, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order,
-                                   sAcc);
+      m2l_steps16<PM, true, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
     else
-      m2l_steps<PM, false, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order,
-                                    sAcc);
+      m2l_steps16<PM, false, ADJ, TV>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
   }
-  __syncwarp();
+  if (SPLIT) __syncthreads();
+  else __syncwarp();
   const int nm = ((order + 1) * (order + 2) * (order + 3)) / 6;
   const double ieps = 1.0 / eps;
-  for (int e = lane; e < nm; e += 32) {
-    const double S1 = sAcc[e], S2 = sAcc[NMP + e], S3 = sAcc[2 * NMP + e], S4 = sAcc[3 * NMP + e];
+  for (int e = SPLIT ? threadIdx.x : lane; e < nm; e += kStep) {
+    double S1 = 0.0, S2 = 0.0, S3 = 0.0, S4 = 0.0;
+#pragma unroll
+    for (int w = 0; w < (SPLIT ? Sh::W : 1); w++) {
+      const double *acc = SPLIT ? reinterpret_cast<const double *>(reinterpret_cast<const char *>(m2luSmem) +
+                                                                   (size_t)w * Sh::warpBytes + Sh::colBytes)
+                                : sAcc;
+      S1 += acc[e];
+      S2 += acc[NMP + e];
+      S3 += acc[2 * NMP + e];
+      S4 += acc[3 * NMP + e];
+    }
     const size_t o = (size_t)f * NM + e;
     if (ADJ) {   // sign already folded in
       lec1[o] += eps * S2 - S1 - S3 + S4;
@@ -1005,21 +985,25 @@ __device__ __forceinline__ void m2l_bulk_issue(int nb, int sj, int lane, const f
   if (lane < nb) bulk_g2s(buf + lane * Sh::RS, momF + (size_t)sj * Sh::NMS, Sh::NMS * sizeof(float2), bar);
 }
 
-template <int PM, bool ADJ>
-__global__ void __launch_bounds__(32, M2LBulkShape<PM>::MINB)
+// NW warps per destination cube, which take its batches in turn (several when there are few cubes)
+template <int PM, bool ADJ, int NW>
+__global__ void __launch_bounds__(32 * NW, M2LBulkShape<PM>::MINB / NW < 1 ? 1 : M2LBulkShape<PM>::MINB / NW)
 m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff, const int *__restrict__ m2lSrc,
                 const int *__restrict__ ordOfCube, const double *__restrict__ ctr, float kappa, int NM, double eps,
                 const float2 *__restrict__ momF, double *lec1, double *lec2, double *lec3, double *lec4) {
   typedef M2LBulkShape<PM> Sh;
   constexpr int NMP = Sh::NMP;
   extern __shared__ __align__(16) unsigned char m2lbSmem[];
-  float2 *buf = reinterpret_cast<float2 *>(m2lbSmem);   // [2][32][RS]
-  double *sAcc = reinterpret_cast<double *>(m2lbSmem + Sh::accOff);   // [4][NMP]
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(m2lbSmem + Sh::barOff);
-  const int lane = threadIdx.x;
+  constexpr int kStep = 32 * NW;
+  constexpr size_t kWarpBytes = (Sh::bytes + 15) & ~(size_t)15;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char *base = m2lbSmem + warp * kWarpBytes;
+  float2 *buf = reinterpret_cast<float2 *>(base);   // [2][32][RS]
+  double *sAcc = reinterpret_cast<double *>(base + Sh::accOff);   // [4][NMP]
+  unsigned long long *bar = reinterpret_cast<unsigned long long *>(base + Sh::barOff);
   const int f = dstList[blockIdx.x];
   const int order = ordOfCube[f];
-  const int o0 = m2lOff[f], o1 = m2lOff[f + 1];
+  const int oBeg = m2lOff[f], o0 = oBeg + 32 * warp, o1 = m2lOff[f + 1];
   for (int e = lane; e < 4 * NMP; e += 32) sAcc[e] = 0.0;
   if (lane == 0) {
     mbar_init(&bar[0], 1);
@@ -1030,18 +1014,18 @@ m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff,
   const double cf0 = ctr[3 * f], cf1 = ctr[3 * f + 1], cf2 = ctr[3 * f + 2];
   // batch 0 in flight; batch 1's sources and batch 0's centres loaded
   int srcCur = o0 + lane < o1 ? m2lSrc[o0 + lane] : 0;
-  m2l_bulk_issue<PM>(min(32, o1 - o0), srcCur, lane, momF, buf, &bar[0]);
-  int srcNext = o0 + 32 + lane < o1 ? m2lSrc[o0 + 32 + lane] : 0;
+  if (o0 < o1) m2l_bulk_issue<PM>(min(32, o1 - o0), srcCur, lane, momF, buf, &bar[0]);   // warp-uniform
+  int srcNext = o0 + kStep + lane < o1 ? m2lSrc[o0 + kStep + lane] : 0;
   double cs0 = ctr[3 * srcCur], cs1 = ctr[3 * srcCur + 1], cs2 = ctr[3 * srcCur + 2];
   unsigned phase = 0;   // bit s: the parity to wait for on bar[s]
   bool bad = false;
   int it = 0;
-  for (int b0 = o0; b0 < o1; b0 += 32, it++) {
+  for (int b0 = o0; b0 < o1; b0 += kStep, it++) {
     const int s = it & 1;
     const bool live = b0 + lane < o1;
-    const bool more = b0 + 32 < o1;
-    if (more) m2l_bulk_issue<PM>(min(32, o1 - b0 - 32), srcNext, lane, momF, buf + (s ^ 1) * 32 * Sh::RS, &bar[s ^ 1]);
-    const int srcNext2 = b0 + 64 + lane < o1 ? m2lSrc[b0 + 64 + lane] : 0;
+    const bool more = b0 + kStep < o1;
+    if (more) m2l_bulk_issue<PM>(min(32, o1 - b0 - kStep), srcNext, lane, momF, buf + (s ^ 1) * 32 * Sh::RS, &bar[s ^ 1]);
+    const int srcNext2 = b0 + 2 * kStep + lane < o1 ? m2lSrc[b0 + 2 * kStep + lane] : 0;
     const double cn0 = ctr[3 * srcNext], cn1 = ctr[3 * srcNext + 1], cn2 = ctr[3 * srcNext + 2];
     // the lane's tensor from the pair's offset (forward: x_dst - x_src; transposed: the
     // forward pair's cubes, x_src - x_dst here)
@@ -1066,20 +1050,21 @@ m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff,
     }
     // a lane past the batch reads row 0 (finite moments) with its zero tensor
     M2LRowMoments M{buf + s * 32 * Sh::RS + (live ? lane : 0) * Sh::RS, make_float4(0.f, 0.f, 0.f, 0.f)};
-    M2LSums16 S{};
+    M2LSums16<float> S{};
     if (order == PM)
-      m2l_steps16<PM, true, ADJ>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
+      m2l_steps16<PM, true, ADJ, float>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
     else
-      m2l_steps16<PM, false, ADJ>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
+      m2l_steps16<PM, false, ADJ, float>(std::make_integer_sequence<int, m2l_entries<PM>()>{}, S, M, T, lane, order, sAcc);
     srcNext = srcNext2;
     cs0 = cn0; cs1 = cn1; cs2 = cn2;
   }
-  __syncwarp();
+  if (bad && lane == 0) atomicAdd(&g_m2lStalls, 1u);
+  if (NW > 1) bad = __syncthreads_or(bad);
+  else __syncwarp();
   const int nm = ((order + 1) * (order + 2) * (order + 3)) / 6;
   if (bad) {
-    if (lane == 0) atomicAdd(&g_m2lStalls, 1u);
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    for (int e = lane; e < nm; e += 32) {
+    for (int e = threadIdx.x; e < nm; e += kStep) {
       const size_t o = (size_t)f * NM + e;
       lec1[o] = nan;
       lec2[o] = nan;
@@ -1091,8 +1076,16 @@ m2l_bulk_kernel(const int *__restrict__ dstList, const int *__restrict__ m2lOff,
     return;
   }
   const double ieps = 1.0 / eps;
-  for (int e = lane; e < nm; e += 32) {
-    const double S1 = sAcc[e], S2 = sAcc[NMP + e], S3 = sAcc[2 * NMP + e], S4 = sAcc[3 * NMP + e];
+  for (int e = threadIdx.x; e < nm; e += kStep) {
+    double S1 = 0.0, S2 = 0.0, S3 = 0.0, S4 = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; w++) {   // the warps' sums
+      const double *acc = reinterpret_cast<const double *>(m2lbSmem + w * kWarpBytes + Sh::accOff);
+      S1 += acc[e];
+      S2 += acc[NMP + e];
+      S3 += acc[2 * NMP + e];
+      S4 += acc[3 * NMP + e];
+    }
     const size_t o = (size_t)f * NM + e;
     if (ADJ) {   // sign already folded in
       lec1[o] += eps * S2 - S1 - S3 + S4;
@@ -1213,44 +1206,69 @@ static void launch_leaf_moments(Context &c, int order) {
                                                                    c.d_leafOfPanel, c.d_leafCtr, c.d_Q0, c.d_Q1);
 }
 
+// Destination cubes up to which an M2L splits a cube's batches over four warps: all four times as many warps are then
+// resident at once (16 per SM), and a cube's two to four batches run side by side instead of one after the other.
+// 320 panels (56 cubes) 9.5 us whole, 8.3 split; 20,480 (328 cubes) 11.6 and 9.0; FP64, 1,280 panels (304 cubes) 26.2
+// and 12.5.
+constexpr int kM2LSplitCubes = 592;
+
 // Forward: moments (d_mom) -> local expansions (4 planes of d_lec).
 // Adjoint: adjoint locals g12, g34 (planes 0, 1 of d_lec) -> adjoint moments
 // (pot, dpdn: planes 0, 1 of d_mom) over the transposed pair lists.
+template <int PU, bool ADJ, typename TV, bool SPLIT>
+static void launch_m2l_unrolled_t(Context &c, int nDst, const int *dst, const int *off, const int *src,
+                                  const int *pairIdx, const void *tens, const double *inPot, const double *inDpdn,
+                                  double *o1, double *o2, double *o3, double *o4) {
+  typedef M2LUnrolledShape<PU, TV> Sh;
+  static bool attrDone = false;
+  if (!attrDone) {
+    cudaFuncSetAttribute(m2l_unrolled_kernel<PU, ADJ, TV, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)Sh::bytes);
+    attrDone = true;
+  }
+  const unsigned grid = SPLIT ? nDst : ceil_div((long long)nDst, Sh::W);
+  m2l_unrolled_kernel<PU, ADJ, TV, SPLIT><<<grid, Sh::W * 32, Sh::bytes, c.stream>>>(
+      nDst, dst, off, src, pairIdx, c.d_ordM2L, c.nM2LPairs, (const typename Vec2<TV>::t *)tens, c.d_cubeCtr,
+      (float)c.prm.kappa, c.NM, c.epsilon, inPot, inDpdn, o1, o2, o3, o4);
+}
 template <int PU, bool ADJ, typename TV>
 static void launch_m2l_unrolled(Context &c, int nDst, const int *dst, const int *off, const int *src,
                                 const int *pairIdx, const void *tens, const double *inPot, const double *inDpdn,
                                 double *o1, double *o2, double *o3, double *o4) {
-  typedef M2LUnrolledShape<PU, TV> Sh;
-  static bool attrDone = false;
-  if (!attrDone) {
-    cudaFuncSetAttribute(m2l_unrolled_kernel<PU, ADJ, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Sh::bytes);
-    attrDone = true;
-  }
-  const unsigned grid = ceil_div((long long)nDst, Sh::W);
-  m2l_unrolled_kernel<PU, ADJ, TV><<<grid, Sh::W * 32, Sh::bytes, c.stream>>>(
-      nDst, dst, off, src, pairIdx, c.d_ordM2L, c.nM2LPairs, (const typename Vec2<TV>::t *)tens, c.d_cubeCtr,
-      (float)c.prm.kappa, c.NM, c.epsilon, inPot, inDpdn, o1, o2, o3, o4);
+  if (M2LUnrolledShape<PU, TV>::W > 1 && nDst <= kM2LSplitCubes)
+    launch_m2l_unrolled_t<PU, ADJ, TV, true>(c, nDst, dst, off, src, pairIdx, tens, inPot, inDpdn, o1, o2, o3, o4);
+  else
+    launch_m2l_unrolled_t<PU, ADJ, TV, false>(c, nDst, dst, off, src, pairIdx, tens, inPot, inDpdn, o1, o2, o3, o4);
 }
 
 // The bulk-copy staged M2L of a mixed context: the input rows packed to FP32,
-// then one warp per destination cube.
-template <int PU, bool ADJ>
-static void launch_m2l_bulk(Context &c, int nDst, const int *dst, const int *off, const int *src,
-                            const double *inPot, const double *inDpdn, double *o1, double *o2, double *o3,
-                            double *o4) {
+// then NW warps per destination cube.
+template <int PU, bool ADJ, int NW>
+static void launch_m2l_bulk_t(Context &c, int nDst, const int *dst, const int *off, const int *src,
+                              const double *inPot, const double *inDpdn, double *o1, double *o2, double *o3,
+                              double *o4) {
   typedef M2LBulkShape<PU> Sh;
+  constexpr size_t bytes = NW * ((Sh::bytes + 15) & ~(size_t)15);
   static bool attrDone = false;
   if (!attrDone) {
-    cudaFuncSetAttribute(m2l_bulk_kernel<PU, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::bytes);
+    cudaFuncSetAttribute(m2l_bulk_kernel<PU, ADJ, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     attrDone = true;
   }
   const long long total = (long long)c.pt.nFmm * Sh::NMS;
   m2l_pack_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(total, c.NM, Sh::NMS, inPot, inDpdn, c.d_momF2);
-  m2l_bulk_kernel<PU, ADJ><<<nDst, 32, Sh::bytes, c.stream>>>(dst, off, src, c.d_ordM2L, c.d_cubeCtr,
-                                                              (float)c.prm.kappa, c.NM, c.epsilon, c.d_momF2, o1,
-                                                              o2, o3, o4);
+  m2l_bulk_kernel<PU, ADJ, NW><<<nDst, 32 * NW, bytes, c.stream>>>(dst, off, src, c.d_ordM2L, c.d_cubeCtr,
+                                                                   (float)c.prm.kappa, c.NM, c.epsilon, c.d_momF2, o1,
+                                                                   o2, o3, o4);
   c.launches += 1;   // the pack
+}
+template <int PU, bool ADJ>
+static void launch_m2l_bulk(Context &c, int nDst, const int *dst, const int *off, const int *src,
+                            const double *inPot, const double *inDpdn, double *o1, double *o2, double *o3,
+                            double *o4) {
+  if (nDst <= kM2LSplitCubes)
+    launch_m2l_bulk_t<PU, ADJ, 4>(c, nDst, dst, off, src, inPot, inDpdn, o1, o2, o3, o4);
+  else
+    launch_m2l_bulk_t<PU, ADJ, 1>(c, nDst, dst, off, src, inPot, inDpdn, o1, o2, o3, o4);
 }
 
 // Forward: moments (d_mom) -> local expansions (4 planes of d_lec).

@@ -1,4 +1,4 @@
-"""Preconditioner and GMRES kernels at the sizes where their dispatch changes, against the FP64
+"""Preconditioner, GMRES and translation kernels at the sizes where their dispatch changes, against the FP64
 restatement oracle.
 
 Tolerances: FP64 operators 1e-12 and block inverses 1e-11 relative L2, as for the golden cases; block inverses of mixed
@@ -81,3 +81,16 @@ def test_gmres_restart_lengths(restart):
     xr, itr, resr, infor = o.gmres(b, b.copy(), restart, 100, 1e-14)
     assert (it, info) == (itr, infor) and abs(res - resr) <= 1e-6 * resr
     assert rel_l2(x, xr) < 1e-8
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-12), (lib.MIXED, 5e-6)])
+@pytest.mark.parametrize("order", [1, 2, 3, 5, 7])
+@pytest.mark.parametrize("depth", [3, 4])
+def test_far_field_cube_counts(depth, order, precision, tol):
+    """Fewer and more destination cubes than the M2L kernels' dispatch line."""
+    unit, faces = meshgen.icosphere(4)
+    pan = meshio.build_panels(20.0 * unit, unit, faces)
+    opts = dict(order=order, depth=depth, height=2)
+    s, o = lib.Surface(pan, lib.params(precision=precision, **opts)), O.Oracle(pan, O.make_params(**opts))
+    v = np.random.default_rng(order).standard_normal(2 * s.n)
+    assert rel_l2(s.apply(v, part=lib.FAR), o.far_apply(v)) < tol
