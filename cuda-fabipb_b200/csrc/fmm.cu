@@ -20,6 +20,7 @@
 #include <cmath>
 #include <vector>
 
+#include <type_traits>
 #include <utility>
 
 #include "context.cuh"
@@ -36,6 +37,9 @@ __constant__ double c_ifact3[kTabN];
 __constant__ double c_sgn3[kTabN];
 __constant__ double c_fact[kTabOrder + 4];
 __constant__ double c_ifact[kTabOrder + 4];
+// copies for reads at an index that differs from lane to lane
+__device__ int g_mi[kTabN];             // i1 | i2 << 8 | i3 << 16 | (i1 + i2 + i3) << 24
+__device__ double g_ifact3[kTabN];
 
 __device__ __forceinline__ int IDX(int a, int b, int c) { return c_idx3[(a * kTabDim + b) * kTabDim + c]; }
 
@@ -74,6 +78,10 @@ static bool upload_tables() {
   FB_CUDA(cudaMemcpyToSymbol(c_idx3, h.idx3.data(), h.idx3.size() * sizeof(short)));
   FB_CUDA(cudaMemcpyToSymbol(c_mi, h.mi.data(), h.mi.size() * sizeof(char4)));
   FB_CUDA(cudaMemcpyToSymbol(c_ifact3, h.ifact3.data(), h.ifact3.size() * sizeof(double)));
+  std::vector<int> mi(h.mi.size());
+  for (size_t k = 0; k < mi.size(); k++) mi[k] = h.mi[k].x | h.mi[k].y << 8 | h.mi[k].z << 16 | h.mi[k].w << 24;
+  FB_CUDA(cudaMemcpyToSymbol(g_mi, mi.data(), mi.size() * sizeof(int)));
+  FB_CUDA(cudaMemcpyToSymbol(g_ifact3, h.ifact3.data(), h.ifact3.size() * sizeof(double)));
   FB_CUDA(cudaMemcpyToSymbol(c_sgn3, h.sgn3.data(), h.sgn3.size() * sizeof(double)));
   FB_CUDA(cudaMemcpyToSymbol(c_fact, h.fact.data(), h.fact.size() * sizeof(double)));
   FB_CUDA(cudaMemcpyToSymbol(c_ifact, h.ifact.data(), h.ifact.size() * sizeof(double)));
@@ -267,7 +275,30 @@ __global__ void q2m_kernel(int nLeaves, int n, int NMleaf, int NM, const int *__
 // w, w + 8, ... when a cube had more than eight), lanes over the output
 // coefficients; the warps' shifted moments are added in warp order.
 // L2L: one warp per child cube, eight cubes per block.
+// Both are chains of dependent loads and a few hundred FMAs per cube: the
+// shift vector's powers are formed once per warp, the tables read at lane-varying
+// indices come from global memory (constant memory serialises them), and the
+// term loops have known bounds, so that their loads overlap.  One level of 20,000 panels' tree:
+// M2M 9.6 us before, 8.6 now, L2L 15.3 and 13.4; 1,127 parents of 204,800 panels: M2M 18.6 and 15.0.
 constexpr int kShiftWarps = 8;
+
+// a[e] = t^g / g! over the multi-indices g of e < ne (setupConVect, src/moments.c:390-410); one warp,
+// which synchronises before its first use; pw: 3 x (kMaxOrder + 1) values of its own
+__device__ __forceinline__ void warp_conv_entries(const double *t, int order, int ne, int lane, double *pw, double *a) {
+  if (lane < 3) {
+    double f = 1.0;
+    for (int k = 0; k <= order; k++) {
+      pw[lane * (kMaxOrder + 1) + k] = f;
+      f *= t[lane];
+    }
+  }
+  __syncwarp();
+  for (int e = lane; e < ne; e += 32) {
+    const int m = g_mi[e];
+    a[e] = pw[m & 255] * pw[kMaxOrder + 1 + ((m >> 8) & 255)] * pw[2 * (kMaxOrder + 1) + ((m >> 16) & 255)] *
+           g_ifact3[e];
+  }
+}
 
 __global__ void __launch_bounds__(kShiftWarps * 32)
 m2m_kernel(int first, int count, int NM, int ordOut, int ordIn, const int *__restrict__ kidFirst,
@@ -276,6 +307,7 @@ m2m_kernel(int first, int count, int NM, int ordOut, int ordIn, const int *__res
   // per warp: shift entries a, child moments b1, b2, and the child's shifted
   // contribution o1, o2 (nOut each); then the term list (offsets, entries)
   extern __shared__ double sm[];
+  __shared__ double pw[kShiftWarps][3 * (kMaxOrder + 1)];
   if ((int)blockIdx.x >= count) return;
   const int f = first + blockIdx.x;
   const int nOut = nmom(ordOut), nIn = nmom(ordIn);
@@ -292,15 +324,17 @@ m2m_kernel(int first, int count, int NM, int ordOut, int ordIn, const int *__res
     const double t[3] = {ctr[3 * kid] - ctr[3 * f], ctr[3 * kid + 1] - ctr[3 * f + 1],
                          ctr[3 * kid + 2] - ctr[3 * f + 2]};
     __syncwarp();   // the previous child's reads of a, b1, b2 are done
+    warp_conv_entries(t, ordOut, nOut, lane, pw[warp], a);
     for (int e = lane; e < nOut; e += 32) {
-      a[e] = conv_entry(t, e);
       b1[e] = (e < nIn) ? momPot[(size_t)kid * NM + e] : 0.0;
       b2[e] = (e < nIn) ? momDpdn[(size_t)kid * NM + e] : 0.0;
     }
     __syncwarp();
     for (int al = lane; al < nOut; al += 32) {
       double s1 = 0.0, s2 = 0.0;
-      for (int q = lstOff[al]; q < lstOff[al + 1]; q++) {
+      const int q1 = lstOff[al + 1];
+#pragma unroll 4
+      for (int q = lstOff[al]; q < q1; q++) {
         const int ent = lst[q];
         const int ia = ent & 1023, ib = (ent >> 10) & 1023;
         s1 += a[ia] * b1[ib];
@@ -1117,6 +1151,7 @@ l2l_kernel(int first, int count, int NM, int ordIn, int ordOut, const int *__res
   // per warp: shift entries a and the parent's locals i1..i4 (nIn each); then
   // the term list (offsets, entries)
   extern __shared__ double sm[];
+  __shared__ double pw[kShiftWarps][3 * (kMaxOrder + 1)];
   const int nIn = nmom(ordIn), nOut = nmom(ordOut);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int *lstOff = reinterpret_cast<int *>(sm + (size_t)kShiftWarps * 5 * nIn), *lst = lstOff + nOut + 1;
@@ -1129,8 +1164,8 @@ l2l_kernel(int first, int count, int NM, int ordIn, int ordOut, const int *__res
   const int f = first + cube;
   const int p = parent[f];
   const double t[3] = {ctr[3 * f] - ctr[3 * p], ctr[3 * f + 1] - ctr[3 * p + 1], ctr[3 * f + 2] - ctr[3 * p + 2]};
+  warp_conv_entries(t, ordIn, nIn, lane, pw[warp], a);
   for (int e = lane; e < nIn; e += 32) {
-    a[e] = conv_entry(t, e);
     i1[e] = lec1[(size_t)p * NM + e];
     i2[e] = lec2[(size_t)p * NM + e];
     i3[e] = lec3[(size_t)p * NM + e];
@@ -1138,12 +1173,14 @@ l2l_kernel(int first, int count, int NM, int ordIn, int ordOut, const int *__res
   }
   __syncwarp();
   for (int al = lane; al < nOut; al += 32) {
-    const int degA = c_mi[al].w;
+    // beta runs in graded order: those of degree up to ordIn - |alpha|
+    const int left = ordIn - (g_mi[al] >> 24);
+    const int q0 = lstOff[al], q1 = min(lstOff[al + 1], q0 + (left < 0 ? 0 : nmom(left)));
     double t1 = 0.0, t2 = 0.0, t3 = 0.0, t4 = 0.0;
-    for (int q = lstOff[al]; q < lstOff[al + 1]; q++) {
+#pragma unroll 4
+    for (int q = q0; q < q1; q++) {
       const int ent = lst[q];
-      const int ib = ent & 1023, ig = (ent >> 10) & 1023, db = ent >> 20;
-      if (db > ordIn - degA) break;
+      const int ib = ent & 1023, ig = (ent >> 10) & 1023;
       t1 += a[ib] * i1[ig];
       t2 += a[ib] * i2[ig];
       t3 += a[ib] * i3[ig];
@@ -1193,6 +1230,52 @@ __global__ void l2p_kernel(int n, int NMleaf, int NM, const int *__restrict__ le
   }
   out[i] = o0;
   out[n + i] = o1;
+}
+
+// The same with kL2pSlices threads to a panel, each over every kL2pSlices-th
+// coefficient, their sums added in order: while a thread per panel would leave
+// the chip short of warps, the loop over the coefficients is one chain of loads
+// (320 panels: 15.3 us with a thread per panel, 7.6 sliced; 20,480: 16.3 and
+// 8.1; above kL2pSliced panels the loads of a thread per panel fill HBM).
+constexpr int kL2pSlices = 8;
+constexpr int kL2pSliced = 2 * 148 * 256;
+
+template <typename TQ>
+__global__ void __launch_bounds__(256)
+l2p_sliced_kernel(int n, int NMleaf, int NM, const int *__restrict__ leafOfPanel,
+                  const int *__restrict__ leafFmm, const TQ *__restrict__ Q0,
+                  const TQ *__restrict__ Q1, const double *__restrict__ lec1,
+                  const double *__restrict__ lec2, const double *__restrict__ lec3,
+                  const double *__restrict__ lec4, double alpha, double beta, const double *__restrict__ area,
+                  const double *__restrict__ diagX, double s1, double s2, int swap,
+                  const double *__restrict__ addend, double *out) {
+  constexpr int PB = 256 / kL2pSlices;   // panels per block: one per lane of a warp
+  __shared__ double red[2][kL2pSlices][PB];
+  const int slice = threadIdx.x / PB, lane = threadIdx.x % PB;
+  const int i = blockIdx.x * PB + lane;
+  double a = 0.0, b = 0.0;
+  if (i < n) {
+    const size_t f = (size_t)leafFmm[leafOfPanel[i]] * NM;
+#pragma unroll 4
+    for (int m = slice; m < NMleaf; m += kL2pSlices) {
+      a += (double)Q0[(size_t)m * n + i] * (lec1[f + m] + lec2[f + m]);
+      b += (double)Q1[(size_t)m * n + i] * (lec3[f + m] + lec4[f + m]);
+    }
+  }
+  red[0][slice][lane] = a;
+  red[1][slice][lane] = b;
+  __syncthreads();
+  if (slice > 1 || i >= n) return;   // slice 0 the potential half, slice 1 the other
+  const int from = swap ? 1 - slice : slice;
+  double v = 0.0;
+#pragma unroll
+  for (int w = 0; w < kL2pSlices; w++) v += red[from][w][lane];
+  const size_t at = (size_t)slice * n + i;
+  double o = (beta == 0.0) ? 0.0 : beta * out[at];
+  o += alpha * v;
+  if (diagX) o += (slice ? s2 : s1) * area[i] * diagX[at];
+  if (addend) o += addend[at];
+  out[at] = o;
 }
 
 // ------------------------------------------------------------------------
@@ -1469,6 +1552,18 @@ static bool setup_m2l_adjoint(Context &c) {
   return true;
 }
 
+// the moments of `count` cubes from their children's, two planes
+static bool launch_m2m(Context &c, int first, int count, int ordOut, int ordIn, const int *kidFirst,
+                       const int *kidCount, const double *ctr, double *m1, double *m2, cudaStream_t s) {
+  const int nOut = nmom(ordOut), nLst = c.h_mOff[nOut];
+  const size_t shm = (size_t)kShiftWarps * 5 * nOut * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
+  if (shm > 44 * 1024)
+    FB_CUDA(cudaFuncSetAttribute(m2m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+  m2m_kernel<<<count, kShiftWarps * 32, shm, s>>>(first, count, c.NM, ordOut, ordIn, kidFirst, kidCount, ctr,
+                                                  c.d_mOff, c.d_mLst, nLst, m1, m2);
+  return true;
+}
+
 // Forward: Q2M, M2M, M2L, L2L; the leaves' local expansions end in d_lec.
 // Adjoint (the transposed far operator, read right to left): L2P^T (Q2M with
 // the halves exchanged) -> g12, g34 in d_lec planes 0, 1; L2L^T, which is the
@@ -1493,13 +1588,9 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
                                                   c.d_leafFmm, c.d_Q0, c.d_Q1, sgm, adjoint ? 1 : 0, up1, up2);
   if (marks) cudaEventRecord(marks[0], s);
   for (int lev = depth - 1; lev >= height; lev--) {
-    int ordOut = pt.ordMom[lev], ordIn = pt.ordMom[lev + 1];
-    const int nOut = nmom(ordOut), nLst = c.h_mOff[nOut];
-    const size_t shm = (size_t)kShiftWarps * 5 * nOut * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
-    if (shm > 48 * 1024) cudaFuncSetAttribute(m2m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    m2m_kernel<<<pt.fmmLevelCount[lev], kShiftWarps * 32, shm, s>>>(
-        pt.fmmLevelStart[lev], pt.fmmLevelCount[lev], c.NM, ordOut, ordIn, c.d_kidFirst, c.d_kidCount, c.d_cubeCtr,
-        c.d_mOff, c.d_mLst, nLst, up1, up2);
+    if (!launch_m2m(c, pt.fmmLevelStart[lev], pt.fmmLevelCount[lev], pt.ordMom[lev], pt.ordMom[lev + 1], c.d_kidFirst,
+                    c.d_kidCount, c.d_cubeCtr, up1, up2, s))
+      return false;
   }
   if (marks) cudaEventRecord(marks[1], s);
   if (!launch_m2l_only(c, adjoint, fp64)) return false;
@@ -1511,7 +1602,7 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
     int ordIn = pt.ordMom[lev], ordOut = pt.ordMom[lev + 1];
     const int nOut = nmom(ordOut), nLst = c.h_lstOff[nOut];
     const size_t shm = (size_t)kShiftWarps * 5 * nmom(ordIn) * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
-    if (shm > 48 * 1024) cudaFuncSetAttribute(l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    if (shm > 44 * 1024) cudaFuncSetAttribute(l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
     l2l_kernel<<<ceil_div(pt.fmmLevelCount[lev + 1], kShiftWarps), kShiftWarps * 32, shm, s>>>(
         pt.fmmLevelStart[lev + 1], pt.fmmLevelCount[lev + 1], c.NM, ordIn, ordOut, c.d_fmmParent, c.d_cubeCtr,
         c.d_lstOff, c.d_lst, nLst, d1, d2, c.d_lec + 2 * plane, c.d_lec + 3 * plane);
@@ -1537,15 +1628,16 @@ bool launch_l2p(Context &c, double alpha, double beta, double *out, const double
   // adjoint: Q0 . (adjoint dpdn moments + 0) -> dpdn half, Q1 . (adjoint pot moments + 0) -> pot half
   const double *l1 = adjoint ? c.d_mom + plane : c.d_lec, *l2 = c.d_lec + (adjoint ? 2 : 1) * plane;
   const double *l3 = adjoint ? c.d_mom : c.d_lec + 2 * plane, *l4 = c.d_lec + 3 * plane;
-  if (c.d_Q0F && !fp64)
-    l2p_kernel<float><<<ceil_div(c.n, 256), 256, 0, c.stream>>>(c.n, c.NMleaf, c.NM, c.d_leafOfPanel, c.d_leafFmm,
-                                                                c.d_Q0F, c.d_Q1F, l1, l2, l3, l4, alpha, beta,
-                                                                c.d_area, diagX, s1, s2, adjoint ? 1 : 0, addend, out);
-  else
-    l2p_kernel<double><<<ceil_div(c.n, 256), 256, 0, c.stream>>>(c.n, c.NMleaf, c.NM, c.d_leafOfPanel, c.d_leafFmm,
-                                                                 c.d_Q0, c.d_Q1, l1, l2, l3, l4, alpha, beta,
-                                                                 c.d_area, diagX, s1, s2, adjoint ? 1 : 0, addend,
-                                                                 out);
+  auto run = [&](auto q0, auto q1) {
+    typedef typename std::remove_const<typename std::remove_pointer<decltype(q0)>::type>::type TQ;
+    const bool sliced = c.n <= kL2pSliced;
+    auto kern = sliced ? l2p_sliced_kernel<TQ> : l2p_kernel<TQ>;
+    kern<<<ceil_div(c.n, sliced ? 256 / kL2pSlices : 256), 256, 0, c.stream>>>(
+        c.n, c.NMleaf, c.NM, c.d_leafOfPanel, c.d_leafFmm, q0, q1, l1, l2, l3, l4, alpha, beta, c.d_area, diagX, s1,
+        s2, adjoint ? 1 : 0, addend, out);
+  };
+  if (c.d_Q0F && !fp64) run((const float *)c.d_Q0F, (const float *)c.d_Q1F);
+  else run((const double *)c.d_Q0, (const double *)c.d_Q1);
   FB_CUDA(cudaGetLastError());
   return true;
 }
