@@ -1480,8 +1480,8 @@ bool setup_fmm(Context &c) {
       !c.arena.upload(&c.d_m2lOff, pt.m2lOff, s) || !c.arena.upload(&c.d_m2lSrc, pt.m2lSrc, s) ||
       !c.arena.upload(&c.d_m2lDst, c.h_m2lDst, s))
     return false;
-  if (!c.arena.alloc_n(&c.d_mom, 2 * (size_t)pt.nFmm * c.NM) || !c.arena.alloc_n(&c.d_lec, 4 * (size_t)pt.nFmm * c.NM))
-    return false;
+  if (!c.arena.alloc_n(&c.d_mom, 6 * (size_t)pt.nFmm * c.NM)) return false;
+  c.d_lec = c.d_mom + 2 * (size_t)pt.nFmm * c.NM;   // one buffer, zeroed by one memset per product
   StageTimer tm("fmm_setup", s);
   // M2L derivative tensors, once per geometry
   c.nM2LPairs = (long long)pt.m2lSrc.size();
@@ -1575,8 +1575,7 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
   cudaStream_t s = c.stream;
   const size_t plane = (size_t)pt.nFmm * c.NM;
   if (adjoint && !setup_m2l_adjoint(c)) return false;
-  FB_CUDA(cudaMemsetAsync(c.d_mom, 0, 2 * plane * sizeof(double), s));
-  FB_CUDA(cudaMemsetAsync(c.d_lec, 0, 4 * plane * sizeof(double), s));
+  FB_CUDA(cudaMemsetAsync(c.d_mom, 0, 6 * plane * sizeof(double), s));   // d_lec's planes follow
   c.launches += 1 + 2 * (depth - height);
   // upward arrays: moments (forward) or adjoint locals (adjoint)
   double *up1 = adjoint ? c.d_lec + plane : c.d_mom, *up2 = adjoint ? c.d_lec : c.d_mom + plane;
