@@ -292,6 +292,9 @@ __global__ void charges_to_float_kernel(int m, const double *__restrict__ pos, c
                        (float)(pos[3 * (size_t)j + 2] - oz), (float)chr[j]);
 }
 
+// threads per block of the mixed direct sums, one panel each: 64 while blocks of 256 would be fewer than two per SM
+static int direct_sum_threads(int n) { return n < 2 * 148 * 256 ? 64 : 256; }
+
 // Stages charges [base, base + cnt) as (cnt + 1) / 2 interleaved pairs with
 // negated positions, s[2p] = (-x0 -x1 -y0 -y1), s[2p + 1] = (-z0 -z1 q0 q1),
 // so every packed operand is one half of a staged float4; an odd count pads
@@ -602,8 +605,13 @@ __device__ __forceinline__ void walk_warp(const WalkTree &t, bool active, const 
   }
 }
 
+// Bound by latency, so by resident warps: the FP32 energy walk's 166 registers
+// (orders up to 4) left one block of 8 warps per SM; held to 128, which spills
+// 40 bytes, two fit.  The RHS walk, which needs no sum over the block, runs in
+// blocks of two warps, so that a slow warp holds up only its neighbour.
+// 204,800 panels, 20,000 charges: one right-hand side and one energy took 1.48 ms; 562 and 645 us now.
 template <int PM, typename T, int MODE>
-__global__ void __launch_bounds__(kWalkThreads)
+__global__ void __launch_bounds__(kWalkThreads, sizeof(T) == 4 && PM <= 5 ? 2 : 1)
 tree_walk_kernel(int n, int q, const double *__restrict__ vtx, const double *__restrict__ nrm,
                  const double *__restrict__ area, WalkTree t, double kappa, double eps, double fac,
                  const double *__restrict__ sgm, double *rhs, double *partial) {
@@ -683,7 +691,8 @@ static void launch_walk(Context &c, int mode, const double *sgm, double *rhs, do
                                    : mode == 1 ? tree_walk_kernel<PM, float, 1> : tree_walk_kernel<PM, float, 2>)
                       : (mode == 0 ? tree_walk_kernel<PM, double, 0>
                                    : mode == 1 ? tree_walk_kernel<PM, double, 1> : tree_walk_kernel<PM, double, 2>);
-  kern<<<ceil_div(c.n, kWalkThreads), kWalkThreads, 0, c.stream>>>(
+  const int threads = mode == 0 ? 64 : kWalkThreads;
+  kern<<<ceil_div(c.n, threads), threads, 0, c.stream>>>(
       c.n, c.prm.quad_order, c.d_vtx, c.d_nrm, c.d_area, t, c.prm.kappa, c.epsilon,
       c.rhsFac != 0.0 ? c.rhsFac : kFourPiI / c.prm.eps1, sgm, rhs, partial);
 }
@@ -724,7 +733,8 @@ bool launch_rhs(Context &c, int useTree, double *rhs) {
   if (!useTree && c.mixed && c.prm.quad_order == 1) {
     double ox, oy, oz;
     if (!charges_f32(c, &ox, &oy, &oz)) return false;
-    rhs_direct_f2_kernel<<<ceil_div(c.n, 256), 256, 0, c.stream>>>(
+    const int th = direct_sum_threads(c.n);
+    rhs_direct_f2_kernel<<<ceil_div(c.n, th), th, 0, c.stream>>>(
         c.n, c.nChar, c.d_vtx, c.d_nrm, c.d_area, c.ct->d_chgF, ox, oy, oz,
         c.rhsFac != 0.0 ? c.rhsFac : kFourPiI / c.prm.eps1, rhs);
     FB_CUDA(cudaGetLastError());
