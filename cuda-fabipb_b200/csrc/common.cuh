@@ -110,6 +110,12 @@ struct DevArena {
   }
 };
 
+// gives a set-up step's temporaries back when it ends
+struct ArenaScope {
+  DevArena &a;
+  ~ArenaScope() { a.release(); }
+};
+
 inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 }  // namespace fb

@@ -259,12 +259,6 @@ __global__ void tree_nbr_fill_kernel(TreeCands C, const double *__restrict__ x, 
   nNbr2[c] = i2;
 }
 
-// releases a scratch arena on every return path
-struct ArenaScope {
-  DevArena &a;
-  ~ArenaScope() { a.release(); }
-};
-
 template <typename T>
 static bool d2h_vec(std::vector<T> &h, const T *d, size_t n, cudaStream_t s) {
   h.resize(n);

@@ -1,4 +1,4 @@
-"""Preconditioner, GMRES and translation kernels at the sizes where their dispatch changes, against the FP64
+"""Preconditioner, GMRES, translation and charge-tree kernels at the sizes where their dispatch changes, against the FP64
 restatement oracle.
 
 Tolerances: FP64 operators 1e-12 and block inverses 1e-11 relative L2, as for the golden cases; block inverses of mixed
@@ -94,3 +94,16 @@ def test_far_field_cube_counts(depth, order, precision, tol):
     s, o = lib.Surface(pan, lib.params(precision=precision, **opts)), O.Oracle(pan, O.make_params(**opts))
     v = np.random.default_rng(order).standard_normal(2 * s.n)
     assert rel_l2(s.apply(v, part=lib.FAR), o.far_apply(v)) < tol
+
+
+@pytest.mark.parametrize("order", [1, 3, 6])
+@pytest.mark.parametrize("charges", [1, 2, 33, 257, 3000])
+def test_charge_tree_moments(charges, order):
+    """Right-hand side by the charge tree, whose moments are formed on the device, against the oracle's tree."""
+    pan = cut_sphere(300)
+    rng = np.random.default_rng(charges)
+    ch = meshio.ChargeSet(rng.uniform(-9, 9, (charges, 3)), rng.standard_normal(charges), np.ones(charges))
+    opts = dict(order=order, depth=3, height=2)
+    s = lib.Surface(pan, lib.params(precision=lib.FP64, **opts), charges=ch)
+    o = O.Oracle(pan, O.make_params(**opts), charges=ch)
+    assert rel_l2(s.rhs(use_tree=True), o.rhs_tree()) < 1e-12
