@@ -1115,6 +1115,7 @@ static int special_pairs_device(Context &c, const std::vector<int> &nearSortedFl
   const int n = c.n, nc = 3 * n;
   cudaStream_t s = c.stream;
   DevArena tmp;
+  ArenaScope scope{tmp};
   unsigned long long *keys = nullptr, *keysS = nullptr;
   int *vals = nullptr, *valsS = nullptr, *flag = nullptr, *gid = nullptr, *cornerGroup = nullptr, *gStart = nullptr;
   int *cnt = nullptr, *err = nullptr, *d_nearSorted = nullptr;
@@ -1325,6 +1326,17 @@ static bool special_pairs_host(Context &c, const std::vector<int> &nearSortedFla
 constexpr double kDenseScratch = 512.0 * 1024 * 1024;
 static bool equal_parts(const Context &c) { return c.dense && !c.mixed && c.prm.quad_order == 1; }
 
+// the indices of small non-negative keys, the largest first, equal ones in order (a counting sort)
+static std::vector<int> by_decreasing(const std::vector<int> &key) {
+  int top = 0;
+  for (int k : key) top = std::max(top, k);
+  std::vector<int> at(top + 2, 0), out(key.size());
+  for (int k : key) at[top - k + 1]++;
+  for (int k = 0; k <= top; k++) at[k + 1] += at[k];
+  for (size_t i = 0; i < key.size(); i++) out[at[top - key[i]]++] = (int)i;
+  return out;
+}
+
 static bool setup_near_parts(Context &c) {
   const PanelTree &pt = c.pt;
   cudaStream_t s = c.stream;
@@ -1354,10 +1366,8 @@ static bool setup_near_parts(Context &c) {
   }
   // the finishing kernel's blocks: (part, group of 32 targets), the largest parts first
   std::vector<int2> work;
-  for (int L = 0; L < (int)c.partCount.size(); L++)
+  for (int L : by_decreasing(c.partCount))
     for (int g = 0; g * 32 < c.partCount[L]; g++) work.push_back(make_int2(L, g));
-  std::stable_sort(work.begin(), work.end(),
-                   [&](const int2 &a, const int2 &b) { return c.partCount[a.x] > c.partCount[b.x]; });
   c.nWork = (int)work.size();
   if (!c.arena.upload(&c.d_work, work, s)) return false;
   FB_CUDA(cudaStreamSynchronize(s));   // the host vectors go out of scope
@@ -1368,16 +1378,24 @@ static bool setup_near_parts(Context &c) {
 // parts whose smaller one has at least FB_NEAR_SYM_MIN_LEAF panels, the larger
 // on the register side, largest tasks first.  FABIPB_B200_NEAR_SYM=0 turns them
 // off (every pair in the finishing kernel), as does a mixed direct context
-// whose scratch would pass kDenseScratch.
+// whose scratch would pass kDenseScratch.  In FP64 a pair also needs
+// FB_NEAR_SYM64_MIN_PAIRS panel pairs -- below that a 16 x 16 tile is so empty
+// that two ordered passes cost less -- and the tasks at least half of all
+// panel pairs, else their launches cost more than they save (1,280 panels in
+// leaves of 5: a GMRES solve took 1.04 ms with tasks on every pair, 1.01 in
+// ordered passes).
 #ifndef FB_NEAR_SYM_MIN_LEAF
 #define FB_NEAR_SYM_MIN_LEAF 4
+#endif
+#ifndef FB_NEAR_SYM64_MIN_PAIRS
+#define FB_NEAR_SYM64_MIN_PAIRS 128
 #endif
 // cost of a padded pair on a half-warp, percent of that on a warp
 #ifndef FB_NEAR_SYM16_COST
 #define FB_NEAR_SYM16_COST 110
 #endif
 static bool setup_near_sym(Context &c) {
-  c.nSymTasks = 0;
+  c.nSymTasks = c.nSym32 = 0;
   const PanelTree &pt = c.pt;
   cudaStream_t s = c.stream;
   const char *env = getenv("FABIPB_B200_NEAR_SYM");
@@ -1385,17 +1403,28 @@ static bool setup_near_sym(Context &c) {
   const int nParts = (int)c.partCount.size();
   const std::vector<int> &count = c.partCount;
   const size_t esz = c.mixed ? sizeof(float2) : sizeof(double2);
-  const bool off = (env && atoi(env) == 0) || (c.dense && c.prm.quad_order > 1) ||
+  bool off = (env && atoi(env) == 0) || (c.dense && c.prm.quad_order > 1) ||
                    (c.dense && (double)esz * c.n * nParts > 1.02 * kDenseScratch);
-  auto on_tasks = [&](int a, int b) { return !off && a != b && std::min(count[a], count[b]) >= FB_NEAR_SYM_MIN_LEAF; };
+  auto on_tasks = [&](int a, int b) {
+    return !off && a != b && std::min(count[a], count[b]) >= FB_NEAR_SYM_MIN_LEAF &&
+           (c.mixed || (long long)count[a] * count[b] >= FB_NEAR_SYM64_MIN_PAIRS);
+  };
   // the near parts of part L
   std::vector<int> all;
   if (equal)
     for (int L = 0; L < nParts; L++) all.push_back(L);
   auto near_begin = [&](int L) { return equal ? all.data() : pt.nearSrc.data() + pt.nearOff[L]; };
   auto near_end = [&](int L) { return equal ? all.data() + nParts : pt.nearSrc.data() + pt.nearOff[L + 1]; };
-  std::vector<NearTask> tasks;
-  std::vector<std::vector<int>> slots(nParts);   // per part, the slots of its sums
+  if (!off && !c.mixed) {
+    long long sum = 0, on = 0;
+    for (int L = 0; L < nParts; L++)
+      for (const int *p = near_begin(L); p != near_end(L); p++) {
+        const long long k = (long long)count[L] * count[*p];
+        sum += k;
+        if (on_tasks(L, *p)) on += k;
+      }
+    off = 2 * on < sum;
+  }
   if (!off) {
     // panels of R per task: whole parts up to 256 panels; 64 when that leaves fewer padded 32 x 32
     // tiles than eight for each of the chip's 2,368 resident warps (a task is one warp's serial work)
@@ -1404,8 +1433,12 @@ static bool setup_near_sym(Context &c) {
       for (const int *p = near_begin(L); p != near_end(L); p++)
         if (*p > L) tiles += (long long)((count[L] + 31) / 32) * ((count[*p] + 31) / 32);
     const int chunk = tiles < 8 * 2368 ? 64 : 256;
-    std::vector<long long> cost;
+    constexpr long long kTopCost = 1 << 20;
+    std::vector<NearTask> tasks;
+    std::vector<int> cost;   // panel pairs, at most kTopCost
     std::vector<char> half;
+    int top16 = 0;           // the dearest half-warp task
+    std::vector<int> gatOff(nParts + 1, 0);
     long long tot = 0;
     for (int L = 0; L < nParts; L++)
       for (const int *p = near_begin(L); p != near_end(L); p++) {
@@ -1421,31 +1454,33 @@ static bool setup_near_sym(Context &c) {
         FB_CHECK(tot + cr + (long long)nch * ct < 2147483647LL, "symmetric near-field scratch above 2^31 slots");
         const int scrR = (int)tot;
         tot += cr;
-        slots[R].push_back(scrR);
-        for (int k = 0; k < nch; k++) {
-          const int r0 = k * chunk, r1 = std::min(cr, r0 + chunk);
+        gatOff[R + 1]++;
+        gatOff[T + 1] += nch;
+        for (int r0 = 0; r0 < cr; r0 += chunk) {
+          const int r1 = std::min(cr, r0 + chunk);
           tasks.push_back(NearTask{R, T, r0, r1, scrR, (int)tot});
-          slots[T].push_back((int)tot);
           tot += ct;
-          cost.push_back((long long)(r1 - r0) * ct);
+          cost.push_back((int)std::min((long long)(r1 - r0) * ct, kTopCost));
           half.push_back(small);
+          if (small) top16 = std::max(top16, cost.back());
+          c.nSym32 += small ? 0 : 1;
         }
       }
-    // the warp tasks first, then the half-warp ones, each by decreasing cost
-    std::vector<int> ord(tasks.size());
-    for (size_t i = 0; i < ord.size(); i++) ord[i] = (int)i;
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
-      return half[a] != half[b] ? half[b] != 0 : cost[a] > cost[b];
-    });
-    std::vector<NearTask> sorted(tasks.size());
-    for (size_t i = 0; i < ord.size(); i++) sorted[i] = tasks[ord[i]];
-    c.nSymTasks = (int)sorted.size();
-    c.nSym32 = (int)std::count(half.begin(), half.end(), 0);
+    c.nSymTasks = (int)tasks.size();
     if (c.nSymTasks > 0) {
-      std::vector<int> gatOff(nParts + 1, 0), gatSlot;
-      for (int L = 0; L < nParts; L++) {
-        gatSlot.insert(gatSlot.end(), slots[L].begin(), slots[L].end());
-        gatOff[L + 1] = (int)gatSlot.size();
+      std::vector<NearTask> sorted;
+      sorted.reserve(tasks.size());
+      // the warp tasks first, then the half-warp ones (two to a warp, so neighbours should cost the same), each by
+      // decreasing cost
+      for (size_t i = 0; i < tasks.size(); i++)
+        if (!half[i]) cost[i] += top16 + 1;
+      for (int i : by_decreasing(cost)) sorted.push_back(tasks[i]);
+      // every part's slots, in the order of the tasks' making
+      for (int L = 0; L < nParts; L++) gatOff[L + 1] += gatOff[L];
+      std::vector<int> gatSlot(gatOff[nParts]), at(gatOff.begin(), gatOff.end() - 1);
+      for (const NearTask &t : tasks) {
+        if (t.r0 == 0) gatSlot[at[t.R]++] = t.scrR;
+        gatSlot[at[t.T]++] = t.scrT;
       }
       if (!c.arena.upload(&c.d_symTask, sorted, s) || !c.arena.upload(&c.d_gatOff, gatOff, s) ||
           !c.arena.upload(&c.d_gatSlot, gatSlot, s) || !c.arena.alloc(&c.d_symScr, esz * (size_t)tot) ||
@@ -1584,6 +1619,7 @@ static bool setup_near_adjoint(Context &c) {
   // (ascending) row of Y, on the device
   const int n = c.n;
   DevArena tmp;
+  ArenaScope scope{tmp};
   long long *d_mate = nullptr;
   int *d_bad = nullptr;
   if (!tmp.alloc_n(&d_mate, (size_t)std::max<long long>(c.nSpecial, 1)) || !tmp.alloc_n(&d_bad, 1)) return false;
