@@ -651,7 +651,7 @@ def run_ours(args):
     # the near-field pass: the symmetric kernel (unordered leaf pairs) and the ordered kernel (self
     # pairs, scratch sums, FP64 special pairs), timed together as one apply
     kname = ("near_sym_f2_kernel<0> + near_apply_f2_kernel<0>" if prec == lib.MIXED
-             else "near_sym_kernel<double,0> + near_apply_kernel<double,0>")
+             else "near_sym_kernel<0> + near_apply_kernel<0>")
     kfiles = (("near_sym_f2_kernel", "near_apply_f2_kernel") if prec == lib.MIXED
               else ("near_sym_kernel_double", "near_apply_kernel_double"))
     traffic, traffic_src = None, None

@@ -21,7 +21,6 @@
 // deterministic.
 #include <algorithm>
 #include <cstring>
-#include <thread>
 #include <utility>
 
 #include "context.cuh"
