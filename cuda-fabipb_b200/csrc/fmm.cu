@@ -1236,7 +1236,8 @@ __global__ void l2p_kernel(int n, int NMleaf, int NM, const int *__restrict__ le
 // coefficient, their sums added in order: while a thread per panel would leave
 // the chip short of warps, the loop over the coefficients is one chain of loads
 // (320 panels: 15.3 us with a thread per panel, 7.6 sliced; 20,480: 16.3 and
-// 8.1; above kL2pSliced panels the loads of a thread per panel fill HBM).
+// 8.1; but 204,800: 25.9 and 44, the sums' barrier and the shorter rows costing
+// more once HBM is busy).  The line is two blocks of a thread per panel per SM.
 constexpr int kL2pSlices = 8;
 constexpr int kL2pSliced = 2 * 148 * 256;
 
