@@ -174,7 +174,8 @@ __global__ void identity_kernel(int nList, const int *__restrict__ list, const i
 //     A(:, j) = A(:, j) without the pivot rows + Panel * A(pivot rows, j).
 // Rows are never interchanged: perm[k] is the row that column k was eliminated
 // with, stored column c multiplies input component colSrc[c] = perm[c], and
-// stored row perm[k] is output component rowDst[perm[k]] = k.
+// stored row perm[k] is output component rowDst[perm[k]] = k.  info[b] = k + 1 for the first column whose pivot is
+// zero, not finite or without a finite reciprocal; perm stays a permutation of the rows whatever the values are.
 //
 // 2 M^3 operations; bound by the blocks' traffic in the updates (every panel
 // reads and writes a whole block, and the blocks in work exceed the L2) and by
@@ -205,7 +206,8 @@ __host__ __device__ constexpr size_t inv_smem_bytes(int maxM) {
   return sizeof(TV) * ((size_t)NB * ((maxM + 3) & ~3) + (size_t)NB * 64 * QC) + (size_t)maxM * (sizeof(int) + 1);
 }
 
-// the largest value of the warp and the lowest index among the lanes that hold it (v >= 0, or -1 for none)
+// the largest value of the warp and the lowest index among the lanes that hold it (v >= 0, or -1 for none; a NaN,
+// its sign cleared, counts as larger than infinity)
 __device__ __forceinline__ int warp_first_max(float v, int i) {
   const unsigned b = v < 0.f ? 0u : __float_as_uint(v) + 1u;
   const unsigned m = __reduce_max_sync(0xffffffffu, b);
@@ -217,6 +219,12 @@ __device__ __forceinline__ int warp_first_max(double v, int i) {
   const unsigned lo = hi == mh ? (unsigned)__double2loint(v) : 0u;
   const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
   return __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? i : INT_MAX);
+}
+
+// d = 1/pivot (0 for a zero pivot): the elimination can go on with finite numbers
+template <typename TV>
+__device__ __forceinline__ bool usable_pivot(TV d) {
+  return fabs(d) > (TV)0 && !isinf(d);
 }
 
 template <typename TV, int NB, int CS, int RPT, int QC, int NT>
@@ -276,7 +284,7 @@ pc_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart, c
         for (int r = 0; r < RPT; r++) {
           const int i = t + r * NT;
           const TV a = fabs(v[r][kk]);
-          if (i < M && !((used >> r) & 1u) && a > best) {
+          if (i < M && !((used >> r) & 1u) && !(a <= best)) {   // a NaN is taken too: some row always is
             best = a;
             bi = i;
           }
@@ -302,7 +310,7 @@ pc_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart, c
         const int pw = __ffs(__ballot_sync(0xffffffffu, ci == pv)) - 1;
         const TV piv = cRow[par][pw][kk];
         const TV d = piv != (TV)0 ? (TV)1 / piv : (TV)0;
-        if (piv == (TV)0) bad = bad ? bad : k0 + c0 + kk + 1;
+        if (!usable_pivot(d)) bad = bad ? bad : k0 + c0 + kk + 1;
         if (t == 0) perm[k0 + c0 + kk] = pv;
         TV row[kInvSub];
 #pragma unroll
@@ -1130,7 +1138,7 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   tmp.release();
   FB_CHECK(ok, "preconditioner inversion failed: %s", cudaGetErrorString(cudaGetLastError()));
   for (int b = 0; b < p.nBlocks; b++)
-    FB_CHECK(info[b] == 0, "zero pivot in preconditioner block %d (step %d)", b, info[b]);
+    FB_CHECK(info[b] == 0, "zero or non-finite pivot in preconditioner block %d (step %d)", b, info[b]);
   return true;
 }
 

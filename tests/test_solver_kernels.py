@@ -41,6 +41,23 @@ def test_block_inverse_classes(panels, precision, tol):
     assert rel_l2(s.precond_apply(b), o.precond_apply(b)) < tol
 
 
+@pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
+@pytest.mark.parametrize("panels", [1, 17, 193, 385])
+@pytest.mark.parametrize("where", [0, -1])
+def test_block_inverse_of_a_non_finite_panel(panels, where, precision):
+    """A panel whose normal is 0/0 makes a row and a column of its block NaN: an error in every class, and the
+    context is as good as before."""
+    pan = patch_and_far_panel(panels)
+    normal = pan.normal.copy()
+    normal[0 if where == 0 else panels - 1] = np.nan
+    s = lib.Surface(meshio.PanelSet(pan.vtx, normal, pan.area, pan.face_index),
+                    lib.params(order=2, depth=1, height=1, precision=precision))
+    with pytest.raises(RuntimeError, match="non-finite pivot"):
+        s.precond_setup(2)
+    s.precond_setup(3)   # the diagonal, which reads areas only
+    assert np.isfinite(s.precond_apply(np.ones(2 * s.n))).all()
+
+
 @pytest.mark.parametrize("panels,depth", [(5, 2), (331, 2), (643, 1)])
 def test_adjoint_block_application(panels, depth):
     """The energy is quadratic in the charges, so q . dE/dq = 2 E; the transposed solve takes the forward one's steps."""
