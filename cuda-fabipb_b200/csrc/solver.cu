@@ -476,7 +476,7 @@ pc_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart, c
 // The column interchanges that end Gauss-Jordan are not carried out:
 // colSrc[c] records which input component stored column c multiplies, and
 // the apply kernels gather through it (rowDst is the identity).  info[b] = k+1
-// for an exactly zero pivot k.
+// for the first pivot k that is zero, not finite or without a finite reciprocal.
 constexpr int kGjThreads = 256;
 
 template <typename TV, int NB>
@@ -524,25 +524,24 @@ pc_gj_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart
     // step's write phase also finds the thread's candidate pivot of the next
     // column among its own rows, so a step needs two barriers.
     TV best = (TV)-1;
-    int bi = M;
+    int bi = INT_MAX;
     for (int i = t; i < M; i += kGjThreads) {
       if (i < k0) continue;
       const TV v = fabs(P[i]);
-      if (v > best) { best = v; bi = i; }
+      if (!(v <= best)) { best = v; bi = i; }   // a NaN is taken too: some row always is
     }
     for (int kk = 0; kk < nb; kk++) {
       const int k = k0 + kk;
-      for (int o = 16; o > 0; o >>= 1) {   // first largest within the warp
-        const TV ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+      const int wi = warp_first_max(best, bi);   // first largest within the warp
+      if (wi == INT_MAX) {   // no row left in this warp
+        if (lane == 0) { wbest[warp] = (TV)-1; wbi[warp] = INT_MAX; }
+      } else if (bi == wi) {
+        wbest[warp] = best;
+        wbi[warp] = wi;
       }
-      if (lane == 0) { wbest[warp] = best; wbi[warp] = bi; }
       __syncthreads();
-      int pv = wbi[0];
-      TV pb = wbest[0];
-      for (int w = 1; w < kGjThreads / 32; w++)
-        if (wbest[w] > pb || (wbest[w] == pb && wbi[w] < pv)) { pb = wbest[w]; pv = wbi[w]; }
+      const int pv = warp_first_max(lane < kGjThreads / 32 ? wbest[lane] : (TV)-1,
+                                    lane < kGjThreads / 32 ? wbi[lane] : INT_MAX);
       if (t == 0) perm[k] = pv;
       // read phase: the pivot row (old row pv, scaled; sRk[kk] = 1/pivot) and
       // the old row k, which moves to row pv
@@ -552,12 +551,12 @@ pc_gj_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart
         sRk[t] = (t == kk) ? d : P[t * M + pv] * d;
         sOk[t] = P[t * M + k];
       }
-      if (P[kk * M + pv] == (TV)0) bad = bad ? bad : k + 1;
       __syncthreads();
       // write phase, and the candidates for the next column
       const TV d = sRk[kk];
+      if (!usable_pivot(d)) bad = bad ? bad : k + 1;
       best = (TV)-1;
-      bi = M;
+      bi = INT_MAX;
       const bool more = kk + 1 < nb;
       for (int i = t; i < M; i += kGjThreads) {
         if (i == k) {
@@ -573,7 +572,7 @@ pc_gj_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart
         }
         if (more && i > k) {
           const TV v = fabs(P[(kk + 1) * M + i]);
-          if (v > best) { best = v; bi = i; }
+          if (!(v <= best)) { best = v; bi = i; }
         }
       }
       // the next step's first barrier orders this write phase before its reads

@@ -42,7 +42,7 @@ def test_block_inverse_classes(panels, precision, tol):
 
 
 @pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
-@pytest.mark.parametrize("panels", [1, 17, 193, 385])
+@pytest.mark.parametrize("panels", [1, 17, 193, 385, 800])
 @pytest.mark.parametrize("where", [0, -1])
 def test_block_inverse_of_a_non_finite_panel(panels, where, precision):
     """A panel whose normal is 0/0 makes a row and a column of its block NaN: an error in every class, and the
