@@ -131,13 +131,15 @@ struct NearConstF {
 struct NearPairD {
   double y0, y3, a1, a2, b1, b2;   // a1 = (n_s.d) F, a2 = (n_t.d) F, b1 = (n_s.d) Fi, b2 = (n_t.d) Fi
 };
-// SELF: the target's own leaf, where 1/r of the coincident pair is 0
+// SELF: the two sides may hold panels with the same one-point node (the target's own leaf; any two parts of a
+// direct context, whose runs of panels cut leaves): 1/r of a coincident pair is 0.  (The test reads r2's high word,
+// beside the FP64 pipe; an r2 below the normal numbers counts as 0.)
 template <bool SELF>
 __device__ __forceinline__ NearPairD near_terms(double dx, double dy, double dz, double tnx, double tny, double tnz,
                                                 double snx, double sny, double snz, const NearConstD &K,
                                                 const double *tab) {
   const double r2 = dx * dx + dy * dy + dz * dz;
-  const double g = SELF && !(r2 > 0.0) ? 0.0 : rsqrt_pos(r2);
+  const double g = SELF && __double2hiint(r2) < 0x00100000 ? 0.0 : rsqrt_pos(r2);
   const double r = r2 * g;
   const double e = exp_tab(K.kexp * r, tab);
   const double g2 = g * g, h = g2 * g, he = h * e, hc = he * (K.kappa * r + 1.0);
@@ -434,7 +436,8 @@ near_sym_f2_kernel(int n32, int nTasks, const NearTask *__restrict__ tasks, cons
 // Measured (whole FP64 products, before -> after): star 204,800 panels 1.73 ->
 // 1.34 ms, direct 12,797 panels 1.43 -> 0.44 ms (that one also by taking the
 // direct operator's pairs in equal runs of panels, once for both directions).
-template <bool ADJ, int W, int G>
+// MEET: parts that may hold coincident panels (near_terms).
+template <bool ADJ, bool MEET, int W, int G>
 __device__ __forceinline__ void near_sym_group(double2 *Q, unsigned mask, int hl, int r0, int r1, int rb, int tb,
                                                int tc, double sx, double sy, double sz, bool first,
                                                const double4 *__restrict__ recA, const double4 *__restrict__ recB,
@@ -471,7 +474,7 @@ __device__ __forceinline__ void near_sym_group(double2 *Q, unsigned mask, int hl
       const double wa = B.y, wb = D.y;
 #pragma unroll
       for (int k = 0; k < G; k++) {
-        const NearPairD p = near_terms<false>(ta[k].x - A.x, ta[k].y - A.y, ta[k].z - B.x, tn[k].x, tn[k].y, tn[k].z,
+        const NearPairD p = near_terms<MEET>(ta[k].x - A.x, ta[k].y - A.y, ta[k].z - B.x, tn[k].x, tn[k].y, tn[k].z,
                                               C.x, C.y, D.x, K, tab);
         if (ADJ) {
           acc0[k] += p.y3 * wa - p.a2 * wb;
@@ -498,7 +501,7 @@ __device__ __forceinline__ void near_sym_group(double2 *Q, unsigned mask, int hl
   }
 }
 
-template <bool ADJ, int W>
+template <bool ADJ, bool MEET, int W>
 __device__ __forceinline__ void near_sym_task(const NearTask tk, double2 *Q, const int *__restrict__ leafStart,
                                               const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
                                               const double4 *__restrict__ recA, const double4 *__restrict__ recB,
@@ -512,17 +515,17 @@ __device__ __forceinline__ void near_sym_task(const NearTask tk, double2 *Q, con
   double2 *scrR = scr + tk.scrR, *scrT = scr + tk.scrT;
   int r0 = tk.r0;
   for (; r0 + W < tk.r1; r0 += 2 * W)
-    near_sym_group<ADJ, W, 2>(Q, mask, hl, r0, tk.r1, rb, tb, tc, sx, sy, sz, r0 == tk.r0, recA, recB, K, tab, scrR,
+    near_sym_group<ADJ, MEET, W, 2>(Q, mask, hl, r0, tk.r1, rb, tb, tc, sx, sy, sz, r0 == tk.r0, recA, recB, K, tab, scrR,
                               scrT);
   if (r0 < tk.r1)
-    near_sym_group<ADJ, W, 1>(Q, mask, hl, r0, tk.r1, rb, tb, tc, sx, sy, sz, r0 == tk.r0, recA, recB, K, tab, scrR,
+    near_sym_group<ADJ, MEET, W, 1>(Q, mask, hl, r0, tk.r1, rb, tb, tc, sx, sy, sz, r0 == tk.r0, recA, recB, K, tab, scrR,
                               scrT);
 }
 
 #ifndef FB_NEAR_SYM64_MIN_BLOCKS
 #define FB_NEAR_SYM64_MIN_BLOCKS 4
 #endif
-template <bool ADJ>
+template <bool ADJ, bool MEET>
 __global__ void __launch_bounds__(kSymWarps * 32, FB_NEAR_SYM64_MIN_BLOCKS)
 near_sym_kernel(int n32, int nTasks, const NearTask *__restrict__ tasks, const int *__restrict__ leafStart,
                 const int *__restrict__ leafCount, const double *__restrict__ leafCtr,
@@ -535,11 +538,11 @@ near_sym_kernel(int n32, int nTasks, const NearTask *__restrict__ tasks, const i
   if ((int)blockIdx.x < blocks32) {
     const int warp = threadIdx.x >> 5, task = blockIdx.x * kSymWarps + warp;
     if (task < n32)   // warp-uniform
-      near_sym_task<ADJ, 32>(tasks[task], sQ + warp * 128, leafStart, leafCount, leafCtr, recA, recB, K, tab, scr);
+      near_sym_task<ADJ, MEET, 32>(tasks[task], sQ + warp * 128, leafStart, leafCount, leafCtr, recA, recB, K, tab, scr);
   } else {
     const int half = threadIdx.x >> 4, task = n32 + ((int)blockIdx.x - blocks32) * 2 * kSymWarps + half;
     if (task < nTasks)   // uniform over the half-warp
-      near_sym_task<ADJ, 16>(tasks[task], sQ + half * 64, leafStart, leafCount, leafCtr, recA, recB, K, tab, scr);
+      near_sym_task<ADJ, MEET, 16>(tasks[task], sQ + half * 64, leafStart, leafCount, leafCtr, recA, recB, K, tab, scr);
   }
 }
 
@@ -706,7 +709,7 @@ near_apply_kernel(const int2 *__restrict__ work, const int *__restrict__ leafSta
                   const int *__restrict__ spOff, const int *__restrict__ spSrc, const double4 *__restrict__ spK,
                   const double *__restrict__ sgm, const double *__restrict__ area, int n, NearConstD K, double coef,
                   int accumulate, double *out, const int *__restrict__ gatOff, const int *__restrict__ gatSlot,
-                  const double2 *__restrict__ scr) {
+                  const double2 *__restrict__ scr, bool meet) {
   __shared__ double4 sA[kNearWarps][32], sB[kNearWarps][32];
   __shared__ double tab[kExpTab];
   load_exp_tab(tab);
@@ -737,7 +740,7 @@ near_apply_kernel(const int2 *__restrict__ work, const int *__restrict__ leafSta
       if (lane < m)
         near_record<double>(sb + j0 + lane, n, tgtP, tgtN, area, sgm, sA[warp][lane], sB[warp][lane]);
       __syncwarp();
-      if (S == L) {   // warp-uniform
+      if (S == L || meet) {   // warp-uniform; meet: any two parts may hold coincident panels
 #pragma unroll 2
         for (int jj = sub; jj < m; jj += k)
           near_pair<ADJ, true>(sA[warp][jj], sB[warp][jj], tx, ty, tz, tn, K, tab, p.s0, p.s1);
@@ -1354,8 +1357,7 @@ static bool setup_near_parts(Context &c) {
     c.partCount.clear();
     partOf.resize(c.n);
     for (int i = 0; i < c.n; i += len) {
-      const int L = (int)(std::upper_bound(pt.leafStart.begin(), pt.leafStart.end(), i) - pt.leafStart.begin()) - 1;
-      for (int k = 0; k < 3; k++) ctr.push_back(pt.t.x[3 * (size_t)pt.leafCube[L] + k]);   // the first panel's leaf
+      ctr.insert(ctr.end(), 3, 0.0);   // one frame for all: coincident panels of two parts differ by exactly 0
       for (int j = i; j < std::min(c.n, i + len); j++) partOf[j] = (int)c.partStart.size();
       c.partStart.push_back(i);
       c.partCount.push_back(std::min(len, c.n - i));
@@ -1550,22 +1552,22 @@ template <bool ADJ>
 static void launch_near_f64(Context &c, const double *sgm, double coef, double *out, cudaStream_t s, bool accumulate) {
   const double kap = c.prm.kappa, eps = c.epsilon;
   const NearConstD K{kap, -kap * kExpScale, eps, 1.0 / eps, kap * kap};
-  const bool own = !c.mixed, sym = own && c.nSymTasks > 0;
+  const bool own = !c.mixed, sym = own && c.nSymTasks > 0, meet = equal_parts(c);
   const double4 *tgtP = (const double4 *)(own ? c.d_tgtP : c.d_tgtP64);
   const double4 *tgtN = (const double4 *)(own ? c.d_tgtN : c.d_tgtN64);
   if (sym) {
     double4 *recA = (double4 *)c.d_recA, *recB = (double4 *)c.d_recB;
     near_pack_kernel<double><<<ceil_div(c.n, 256), 256, 0, s>>>(c.n, tgtP, tgtN, c.d_area, sgm, recA, recB);
     const unsigned blocks = ceil_div(c.nSym32, kSymWarps) + ceil_div(c.nSymTasks - c.nSym32, 2 * kSymWarps);
-    near_sym_kernel<ADJ><<<blocks, kSymWarps * 32, 0, s>>>(c.nSym32, c.nSymTasks, c.d_symTask, c.d_partStart,
-                                                           c.d_partCount, c.d_partCtr, recA, recB, K,
-                                                           (double2 *)c.d_symScr);
+    auto kern = meet ? near_sym_kernel<ADJ, true> : near_sym_kernel<ADJ, false>;
+    kern<<<blocks, kSymWarps * 32, 0, s>>>(c.nSym32, c.nSymTasks, c.d_symTask, c.d_partStart, c.d_partCount,
+                                           c.d_partCtr, recA, recB, K, (double2 *)c.d_symScr);
     c.launches += 2;
   }
   near_apply_kernel<ADJ><<<c.nWork, kNearWarps * 32, 0, s>>>(
       c.d_work, c.d_partStart, c.d_partCount, own ? c.d_ordOff : c.d_nearOff, own ? c.d_ordSrc : c.d_nearSrc,
       c.d_partCtr, tgtP, tgtN, c.d_spOff, c.d_spSrc, ADJ ? c.d_spKT : c.d_spK, sgm, c.d_area, c.n, K, coef,
-      accumulate ? 1 : 0, out, sym ? c.d_gatOff : nullptr, c.d_gatSlot, (const double2 *)c.d_symScr);
+      accumulate ? 1 : 0, out, sym ? c.d_gatOff : nullptr, c.d_gatSlot, (const double2 *)c.d_symScr, meet);
   c.launches += 1;
 }
 

@@ -81,3 +81,20 @@ def test_direct_operator_parts(panels, depth, precision, tol):
     opts = dict(order=3, depth=depth, sep_ratio=1e-9)
     s = lib.Surface(pan, lib.params(precision=precision, **opts), direct=True)
     check(s, O.Oracle(pan, O.make_params(**opts)), tol)
+
+
+@pytest.mark.parametrize("panels,doubled", [(641, 40), (1280, 100)])
+@pytest.mark.parametrize("sym", ["1", "0"])
+def test_direct_operator_coincident_panels(panels, doubled, sym, monkeypatch):
+    """Doubled faces whose two panels fall into different runs of 128: their one-point term is 0 and their
+    special-pair value stands alone, in the symmetric tasks and in the ordered passes."""
+    monkeypatch.setenv("FABIPB_B200_NEAR_SYM", sym)
+    pan = cut_sphere(panels, seed=panels)
+    twice = np.r_[np.arange(panels), np.linspace(0, panels - 1, doubled).astype(int)]
+    pan = meshio.PanelSet(pan.vtx[twice], pan.normal[twice], pan.area[twice], np.arange(len(twice), dtype=np.int32))
+    opts = dict(order=3, depth=1, height=1, sep_ratio=1e-9)
+    s = lib.Surface(pan, lib.params(precision=lib.FP64, **opts), direct=True)
+    run = np.empty(len(twice), int)
+    run[s.panel_order()] = np.arange(len(twice)) // 128
+    assert (run[twice[panels:]] != run[panels:]).any()
+    check(s, O.Oracle(pan, O.make_params(**opts)), 1e-12)
