@@ -30,6 +30,7 @@
 
 #include "context.cuh"
 #include "fastmath.cuh"
+#include "near_plan.hpp"
 #include "quad.cuh"
 
 namespace fb {
@@ -1324,9 +1325,7 @@ static bool special_pairs_host(Context &c, const std::vector<int> &nearSortedFla
 
 // The parts that the near-field kernels pair up: the leaves.  A direct context
 // pairs everything with everything, so in FP64, where positions need no
-// leaf's frame, its parts are equal runs of panels: of 128, or so many that the
-// symmetric tasks' scratch (16 bytes per panel and part) stays under 512 MiB.
-constexpr double kDenseScratch = 512.0 * 1024 * 1024;
+// leaf's frame, its parts are equal runs of panels (equal_part_length).
 static bool equal_parts(const Context &c) { return c.dense && !c.mixed && c.prm.quad_order == 1; }
 
 // the indices of small non-negative keys, the largest first, equal ones in order (a counting sort)
@@ -1352,7 +1351,7 @@ static bool setup_near_parts(Context &c) {
   std::vector<int> partOf;
   std::vector<double> ctr;
   if (equal_parts(c)) {
-    const int len = std::max(128, (int)(16.0 * c.n / kDenseScratch * c.n / 64 + 1) * 64);
+    const int len = equal_part_length(c.n);
     c.partStart.clear();
     c.partCount.clear();
     partOf.resize(c.n);
@@ -1378,9 +1377,9 @@ static bool setup_near_parts(Context &c) {
 
 // The symmetric near field's tasks: every unordered pair of distinct near
 // parts whose smaller one has at least FB_NEAR_SYM_MIN_LEAF panels, the larger
-// on the register side, largest tasks first.  FABIPB_B200_NEAR_SYM=0 turns them
-// off (every pair in the finishing kernel), as does a mixed direct context
-// whose scratch would pass kDenseScratch.  In FP64 a pair also needs
+// on the register side, largest tasks first, cut into chunks by
+// plan_near_tasks.  FABIPB_B200_NEAR_SYM=0 turns them off (every pair in the
+// finishing kernel), as does a plan without tasks.  In FP64 a pair also needs
 // FB_NEAR_SYM64_MIN_PAIRS panel pairs -- below that a 16 x 16 tile is so empty
 // that two ordered passes cost less -- and the tasks at least half of all
 // panel pairs, else their launches cost more than they save (1,280 panels in
@@ -1405,8 +1404,7 @@ static bool setup_near_sym(Context &c) {
   const int nParts = (int)c.partCount.size();
   const std::vector<int> &count = c.partCount;
   const size_t esz = c.mixed ? sizeof(float2) : sizeof(double2);
-  bool off = (env && atoi(env) == 0) || (c.dense && c.prm.quad_order > 1) ||
-                   (c.dense && (double)esz * c.n * nParts > 1.02 * kDenseScratch);
+  bool off = (env && atoi(env) == 0) || (c.dense && c.prm.quad_order > 1);
   auto on_tasks = [&](int a, int b) {
     return !off && a != b && std::min(count[a], count[b]) >= FB_NEAR_SYM_MIN_LEAF &&
            (c.mixed || (long long)count[a] * count[b] >= FB_NEAR_SYM64_MIN_PAIRS);
@@ -1427,14 +1425,18 @@ static bool setup_near_sym(Context &c) {
       }
     off = 2 * on < sum;
   }
+  NearPlan plan;
   if (!off) {
-    // panels of R per task: whole parts up to 256 panels; 64 when that leaves fewer padded 32 x 32
-    // tiles than eight for each of the chip's 2,368 resident warps (a task is one warp's serial work)
-    long long tiles = 0;
-    for (int L = 0; L < nParts; L++)
-      for (const int *p = near_begin(L); p != near_end(L); p++)
-        if (*p > L) tiles += (long long)((count[L] + 31) / 32) * ((count[*p] + 31) / 32);
-    const int chunk = tiles < 8 * 2368 ? 64 : 256;
+    const double directLimit = !c.dense ? 0.0 : equal ? equal_part_scratch(c.n) : 1.02 * kNearScratch;
+    plan = plan_near_tasks(count, esz, directLimit, [&](auto &&f) {
+      for (int L = 0; L < nParts; L++)
+        for (const int *p = near_begin(L); p != near_end(L); p++)
+          if (*p > L) f(L, *p, on_tasks(L, *p));
+    });
+    off = !plan.tasks;
+  }
+  if (!off) {
+    const int chunk = plan.chunk;
     constexpr long long kTopCost = 1 << 20;
     std::vector<NearTask> tasks;
     std::vector<int> cost;   // panel pairs, at most kTopCost
@@ -1453,7 +1455,6 @@ static bool setup_near_sym(Context &c) {
         const long long p16 = (long long)((cr + 15) / 16) * ((ct + 15) / 16) * 256;
         const bool small = p16 * FB_NEAR_SYM16_COST < p32 * 100;
         const int nch = (cr + chunk - 1) / chunk;
-        FB_CHECK(tot + cr + (long long)nch * ct < 2147483647LL, "symmetric near-field scratch above 2^31 slots");
         const int scrR = (int)tot;
         tot += cr;
         gatOff[R + 1]++;

@@ -98,3 +98,20 @@ def test_direct_operator_coincident_panels(panels, doubled, sym, monkeypatch):
     run[s.panel_order()] = np.arange(len(twice)) // 128
     assert (run[twice[panels:]] != run[panels:]).any()
     check(s, O.Oracle(pan, O.make_params(**opts)), 1e-12)
+
+
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-13), (lib.MIXED, 5e-6)])
+def test_direct_operator_long_parts(precision, tol, monkeypatch):
+    """Parts and chunks above 256 panels, where the direct context's scratch bound sets them: the symmetric tasks
+    against the ordered passes of the same context.  FP64: two orders of 1e5 sums of random sign, 2^-53 * sqrt(1e5)."""
+    unit, faces = meshgen.octasphere(112)
+    pan = meshio.build_panels(20.0 * unit, unit, faces)
+    v = np.random.default_rng(5).standard_normal(2 * pan.n)
+    out = []
+    for sym in ("1", "0"):
+        monkeypatch.setenv("FABIPB_B200_NEAR_SYM", sym)
+        s = lib.Surface(pan, lib.params(precision=precision, order=3, depth=3, height=2), direct=True)
+        out.append(s.apply(v, part=lib.NEAR))
+        out.append(s.apply_adjoint(v, part=lib.NEAR))
+        s.close()
+    assert rel_l2(out[0], out[2]) < tol and rel_l2(out[1], out[3]) < tol
