@@ -1336,10 +1336,19 @@ __device__ __forceinline__ void block_store_partial(double acc, double *red, dou
 // Langou, Ananthan, Yang and Thomas (Numer. Linear Algebra Appl. 28, 2021).
 // gs_dots_kernel takes all products at once (and the newest column's Gram row),
 // gs_update_kernel solves and subtracts, mgs_norm_scale_kernel normalises and
-// takes the Givens step: three launches per step.  One launch per column
+// takes the Givens step: three launches per step (four above kGsStage columns,
+// where gs_solve_kernel solves).  One launch per column
 // took 5.3 us each (20,000 panels: 529 us for the 19 steps of two solves); these
 // take 4.6, 4.7 and 5.0 us (271 us).
 constexpr int kGsCols = 8;   // columns per pass over w in gs_dots_kernel
+
+// the sum of one product's partials, in a fixed order, in every lane
+__device__ __forceinline__ double warp_sum_partials(const double *__restrict__ part, int lane) {
+  double s = 0.0;
+  for (int b = lane; b < kRedBlocks; b += 32) s += part[b];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
 
 // part[k][block] = partial of w.v_k (k < i), part[i + k][block] = partial of v_{i-1}.v_k (k < i - 1)
 __global__ void __launch_bounds__(kRedThreads)
@@ -1385,47 +1394,44 @@ gs_dots_kernel(long long n, int i, const double *__restrict__ V, const double *_
   }
 }
 
-// every block: the sums of the partials in the same order, h from (I + L) h = c (block 0 stores h and the
-// newest Gram row), its share of w -= V h and the partial of w.w.  Dynamic shared memory: gs_smem(i) bytes; the
-// older Gram rows are read there up to kGsStage columns, from global memory above.
+// every block: the sums of the partials in the same order, h from (I + L) h = c (block 0 stores h and the newest Gram
+// row), its share of w -= V h and the partial of w.w.  SOLVE: up to kGsStage columns, whose Gram rows every block holds
+// in gs_smem(i) bytes of dynamic shared memory; above, gs_solve_kernel has formed h and the Gram row.
 constexpr int kGsStage = 64;
-static size_t gs_smem(int i) { return sizeof(double) * (i <= kGsStage ? (size_t)i * (i + 1) : 2 * (size_t)i); }
+static size_t gs_smem(int i) { return i <= kGsStage ? sizeof(double) * i * (i + 1) : 0; }
+template <bool SOLVE>
 __global__ void __launch_bounds__(kRedThreads)
 gs_update_kernel(long long n, int i, int ldg, const double *__restrict__ V, const double *__restrict__ part,
                  double *G, double *hOut, double *w, double *partOut) {
   extern __shared__ double gsSmem[];
   __shared__ double red[kRedThreads];
-  double *h = gsSmem, *row = gsSmem + i, *L = row + i;   // [i], the newest Gram row, the others [i - 1][i] (row k: j < k)
-  const bool staged = i <= kGsStage;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (staged)
+  const double *h = hOut;
+  if constexpr (SOLVE) {
+    double *c = gsSmem, *row = gsSmem + i, *L = row + i;   // [i], the newest Gram row, the others [i - 1][i] (row k: j < k)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int e = threadIdx.x; e < (i - 1) * i; e += blockDim.x) {
       const int k = e / i, j = e % i;
       if (j < k) L[e] = G[(size_t)k * ldg + j];
     }
-  for (int q = warp; q < 2 * i - 1; q += kRedThreads / 32) {
-    double s = 0.0;
-    for (int b = lane; b < kRedBlocks; b += 32) s += part[(size_t)q * kRedBlocks + b];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-      if (q < i) h[q] = s;
-      else row[q - i] = s;
+    for (int q = warp; q < 2 * i - 1; q += kRedThreads / 32) {
+      const double s = warp_sum_partials(part + (size_t)q * kRedBlocks, lane);
+      if (lane == 0) (q < i ? c[q] : row[q - i]) = s;
     }
+    __syncthreads();
+    if (warp == 0)   // forward substitution, column by column
+      for (int k = 0; k < i; k++) {
+        const double hk = c[k];
+        for (int j = k + 1 + lane; j < i; j += 32) c[j] -= hk * (j == i - 1 ? row[k] : L[j * i + k]);
+        __syncwarp();
+      }
+    __syncthreads();
+    if (blockIdx.x == 0)
+      for (int k = threadIdx.x; k < i; k += blockDim.x) {
+        hOut[k] = c[k];
+        if (k < i - 1) G[(size_t)(i - 1) * ldg + k] = row[k];
+      }
+    h = c;
   }
-  __syncthreads();
-  if (warp == 0)   // forward substitution, column by column
-    for (int k = 0; k < i; k++) {
-      const double hk = h[k];
-      for (int j = k + 1 + lane; j < i; j += 32)
-        h[j] -= hk * (j == i - 1 ? row[k] : staged ? L[j * i + k] : G[(size_t)j * ldg + k]);
-      __syncwarp();
-    }
-  __syncthreads();
-  if (blockIdx.x == 0)
-    for (int k = threadIdx.x; k < i; k += blockDim.x) {
-      hOut[k] = h[k];
-      if (k < i - 1) G[(size_t)(i - 1) * ldg + k] = row[k];
-    }
   double acc = 0.0;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     double we = w[e];
@@ -1435,6 +1441,46 @@ gs_update_kernel(long long n, int i, int ldg, const double *__restrict__ V, cons
     acc += we * we;
   }
   block_store_partial(acc, red, partOut);
+}
+
+// h and the newest Gram row of a step with more than kGsStage columns, any number of them, by one block, 32 rows of
+// (I + L) h = c at a time: a warp per row sums the columns solved before, then one warp solves the triangle of 32.
+// Bound by the latency of i / 32 dependent rounds.  (1,568 panels, a step's mean time in a cycle of 200, 1,000 and
+// 2,000 columns: 554, 2,505 and 4,874 us with a launch per column, 179, 1,316 and 5,530 with every block of the update
+// solving for itself from global memory, 158, 486 and 1,015 so.)
+constexpr int kGsRows = 32;
+__global__ void __launch_bounds__(kGsRows * 32)
+gs_solve_kernel(int i, int ldg, const double *__restrict__ part, double *G, double *h) {
+  __shared__ double rest[kGsRows];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double *row = G + (size_t)(i - 1) * ldg;
+  for (int q = warp; q < 2 * i - 1; q += kGsRows) {
+    const double s = warp_sum_partials(part + (size_t)q * kRedBlocks, lane);
+    if (lane == 0) (q < i ? h[q] : row[q - i]) = s;
+  }
+  __syncthreads();
+  for (int k0 = 0; k0 < i; k0 += kGsRows) {
+    const int k = k0 + warp;
+    if (k < i) {   // warp-uniform
+      double s = 0.0;
+#pragma unroll 4
+      for (int j = lane; j < k0; j += 32) s += G[(size_t)k * ldg + j] * h[j];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) rest[warp] = h[k] - s;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int m = min(kGsRows, i - k0);
+      const double *Lr = G + (size_t)(k0 + min(lane, m - 1)) * ldg + k0;   // this lane's row
+      double x = lane < m ? rest[lane] : 0.0;
+      for (int j = 0; j < m; j++) {
+        const double hj = __shfl_sync(0xffffffffu, x, j);
+        if (lane > j && lane < m) x -= Lr[j] * hj;
+      }
+      if (lane < m) h[k0 + lane] = x;
+    }
+    __syncthreads();
+  }
 }
 
 static bool dot_dev(Context &c, long long n, const double *x, const double *y, double *out, bool sq) {
@@ -1726,11 +1772,12 @@ bool gmres_solve(Context &c, const double *b, double *x, int restrt, int maxit, 
       // modified Gram-Schmidt of w against v_0 .. v_{i-1}, then the Givens step
       double *norm = p.d_part + 2 * (size_t)restrt * kRedBlocks;
       gs_dots_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, i, p.d_V, p.d_w, p.d_part);
-      gs_update_kernel<<<kRedBlocks, kRedThreads, gs_smem(i), s>>>(n2, i, restrt, p.d_V, p.d_part, p.d_G, p.d_h, p.d_w,
-                                                                 norm);
+      if (i > kGsStage) gs_solve_kernel<<<1, kGsRows * 32, 0, s>>>(i, restrt, p.d_part, p.d_G, p.d_h);
+      auto update = i <= kGsStage ? gs_update_kernel<true> : gs_update_kernel<false>;
+      update<<<kRedBlocks, kRedThreads, gs_smem(i), s>>>(n2, i, restrt, p.d_V, p.d_part, p.d_G, p.d_h, p.d_w, norm);
       mgs_norm_scale_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n2, norm, p.d_h, p.d_w, p.d_V + (size_t)i * n2, p.d_H,
                                                                ldh, restrt, p.d_sv, i, it, maxit, bnrm2, tol, d_st);
-      c.launches += 3;
+      c.launches += i > kGsStage ? 4 : 3;
       FB_CUDA(cudaGetLastError());
       if (!read_status(c, d_st, h_st)) return false;
       *resid = h_st->resid;

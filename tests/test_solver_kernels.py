@@ -100,6 +100,32 @@ def test_gmres_restart_lengths(restart):
     assert rel_l2(x, xr) < 1e-8
 
 
+def cloud():
+    """49 ellipsoids of 32 panels whose areas spread evenly over 1 to 65: without a preconditioner a decade in 65 steps."""
+    unit, faces = meshgen.octasphere(2)
+    rng = np.random.default_rng(1)
+    parts = []
+    for i in range(49):
+        r, axes = 4 * np.exp(rng.uniform(np.log(0.2), 0)), np.exp(rng.uniform(-0.4, 0.4, 3))
+        normal = unit / axes
+        normal /= np.linalg.norm(normal, axis=1)[:, None]
+        at = 12.0 * np.array([i % 4, i // 4 % 4, i // 16])
+        parts.append(meshio.build_panels(r * unit * axes + at, normal, faces))
+    return meshio.PanelSet(*(np.concatenate([getattr(p, f) for p in parts])
+                             for f in ("vtx", "normal", "area", "face_index")))
+
+
+def test_gmres_cycle_of_thousands_of_columns():
+    """One cycle of more columns than a block's shared memory holds coefficients: every step is taken, and the iterate
+    solves the system as far as 64 bits go (condition 80 * 65, so a residual below 5200 * 2^-53 * sqrt(3000) = 3e-11)."""
+    s = lib.Surface(cloud(), lib.params(precision=lib.FP64, order=3, depth=3))
+    s.precond_setup(-1)
+    b = np.random.default_rng(4).standard_normal(2 * s.n)
+    x, it, _, info = s.solve(b, np.zeros(2 * s.n), restart=3000, maxit=3000, tol=1e-300)
+    assert (it, info) == (3000, 1)
+    assert np.linalg.norm(b - s.matvec(x)) <= 3e-11 * np.linalg.norm(b)
+
+
 @pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-12), (lib.MIXED, 5e-6)])
 @pytest.mark.parametrize("order", [1, 2, 3, 5, 7])
 @pytest.mark.parametrize("depth", [3, 4])
