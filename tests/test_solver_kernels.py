@@ -4,8 +4,11 @@ restatement oracle.
 Tolerances: FP64 operators 1e-12 and block inverses 1e-11 relative L2, as for the golden cases; block inverses of mixed
 contexts 1e-4 (FP32 inverses of well-conditioned blocks: rows * 2^-24 <= 1536 * 6e-8); mixed operators 5e-6.
 """
+import functools
+
 import numpy as np
 import pytest
+import scipy.linalg
 
 from conftest import rel_l2
 from fabipb_b200 import lib, meshgen, meshio
@@ -30,7 +33,8 @@ def patch_and_far_panel(panels):
 @pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-11), (lib.MIXED, 1e-4)])
 @pytest.mark.parametrize("panels", [1, 3, 4, 8, 9, 17, 191, 192, 193, 384, 385, 768, 769])
 def test_block_inverse_classes(panels, precision, tol):
-    """Blocks of 2 * panels rows on both sides of every class of the inversion, and of every batch of the application."""
+    """Blocks of 2 * panels + 2 rows (the patch and the far panel) on both sides of every class of the inversion, and of
+    every batch of the application.  Their pivots all lie on the diagonal; test_block_inverse_pivoting has others."""
     pan = patch_and_far_panel(panels)
     opts = dict(order=2, depth=1, height=1)
     s, o = lib.Surface(pan, lib.params(precision=precision, **opts)), O.Oracle(pan, O.make_params(**opts))
@@ -39,6 +43,59 @@ def test_block_inverse_classes(panels, precision, tol):
     o.precond_setup(2)
     b = np.random.default_rng(panels).standard_normal(2 * s.n)
     assert rel_l2(s.precond_apply(b), o.precond_apply(b)) < tol
+
+
+def three_sheets(panels):
+    """Three parallel sheets of a third of the panels each, 0.3 and 0.2 panel widths apart: the double-layer values of
+    facing panels are above the diagonal, and partial pivoting takes a panel's column to another sheet's row."""
+    unit, faces = meshgen.icosphere(4)
+    pan = meshio.build_panels(20.0 * unit, unit, faces)
+    order, width = np.argsort(-pan.vtx[:, :, 2].mean(1)), np.sqrt(pan.area.mean())
+    parts = []
+    for k, r in enumerate(1.0 + width / 20.0 * np.array([0.0, 0.3, 0.5])):
+        a = np.sort(order[:(panels + 2 - k) // 3])
+        parts.append((r * pan.vtx[a], pan.normal[a], r * r * pan.area[a]))
+    return meshio.PanelSet(*(np.concatenate(x) for x in zip(*parts)), np.arange(panels, dtype=np.int32))
+
+
+@functools.lru_cache(maxsize=None)
+def moved_pivots(panels):
+    """Columns of the three sheets' block whose pivot's own column has yet another pivot, by LAPACK on the host."""
+    o = O.Oracle(three_sheets(panels), O.make_params(order=2, depth=1, height=1))
+    n, area, eps = o.n, o.area(), 80.0
+    K = np.array([[o.panel_ia0(x, y) for y in range(n)] for x in range(n)])
+    A = -np.block([[K[..., 1], K[..., 3]], [K[..., 0], K[..., 2]]])
+    A[np.diag_indices(2 * n)] += np.r_[(1 + eps) / 2 * area, (1 + 1 / eps) / 2 * area]
+    b = np.random.default_rng(0).standard_normal(2 * n)
+    o.precond_setup(2)
+    assert rel_l2(np.linalg.solve(A, b), o.precond_apply(b)) < 1e-12   # the block that the preconditioner inverts
+    perm = np.arange(2 * n)
+    for k, j in enumerate(scipy.linalg.lu_factor(A)[1]):
+        perm[[k, j]] = perm[[j, k]]
+    return int((perm[perm] != np.arange(2 * n)).sum())
+
+
+@pytest.mark.parametrize("panels", [17, 192, 193, 384, 385, 768, 769])
+@pytest.mark.parametrize("precision,tol", [(lib.FP64, 1e-11), (lib.MIXED, 2e-3)])
+def test_block_inverse_pivoting(panels, precision, tol):
+    """Blocks of 2 * panels rows, the last and first of every class, whose pivots lie off the diagonal, in cycles of
+    three and more.  The application against the oracle: the blocks' condition is 550, so an FP32 inverse is within
+    550 * 2^-24 * sqrt(1538) = 1.3e-3.  The transposed application by the steps of the adjoint solve of the direct
+    operator, of which the block is all: as many as the forward solve takes, 5 or 6; with the index lists left out or
+    exchanged it takes 15 to 26."""
+    assert moved_pivots(panels) > 1.5 * panels
+    pan = three_sheets(panels)
+    opts = dict(order=2, depth=1, height=1)
+    s, o = lib.Surface(pan, lib.params(precision=precision, **opts), direct=True), O.Oracle(pan, O.make_params(**opts))
+    s.precond_setup(2)
+    o.precond_setup(2)
+    b = np.random.default_rng(panels).standard_normal(2 * s.n)
+    assert rel_l2(s.precond_apply(b), o.precond_apply(b)) < tol
+    rng = np.random.default_rng(1)
+    s.set_charges(meshio.ChargeSet(rng.uniform(-5, 5, (7, 3)), rng.standard_normal(7), np.ones(7)))
+    _, it, _, info = s.forward(restart=30, maxit=30, tol=1e-10)
+    _, _, it_t, _, info_t = s.backward(1.0, restart=30, maxit=30, tol=1e-10)
+    assert info == 0 and info_t == 0 and it <= 8 and abs(it - it_t) <= 1
 
 
 @pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
