@@ -1018,11 +1018,14 @@ static bool launch_gj(int nb, int nList, int maxM, cudaStream_t st, const int *d
 
 template <typename TV, int NB, int CS, int RPT, int QC, int NT>
 static bool launch_inv_t(int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p, TV *inv,
-                         int *d_info) {
+                         int *d_info, bool share) {
   FB_CHECK(maxM <= RPT * NT, "inversion class of %d rows given %d", RPT * NT, maxM);
   const size_t shm = inv_smem_bytes<TV, NB, QC>(maxM);
   FB_CUDA(cudaFuncSetAttribute(pc_invert_kernel<TV, NB, CS, RPT, QC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)shm));
+  FB_CUDA(cudaFuncSetAttribute(pc_invert_kernel<TV, NB, CS, RPT, QC, NT>,
+                               cudaFuncAttributePreferredSharedMemoryCarveout,
+                               share ? cudaSharedmemCarveoutMaxShared : cudaSharedmemCarveoutDefault));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nList * CS));
   cfg.blockDim = dim3(NT);
@@ -1041,41 +1044,49 @@ static bool launch_inv_t(int nList, int maxM, cudaStream_t st, const int *d_list
   return true;
 }
 
-// Size classes per precision: rows up to, panel width.  Blocks of up to 1,536
-// rows go to pc_invert_kernel on one, two or four CTAs of 256 threads, two per
-// SM, so that one's pivots hide behind the other's updates (FP64 above 768
-// rows: 512 threads, one per SM); larger ones to pc_gj_invert_kernel; blocks
-// above the last class go to cuSOLVER (FP64).  FP32, 422 blocks of 385 to 768
-// rows: 11.7 ms on two CTAs, 14.6 on four, 21.9 on eight (each CTA repeats the
-// pivots), 13.7 with 512 threads; 91 blocks of 769 to 1,226 rows, panels of
-// 16: 15.0 ms on four, 21.7 on two, 18.1 on eight; panels of 32: 15.7 and more
-// (one CTA per SM).  FP64, the same 91: 37.4 ms, 53 on eight.
-struct GjCls { int hi, nb; };
+// Size classes per precision.  Blocks of up to 1,536 rows go to
+// pc_invert_kernel on one, two or four CTAs of 256 threads, two per SM, so that
+// one's pivots hide behind the other's updates (FP64 above 768 rows: 512
+// threads, one per SM); larger ones to pc_gj_invert_kernel; blocks above the
+// last class go to cuSOLVER (FP64).  FP32, 422 blocks of 385 to 768 rows: 11.7
+// ms on two CTAs, 14.6 on four, 21.9 on eight (each CTA repeats the pivots),
+// 13.7 with 512 threads; 91 blocks of 769 to 1,226 rows, panels of 16: 15.0 ms
+// on four, 21.7 on two, 18.1 on eight; panels of 32: 15.7 and more (one CTA per
+// SM).  FP64, the same 91: 37.4 ms, 53 on eight; but eight where four a block
+// would leave SMs idle (8 blocks of up to 1,192 rows: 18.2 ms on four, 11.7 on
+// eight; 28 of up to 1,474: 33 and 22).
+constexpr int kSms = 148;
+static bool wide_clusters(int nList) { return nList * 4 <= kSms; }   // FP64 blocks of 769 to 1,536 rows
+struct InvClass { int hi, nb, cs, perSm; };   // rows up to, panel width, CTAs per block, CTAs per SM
 template <typename TV>
-static const GjCls *gj_classes(int *count) {
+static const InvClass *inv_classes(int *count) {
   // FP64 stops at 3200 rows: above it cuSOLVER's factorisation of a single
   // large block (all SMs) beats the kernel's narrow panels (measured on a
   // 2.1M-panel surface: 7.9 s against 9.8 s for the whole inversion)
-  static const GjCls d64[4] = {{384, 16}, {768, 16}, {1536, 16}, {3200, 8}};
-  static const GjCls d32[6] = {{384, 32}, {768, 32}, {1536, 16}, {3200, 16}, {6000, 8}, {11000, 4}};
+  static const InvClass d64[4] = {{384, 16, 1, 2}, {768, 16, 2, 2}, {1536, 16, 4, 1}, {3200, 8, 8, 1}};
+  static const InvClass d32[6] = {{384, 32, 1, 2}, {768, 32, 2, 2}, {1536, 16, 4, 2},
+                                  {3200, 16, 8, 1}, {6000, 8, 8, 1}, {11000, 4, 8, 1}};
   *count = sizeof(TV) == 8 ? 4 : 6;
   return sizeof(TV) == 8 ? d64 : d32;
 }
 
 template <typename TV>
 static bool launch_inversion(int ci, int nb, int nList, int maxM, cudaStream_t st, const int *d_list, PrecondDev &p,
-                             const long long *d_yOff, TV *inv, TV *d_y, int *d_info) {
+                             const long long *d_yOff, TV *inv, TV *d_y, int *d_info, bool share) {
   constexpr bool f = sizeof(TV) == 4;
-  if (ci == 0) return launch_inv_t<TV, f ? 32 : 16, 1, 2, 1, 256>(nList, maxM, st, d_list, p, inv, d_info);
-  if (ci == 1) return launch_inv_t<TV, f ? 32 : 16, 2, 3, 1, 256>(nList, maxM, st, d_list, p, inv, d_info);
-  if (ci == 2) return launch_inv_t<TV, 16, 4, f ? 6 : 3, 1, f ? 256 : 512>(nList, maxM, st, d_list, p, inv, d_info);
+  if (ci == 0) return launch_inv_t<TV, f ? 32 : 16, 1, 2, 1, 256>(nList, maxM, st, d_list, p, inv, d_info, share);
+  if (ci == 1) return launch_inv_t<TV, f ? 32 : 16, 2, 3, 1, 256>(nList, maxM, st, d_list, p, inv, d_info, share);
+  if constexpr (!f) {
+    if (ci == 2 && wide_clusters(nList)) return launch_inv_t<TV, 16, 8, 3, 1, 512>(nList, maxM, st, d_list, p, inv, d_info, share);
+  }
+  if (ci == 2) return launch_inv_t<TV, 16, 4, f ? 6 : 3, 1, f ? 256 : 512>(nList, maxM, st, d_list, p, inv, d_info, share);
   return launch_gj<TV>(nb, nList, maxM, st, d_list, p, d_yOff, inv, d_y, d_info);
 }
 
 template <typename TV>
 static int gj_max_rows() {
   int n = 0;
-  const GjCls *c = gj_classes<TV>(&n);
+  const InvClass *c = inv_classes<TV>(&n);
   return std::min(c[n - 1].hi, FB_PC_GJ_MAXM);
 }
 
@@ -1086,7 +1097,7 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   cudaStream_t s = c.stream;
   const int cut = gj_max_rows<TV>();
   int ncls = 0;
-  const GjCls *cls = gj_classes<TV>(&ncls);
+  const InvClass *cls = inv_classes<TV>(&ncls);
   std::vector<int> big;
   for (int b = 0; b < p.nBlocks; b++)
     if (2 * p.hSize[b] > cut) big.push_back(b);
@@ -1102,35 +1113,74 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   int *d_info = nullptr;
   DevArena tmp;
   if (!tmp.upload(&d_yOff, yOff, s) || !tmp.alloc_n(&d_y, (size_t)std::max(ytot, 1LL)) ||
-      !tmp.alloc_n(&d_info, (size_t)p.nBlocks))
+      !tmp.alloc_n(&d_info, (size_t)p.nBlocks + 1))
     return false;
   FB_CUDA(cudaMemsetAsync(d_info, 0, (size_t)p.nBlocks * sizeof(int), s));
-  // the classes one after the other, the largest blocks first: side by side they push each other's blocks out of
-  // the L2, and a cluster waits for free SMs (the star's three classes: 59 ms side by side, 31.7 in turn)
-  bool ok = true;
-  for (int ci = ncls - 1; ok && ci >= 0; ci--) {
-    const GjCls &k = cls[ci];
-    const int lo = ci ? cls[ci - 1].hi : 0, hi = std::min(k.hi, cut);
+  struct Job {
+    int ci, maxM = 0;
     std::vector<int> list;
-    int maxM = 0;
+    int *d_list = nullptr;
+  };
+  std::vector<Job> jobs;   // the classes with blocks, the largest blocks first
+  for (int ci = ncls - 1; ci >= 0; ci--) {
+    const int lo = ci ? cls[ci - 1].hi : 0, hi = std::min(cls[ci].hi, cut);
+    Job j{ci};
     for (int b = 0; b < p.nBlocks; b++) {
       const int M = 2 * p.hSize[b];
       if (hi > lo && M > lo && M <= hi) {
-        list.push_back(b);
-        maxM = std::max(maxM, M);
+        j.list.push_back(b);
+        j.maxM = std::max(j.maxM, M);
       }
     }
-    if (list.empty()) continue;
-    std::stable_sort(list.begin(), list.end(), [&](int a, int b) { return p.hSize[a] > p.hSize[b]; });
-    int *d_list = nullptr;
-    ok = tmp.upload(&d_list, list, s) && launch_inversion<TV>(ci, k.nb, (int)list.size(), maxM, s, d_list, p, d_yOff, inv, d_y, d_info);
+    if (j.list.empty()) continue;
+    std::stable_sort(j.list.begin(), j.list.end(), [&](int a, int b) { return p.hSize[a] > p.hSize[b]; });
+    jobs.push_back(std::move(j));
+  }
+  bool ok = true;
+  for (Job &j : jobs) ok = ok && tmp.upload(&j.d_list, j.list, s);
+  // A class starts beside the larger ones while those leave SMs idle, and in turn once they fill the chip, where
+  // classes side by side would push each other's blocks out of the L2 and clusters would wait for free SMs (the star's
+  // three classes of 100 to 600 blocks: 59 ms side by side, 31.7 in turn; FP64, 263 blocks of up to 996 rows: 11.4
+  // and 23.4; FP64, 55 of up to 1,100: 16.5 and 26.8).  The context's other streams carry them; its own is left to
+  // cuSOLVER when there are blocks for it.
+  const bool fork = jobs.size() > 1 || !big.empty();
+  cudaStream_t lane[3] = {c.farStream, c.sideStream, big.empty() ? s : c.sideStream};
+  if (fork)
+    ok = ok && cudaEventRecord(c.evFork, s) == cudaSuccess && cudaStreamWaitEvent(lane[0], c.evFork, 0) == cudaSuccess &&
+         cudaStreamWaitEvent(lane[1], c.evFork, 0) == cudaSuccess;
+  // Classes whose CTAs outnumber the SMs share them, which an SM's blocks of two kernels can only if its shared memory
+  // need not be divided anew: all ask for the largest share then (FP64, the 263 blocks: 16.4 ms without, 11.4 with it;
+  // but 8 FP32 blocks of up to 1,192 rows with the smaller L1 9.8 -> 10.4).
+  long long ctas = 0;
+  for (const Job &j : jobs) ctas += (long long)j.list.size() * cls[j.ci].cs;
+  const bool share = jobs.size() > 1 && ctas > kSms;
+  int filled = 0;   // SMs
+  for (size_t k = 0; ok && k < jobs.size(); k++) {
+    const Job &j = jobs[k];
+    const InvClass &t = cls[j.ci];
+    cudaStream_t st = fork ? lane[std::min<size_t>(k, 2)] : s;
+    if (filled >= kSms) {
+      ok = cudaEventRecord(c.evJoin, lane[std::min<size_t>(k - 1, 2)]) == cudaSuccess;
+      filled = 0;
+    }
+    // the next class starts after this one: its event comes before this launch, and a small fill holds it back until
+    // this one's clusters have their SMs (FP64, 1,100 blocks in three classes: 13.5 ms without the fill, 10.7 with it)
+    if (k > 0)
+      ok = ok && cudaStreamWaitEvent(st, c.evJoin, 0) == cudaSuccess &&
+           cudaMemsetAsync(d_info + p.nBlocks, 0, sizeof(int), st) == cudaSuccess;
+    if (fork) ok = ok && cudaEventRecord(c.evJoin, st) == cudaSuccess;
+    const int nList = (int)j.list.size();
+    ok = ok && launch_inversion<TV>(j.ci, t.nb, nList, j.maxM, st, j.d_list, p, d_yOff, inv, d_y, d_info, share);
+    filled += std::min(kSms, (nList * t.cs + t.perSm - 1) / t.perSm);
     c.launches += 1;
     ok = ok && cudaGetLastError() == cudaSuccess;
   }
-  // the large blocks through cuSOLVER on its own streams
+  // the large blocks meanwhile, through cuSOLVER on its own streams
   if (ok && !big.empty()) {
     if constexpr (sizeof(TV) == 8) ok = factor_cusolver(c, p, big);
   }
+  for (int k = 0; fork && k < 2; k++)
+    if (cudaEventRecord(c.evJoin, lane[k]) != cudaSuccess || cudaStreamWaitEvent(s, c.evJoin, 0) != cudaSuccess) ok = false;
   std::vector<int> info(p.nBlocks, 0);
   if (ok) ok = cudaMemcpyAsync(info.data(), d_info, info.size() * sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess;
   if (ok) ok = cudaStreamSynchronize(s) == cudaSuccess;

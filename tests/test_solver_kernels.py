@@ -98,6 +98,37 @@ def test_block_inverse_pivoting(panels, precision, tol):
     assert info == 0 and info_t == 0 and it <= 8 and abs(it - it_t) <= 1
 
 
+def patches(sizes):
+    """Patches of these many panels, each in an octant of its own."""
+    unit, faces = meshgen.icosphere(4)
+    pan = meshio.build_panels(20.0 * unit, unit, faces)
+    order = np.argsort(-pan.vtx[:, :, 2].mean(1))
+    keep = [np.sort(order[:n]) for n in sizes]
+    at = [300.0 * np.array([1 - 2 * (k & 1), 1 - (k & 2), 1 - (k & 4) / 2]) for k in range(len(sizes))]
+    return meshio.PanelSet(np.concatenate([pan.vtx[k] + a for k, a in zip(keep, at)]),
+                           *(np.concatenate([x[k] for k in keep]) for x in (pan.normal, pan.area)),
+                           np.arange(sum(sizes), dtype=np.int32))
+
+
+@pytest.mark.parametrize("sizes", [(12, 250), (12, 250, 500), (3, 10, 250, 260, 500, 800), (5, 300, 1601)])
+def test_block_inverse_classes_together(sizes):
+    """Blocks of several classes in one surface, which are inverted side by side, up to those of the library LU: FP64
+    against the oracle (to 800 panels), mixed against FP64."""
+    pan = patches(sizes)
+    opts = dict(order=2, depth=2, height=2)
+    s, m = (lib.Surface(pan, lib.params(precision=p, **opts)) for p in (lib.FP64, lib.MIXED))
+    b = np.random.default_rng(len(sizes)).standard_normal(2 * s.n)
+    x = []
+    for t in (s, m, s):   # the third: again on a context that has a preconditioner
+        t.precond_setup(2)
+        x.append(t.precond_apply(b))
+    assert rel_l2(x[1], x[0]) < 1e-4 and (x[2] == x[0]).all()
+    if max(sizes) <= 800:
+        o = O.Oracle(pan, O.make_params(**opts))
+        o.precond_setup(2)
+        assert rel_l2(x[0], o.precond_apply(b)) < 1e-11
+
+
 @pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
 @pytest.mark.parametrize("panels", [1, 17, 193, 385, 800])
 @pytest.mark.parametrize("where", [0, -1])
