@@ -1553,13 +1553,19 @@ static bool setup_m2l_adjoint(Context &c) {
   return true;
 }
 
+// Dynamic shared memory of the M2M and L2L kernels up to kMaxOrder (C(p + 6, 6) list entries), allowed as a whole: a
+// value by the context's order would change under another thread's context between the call and its launch.
+constexpr int kShiftSmem = kShiftWarps * 5 * nmom_c(kMaxOrder) * (int)sizeof(double) +
+                           (nmom_c(kMaxOrder) + 1 + 3003) * (int)sizeof(int);
+static_assert(kMaxOrder == 8, "C(kMaxOrder + 6, 6) above");
+
 // the moments of `count` cubes from their children's, two planes
 static bool launch_m2m(Context &c, int first, int count, int ordOut, int ordIn, const int *kidFirst,
                        const int *kidCount, const double *ctr, double *m1, double *m2, cudaStream_t s) {
   const int nOut = nmom(ordOut), nLst = c.h_mOff[nOut];
   const size_t shm = (size_t)kShiftWarps * 5 * nOut * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
   if (shm > 44 * 1024)
-    FB_CUDA(cudaFuncSetAttribute(m2m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    FB_CUDA(cudaFuncSetAttribute(m2m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kShiftSmem));
   m2m_kernel<<<count, kShiftWarps * 32, shm, s>>>(first, count, c.NM, ordOut, ordIn, kidFirst, kidCount, ctr,
                                                   c.d_mOff, c.d_mLst, nLst, m1, m2);
   return true;
@@ -1602,7 +1608,7 @@ bool launch_far_upward(Context &c, const double *sgm, bool adjoint, cudaEvent_t 
     int ordIn = pt.ordMom[lev], ordOut = pt.ordMom[lev + 1];
     const int nOut = nmom(ordOut), nLst = c.h_lstOff[nOut];
     const size_t shm = (size_t)kShiftWarps * 5 * nmom(ordIn) * sizeof(double) + (size_t)(nOut + 1 + nLst) * sizeof(int);
-    if (shm > 44 * 1024) cudaFuncSetAttribute(l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    if (shm > 44 * 1024) cudaFuncSetAttribute(l2l_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kShiftSmem);
     l2l_kernel<<<ceil_div(pt.fmmLevelCount[lev + 1], kShiftWarps), kShiftWarps * 32, shm, s>>>(
         pt.fmmLevelStart[lev + 1], pt.fmmLevelCount[lev + 1], c.NM, ordIn, ordOut, c.d_fmmParent, c.d_cubeCtr,
         c.d_lstOff, c.d_lst, nLst, d1, d2, c.d_lec + 2 * plane, c.d_lec + 3 * plane);

@@ -986,8 +986,9 @@ static bool launch_gj_t(int nList, int maxM, cudaStream_t st, const int *d_list,
   FB_CHECK(shm + fa.sharedSizeBytes <= (size_t)optin,
            "Gauss-Jordan class NB=%d: %d rows need %zu + %zu bytes of shared memory, above the %d available", NB,
            maxM, shm, (size_t)fa.sharedSizeBytes, optin);
+  // (the same value every time: another thread's set-up may come between this and the launch)
   FB_CUDA(cudaFuncSetAttribute(pc_gj_invert_kernel<TV, NB, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)shm));
+                               optin - (int)fa.sharedSizeBytes));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nList * CS));
   cfg.blockDim = dim3(kGjThreads);
@@ -1021,8 +1022,9 @@ static bool launch_inv_t(int nList, int maxM, cudaStream_t st, const int *d_list
                          int *d_info, bool share) {
   FB_CHECK(maxM <= RPT * NT, "inversion class of %d rows given %d", RPT * NT, maxM);
   const size_t shm = inv_smem_bytes<TV, NB, QC>(maxM);
+  // (the same value every time: another thread's set-up may come between this and the launch)
   FB_CUDA(cudaFuncSetAttribute(pc_invert_kernel<TV, NB, CS, RPT, QC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)shm));
+                               (int)inv_smem_bytes<TV, NB, QC>(RPT * NT)));
   FB_CUDA(cudaFuncSetAttribute(pc_invert_kernel<TV, NB, CS, RPT, QC, NT>,
                                cudaFuncAttributePreferredSharedMemoryCarveout,
                                share ? cudaSharedmemCarveoutMaxShared : cudaSharedmemCarveoutDefault));

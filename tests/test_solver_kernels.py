@@ -4,6 +4,7 @@ restatement oracle.
 Tolerances: FP64 operators 1e-12 and block inverses 1e-11 relative L2, as for the golden cases; block inverses of mixed
 contexts 1e-4 (FP32 inverses of well-conditioned blocks: rows * 2^-24 <= 1536 * 6e-8); mixed operators 5e-6.
 """
+import concurrent.futures
 import functools
 
 import numpy as np
@@ -238,3 +239,24 @@ def test_charge_tree_moments(charges, order):
     s = lib.Surface(pan, lib.params(precision=lib.FP64, **opts), charges=ch)
     o = O.Oracle(pan, O.make_params(**opts), charges=ch)
     assert rel_l2(s.rhs(use_tree=True), o.rhs_tree()) < 1e-12
+
+
+def test_contexts_on_threads():
+    """Contexts of other block sizes and orders at work on two threads: each launch asks for its own shared memory."""
+    def work(case):
+        sizes, order = case
+        pan = patches(sizes)
+        s = lib.Surface(pan, lib.params(order=order, depth=4, height=2, precision=lib.FP64))
+        b = np.random.default_rng(order).standard_normal(2 * s.n)
+        out = []
+        for _ in range(30):
+            s.precond_setup(2)
+            out.append(np.r_[s.precond_apply(b), s.matvec(b)])
+        return out
+
+    cases = [((90, 250, 500), 7), ((60, 200, 400), 8)]
+    with concurrent.futures.ThreadPoolExecutor(2) as pool:
+        both = list(pool.map(work, cases))
+    for case, out in zip(cases, both):
+        alone = work(case)[0]
+        assert all((x == alone).all() for x in out)
