@@ -16,7 +16,8 @@ namespace fb {
 // 1/sqrt(x) for normal x > 0: one third-order Householder step
 //   y (1 + e/2 + 3 e^2 / 8),  e = 1 - x y^2,
 // from the hardware's approximation, whose relative error of at most about
-// 2^-20 leaves a truncation of 5/16 e^3 below 2^-60.
+// 2^-20 makes |e| 2^-19 and leaves a truncation of 5/16 e^3 = 2^-58.7.  With the
+// roundings within 1.6 * 2^-53 of the exact value (1.24 measured, 1.01 for the library).
 __device__ __forceinline__ double rsqrt_pos(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -29,8 +30,8 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
 // |f| <= 1/2, e^t = 2^m 2^(j/64) e^(f ln2/64), the last factor by its Taylor
 // polynomial of degree 5 (truncation below 4e-17).  The caller passes s, whose
 // rounding is the argument's own.  s <= 0; below -64 * 1021 the result is
-// 2^-1021 (about 1e-308) instead of a denormal or zero.  tab: the 64 values, in
-// shared memory (load_exp_tab).
+// 2^-1021 (about 1e-308) instead of a denormal or zero.  Within 2.4 * 2^-53 of
+// e^t (2.03 measured, 1.23 for the library).  tab: the 64 values, in shared memory (load_exp_tab).
 constexpr int kExpTab = 64;
 constexpr double kExpScale = 92.332482616893656877;   // 64 / ln 2
 __device__ double g_expTab[kExpTab];
