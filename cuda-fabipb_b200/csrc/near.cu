@@ -8,17 +8,21 @@
 // rules instead (src/numQuad.c:401-571).
 //
 // B200 design:
-//   * nothing per pair is stored: each warp owns 32 target panels of one
-//     leaf, keeps them in registers, and streams the source panels of every
-//     near leaf through a per-warp shared-memory tile, so the P2P work is pure
-//     FP32 (or FP64) ALU + two MUFU ops per pair;
-//   * positions are stored relative to their own leaf centre, and a target
-//     is moved into each source leaf's frame once per leaf pair, which keeps
+//   * nothing per pair is stored.  Pairs of distinct near parts (leaves, or
+//     runs of panels in a direct FP64 context) are tasks: a warp or a half-warp
+//     evaluates each unordered panel pair once for both directions, one or two
+//     targets per lane in registers and the other part in shared-memory tiles,
+//     and leaves the sums in scratch slots.  A finishing kernel takes what is
+//     left (each part with itself, parts of a few panels) and adds the slots in
+//     a fixed order.  The work is FP32 (or FP64) arithmetic: two MUFU per pair
+//     in FP32, own reciprocal root and exponential in FP64 (fastmath.cuh);
+//   * positions are stored relative to their own part's centre, and a target
+//     is moved into each source part's frame once per pair of parts, which keeps
 //     FP32 differences of close panels accurate to ~1e-7 relative;
 //   * the coincident pair is masked (r = 0 gives 0), and every pair with a
 //     shared vertex carries an FP64 correction "exact Sauter value minus the
 //     one-point value" in a CSR table built once on the device, applied in
-//     FP64 in the same kernel.
+//     FP64 by the finishing kernel.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -820,7 +824,7 @@ __global__ void special_coeff_kernel(long long nSp, const int *__restrict__ spDs
 // their order-q value minus the one-point value.
 // One thread per target, looping over every near pair with the singular rules
 // in line, took 9.4 ms for the product of 2,048 panels at q = 2 (243 near
-// panels each, 16 blocks on the chip); with this it takes 0.147 ms.
+// panels each, 16 blocks on the chip); with this it takes 0.093 ms.
 constexpr int kQuadWarps = 4;
 constexpr int kQuadPoints = 100;   // q <= 10
 

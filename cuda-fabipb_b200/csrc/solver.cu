@@ -167,25 +167,27 @@ __global__ void identity_kernel(int nList, const int *__restrict__ list, const i
 // Per panel of NB columns:
 //   * every CTA of the cluster eliminates the panel in its shared memory (the
 //     same data, so the same result), eight columns at a time with its rows in
-//     registers (row i belongs to thread i mod 256), one barrier per pivot: the
+//     registers (row i belongs to thread i mod NT), one barrier per pivot: the
 //     warps' candidates (largest |a| among the rows not yet taken) carry their
 //     rows along; each eight columns are then a rank-8 update of the panel's rest;
 //   * each CTA takes its share of the other columns, dealt in tiles:
 //     A(:, j) = A(:, j) without the pivot rows + Panel * A(pivot rows, j).
 // Rows are never interchanged: perm[k] is the row that column k was eliminated
 // with, stored column c multiplies input component colSrc[c] = perm[c], and
-// stored row perm[k] is output component rowDst[perm[k]] = k.  info[b] = k + 1 for the first column whose pivot is
-// zero, not finite or without a finite reciprocal; perm stays a permutation of the rows whatever the values are.
+// stored row perm[k] is output component rowDst[perm[k]] = k.  info[b] = k + 1
+// for the first column whose pivot is zero, not finite or without a finite
+// reciprocal; perm stays a permutation of the rows whatever the values are.
 //
-// 2 M^3 operations; bound by the blocks' traffic in the updates (every panel
-// reads and writes a whole block, and the blocks in work exceed the L2) and by
-// the pivots' latency in the panels, so panels are as wide as shared memory
-// allows and two CTAs share an SM.  A panel of 32 columns of a 575-row block on
+// 2 M^3 operations; bound by latency: at two CTAs per SM the updates' loads
+// from the block and from shared memory and the pivots' barriers each stall
+// about as much (every panel reads and writes a whole block, at a quarter of the
+// DRAM's peak rate).  So panels are as wide as shared memory allows.  A panel of 32 columns of a 575-row block on
 // two CTAs: 46 us of pivots and in-panel updates, 26 gathering the pivot rows,
 // 115 updating.  With interchanged rows, panels of 16 eliminated in shared
-// memory with two barriers per pivot, the interchange list formed by one thread
-// and the classes side by side, the 1,127 blocks of the 204,800-panel star
-// surface (mean 363 rows) took 52 ms in FP32; 27.5 now.
+// memory with two barriers per pivot and the interchange list formed by one
+// thread, the 1,108 blocks of a 204,800-panel star surface (mean 370 rows, 96
+// above 768 and one of 1,672) took 74 ms in FP32; 28 now, as long as the one
+// block of the next kernel takes.
 constexpr int kInvSub = 8;   // columns eliminated in registers
 
 template <typename TV>
@@ -264,7 +266,7 @@ pc_invert_kernel(const int *__restrict__ list, const int *__restrict__ bStart, c
 #pragma unroll 16
       for (int c = 0; c < nb; c++) P[c * Mp + i] = src[(size_t)c * M];
     }
-    // (row i of P and of flag: written and read by thread i mod 256 until the next barrier)
+    // (row i of P and of flag: written and read by thread i mod NT until the next barrier)
     for (int c0 = 0; c0 < nb; c0 += kInvSub) {
       const int sb = min(kInvSub, nb - c0);
       TV v[RPT][kInvSub];
@@ -1059,15 +1061,14 @@ static bool launch_inv_t(int nList, int maxM, cudaStream_t st, const int *d_list
 // eight; 28 of up to 1,474: 33 and 22).
 constexpr int kSms = 148;
 static bool wide_clusters(int nList) { return nList * 4 <= kSms; }   // FP64 blocks of 769 to 1,536 rows
-struct InvClass { int hi, nb, cs, perSm; };   // rows up to, panel width, CTAs per block, CTAs per SM
+struct InvClass { int hi, nb, cs; };   // rows up to, panel width, CTAs per block
 template <typename TV>
 static const InvClass *inv_classes(int *count) {
   // FP64 stops at 3200 rows: above it cuSOLVER's factorisation of a single
   // large block (all SMs) beats the kernel's narrow panels (measured on a
   // 2.1M-panel surface: 7.9 s against 9.8 s for the whole inversion)
-  static const InvClass d64[4] = {{384, 16, 1, 2}, {768, 16, 2, 2}, {1536, 16, 4, 1}, {3200, 8, 8, 1}};
-  static const InvClass d32[6] = {{384, 32, 1, 2}, {768, 32, 2, 2}, {1536, 16, 4, 2},
-                                  {3200, 16, 8, 1}, {6000, 8, 8, 1}, {11000, 4, 8, 1}};
+  static const InvClass d64[4] = {{384, 16, 1}, {768, 16, 2}, {1536, 16, 4}, {3200, 8, 8}};
+  static const InvClass d32[6] = {{384, 32, 1}, {768, 32, 2}, {1536, 16, 4}, {3200, 16, 8}, {6000, 8, 8}, {11000, 4, 8}};
   *count = sizeof(TV) == 8 ? 4 : 6;
   return sizeof(TV) == 8 ? d64 : d32;
 }
@@ -1090,6 +1091,11 @@ static int gj_max_rows() {
   int n = 0;
   const InvClass *c = inv_classes<TV>(&n);
   return std::min(c[n - 1].hi, FB_PC_GJ_MAXM);
+}
+
+// about 20 us
+__global__ void pause_kernel() {
+  for (int i = 0; i < 20; i++) __nanosleep(1000);
 }
 
 // Gauss-Jordan inversion of every block of inv (assembled there), class by
@@ -1115,7 +1121,7 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   int *d_info = nullptr;
   DevArena tmp;
   if (!tmp.upload(&d_yOff, yOff, s) || !tmp.alloc_n(&d_y, (size_t)std::max(ytot, 1LL)) ||
-      !tmp.alloc_n(&d_info, (size_t)p.nBlocks + 1))
+      !tmp.alloc_n(&d_info, (size_t)p.nBlocks))
     return false;
   FB_CUDA(cudaMemsetAsync(d_info, 0, (size_t)p.nBlocks * sizeof(int), s));
   struct Job {
@@ -1140,40 +1146,35 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   }
   bool ok = true;
   for (Job &j : jobs) ok = ok && tmp.upload(&j.d_list, j.list, s);
-  // A class starts beside the larger ones while those leave SMs idle, and in turn once they fill the chip, where
-  // classes side by side would push each other's blocks out of the L2 and clusters would wait for free SMs (the star's
-  // three classes of 100 to 600 blocks: 59 ms side by side, 31.7 in turn; FP64, 263 blocks of up to 996 rows: 11.4
-  // and 23.4; FP64, 55 of up to 1,100: 16.5 and 26.8).  The context's other streams carry them; its own is left to
-  // cuSOLVER when there are blocks for it.
+  // The classes run side by side, the largest blocks' clusters placed first, on the context's other streams (its own is
+  // left to cuSOLVER when there are blocks for it): a class alone leaves SMs idle, when it has few blocks and at its
+  // end.  FP64, 263 blocks of up to 996 rows: 23.4 ms in turn, 11.3 side by side; FP64, 55 of up to 1,100: 26.8 and
+  // 16.4; FP32, three stars of 1,100 blocks: 61.8, 37.8 and 28.9 in turn, 30.0, 29.9 and 26.3.
   const bool fork = jobs.size() > 1 || !big.empty();
   cudaStream_t lane[3] = {c.farStream, c.sideStream, big.empty() ? s : c.sideStream};
   if (fork)
     ok = ok && cudaEventRecord(c.evFork, s) == cudaSuccess && cudaStreamWaitEvent(lane[0], c.evFork, 0) == cudaSuccess &&
          cudaStreamWaitEvent(lane[1], c.evFork, 0) == cudaSuccess;
-  // Classes whose CTAs outnumber the SMs share them, which an SM's blocks of two kernels can only if its shared memory
-  // need not be divided anew: all ask for the largest share then (FP64, the 263 blocks: 16.4 ms without, 11.4 with it;
-  // but 8 FP32 blocks of up to 1,192 rows with the smaller L1 9.8 -> 10.4).
+  // Classes whose CTAs outnumber the SMs share them, which blocks of two kernels on an SM can only if its shared memory
+  // need not be divided anew: all ask for the largest share then.  (The 263 blocks: 16.4 ms without, 11.3 with it.
+  // But 8 FP32 blocks of up to 1,192 rows with the smaller L1 9.8 -> 10.4.)
   long long ctas = 0;
   for (const Job &j : jobs) ctas += (long long)j.list.size() * cls[j.ci].cs;
   const bool share = jobs.size() > 1 && ctas > kSms;
-  int filled = 0;   // SMs
   for (size_t k = 0; ok && k < jobs.size(); k++) {
     const Job &j = jobs[k];
-    const InvClass &t = cls[j.ci];
     cudaStream_t st = fork ? lane[std::min<size_t>(k, 2)] : s;
-    if (filled >= kSms) {
-      ok = cudaEventRecord(c.evJoin, lane[std::min<size_t>(k - 1, 2)]) == cudaSuccess;
-      filled = 0;
+    // the next class starts after this one: its event comes before this launch, and a pause holds it back until this
+    // one's clusters have their SMs (without it smaller blocks can take them first: FP64, 1,100 blocks in three classes
+    // 13.5 ms without it, 10.6 with it; the first star 41 and 29.9)
+    if (k > 0) {
+      ok = ok && cudaStreamWaitEvent(st, c.evJoin, 0) == cudaSuccess;
+      if (ok) pause_kernel<<<1, 1, 0, st>>>();
+      c.launches += 1;
     }
-    // the next class starts after this one: its event comes before this launch, and a small fill holds it back until
-    // this one's clusters have their SMs (FP64, 1,100 blocks in three classes: 13.5 ms without the fill, 10.7 with it)
-    if (k > 0)
-      ok = ok && cudaStreamWaitEvent(st, c.evJoin, 0) == cudaSuccess &&
-           cudaMemsetAsync(d_info + p.nBlocks, 0, sizeof(int), st) == cudaSuccess;
     if (fork) ok = ok && cudaEventRecord(c.evJoin, st) == cudaSuccess;
-    const int nList = (int)j.list.size();
-    ok = ok && launch_inversion<TV>(j.ci, t.nb, nList, j.maxM, st, j.d_list, p, d_yOff, inv, d_y, d_info, share);
-    filled += std::min(kSms, (nList * t.cs + t.perSm - 1) / t.perSm);
+    ok = ok && launch_inversion<TV>(j.ci, cls[j.ci].nb, (int)j.list.size(), j.maxM, st, j.d_list, p, d_yOff, inv, d_y,
+                                    d_info, share);
     c.launches += 1;
     ok = ok && cudaGetLastError() == cudaSuccess;
   }
