@@ -705,7 +705,8 @@ near_apply_f2_kernel(const int2 *__restrict__ work, const int *__restrict__ leaf
   if ((int)threadIdx.x < mt) near_store(base + g0 + threadIdx.x, n, p, area, coef, accumulate, out);
 }
 
-template <bool ADJ>
+// MEET: any two parts may hold coincident panels (near_terms)
+template <bool ADJ, bool MEET>
 __global__ void __launch_bounds__(kNearWarps * 32)
 near_apply_kernel(const int2 *__restrict__ work, const int *__restrict__ leafStart,
                   const int *__restrict__ leafCount, const int *__restrict__ ordOff,
@@ -714,7 +715,7 @@ near_apply_kernel(const int2 *__restrict__ work, const int *__restrict__ leafSta
                   const int *__restrict__ spOff, const int *__restrict__ spSrc, const double4 *__restrict__ spK,
                   const double *__restrict__ sgm, const double *__restrict__ area, int n, NearConstD K, double coef,
                   int accumulate, double *out, const int *__restrict__ gatOff, const int *__restrict__ gatSlot,
-                  const double2 *__restrict__ scr, bool meet) {
+                  const double2 *__restrict__ scr) {
   __shared__ double4 sA[kNearWarps][32], sB[kNearWarps][32];
   __shared__ double tab[kExpTab];
   load_exp_tab(tab);
@@ -745,7 +746,7 @@ near_apply_kernel(const int2 *__restrict__ work, const int *__restrict__ leafSta
       if (lane < m)
         near_record<double>(sb + j0 + lane, n, tgtP, tgtN, area, sgm, sA[warp][lane], sB[warp][lane]);
       __syncwarp();
-      if (S == L || meet) {   // warp-uniform; meet: any two parts may hold coincident panels
+      if (MEET || S == L) {   // warp-uniform
 #pragma unroll 2
         for (int jj = sub; jj < m; jj += k)
           near_pair<ADJ, true>(sA[warp][jj], sB[warp][jj], tx, ty, tz, tn, K, tab, p.s0, p.s1);
@@ -1569,10 +1570,11 @@ static void launch_near_f64(Context &c, const double *sgm, double coef, double *
                                            c.d_partCtr, recA, recB, K, (double2 *)c.d_symScr);
     c.launches += 2;
   }
-  near_apply_kernel<ADJ><<<c.nWork, kNearWarps * 32, 0, s>>>(
+  auto apply = meet ? near_apply_kernel<ADJ, true> : near_apply_kernel<ADJ, false>;
+  apply<<<c.nWork, kNearWarps * 32, 0, s>>>(
       c.d_work, c.d_partStart, c.d_partCount, own ? c.d_ordOff : c.d_nearOff, own ? c.d_ordSrc : c.d_nearSrc,
       c.d_partCtr, tgtP, tgtN, c.d_spOff, c.d_spSrc, ADJ ? c.d_spKT : c.d_spK, sgm, c.d_area, c.n, K, coef,
-      accumulate ? 1 : 0, out, sym ? c.d_gatOff : nullptr, c.d_gatSlot, (const double2 *)c.d_symScr, meet);
+      accumulate ? 1 : 0, out, sym ? c.d_gatOff : nullptr, c.d_gatSlot, (const double2 *)c.d_symScr);
   c.launches += 1;
 }
 
