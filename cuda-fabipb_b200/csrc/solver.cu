@@ -1194,12 +1194,8 @@ static bool factor_gauss_jordan(Context &c, PrecondDev &p, TV *inv) {
   return true;
 }
 
-bool precond_setup(Context &c, int mode) {
-  free_precond(c);
-  c.pc = new PrecondDev();
+static bool setup_blocks(Context &c) {
   PrecondDev &p = *c.pc;
-  p.mode = mode;
-  if (mode != 2) return true;   // -1 identity and 3 diagonal need no setup
   const Octree &t = c.pt.t;
   const int lev = t.depth - 1;
   FB_CHECK(lev >= 0, "block preconditioner needs depth >= 1");
@@ -1258,6 +1254,15 @@ bool precond_setup(Context &c, int mode) {
   }
   tm.mark("factor_invert");
   return ok;
+}
+
+bool precond_setup(Context &c, int mode) {
+  free_precond(c);
+  c.pc = new PrecondDev();
+  c.pc->mode = mode;   // -1 identity and 3 diagonal need no setup
+  if (mode != 2 || setup_blocks(c)) return true;
+  free_precond(c);   // no half-built inverse for a later call
+  return false;
 }
 
 bool precond_apply(Context &c, const double *b, double *x, bool adjoint) {

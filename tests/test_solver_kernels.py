@@ -143,6 +143,8 @@ def test_block_inverse_of_a_non_finite_panel(panels, where, precision):
                     lib.params(order=2, depth=1, height=1, precision=precision))
     with pytest.raises(RuntimeError, match="non-finite pivot"):
         s.precond_setup(2)
+    with pytest.raises(RuntimeError, match="not set up"):
+        s.precond_apply(np.ones(2 * s.n))
     s.precond_setup(3)   # the diagonal, which reads areas only
     assert np.isfinite(s.precond_apply(np.ones(2 * s.n))).all()
 
